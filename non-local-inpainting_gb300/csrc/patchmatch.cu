@@ -112,6 +112,26 @@ enum PmVariant { kPmShared = 0, kPmStaged = 1, kPmRegs = 2 };
 
 __host__ __device__ constexpr int pm_threads(int V) { return V == kPmRegs ? 512 : 1024; }
 
+// Launch shape of the persistent kernels for nt target points: one block per
+// SM, with just enough warps that every point has one (up to the variant's
+// most).  A point is one warp's serial chain of loads and evaluations, and a
+// sweep of a coarse level is bound by the warps that share an SM, so the
+// points are spread over all SMs first: a PatchMatch call on a 64 x 48 level
+// (500 points) took 348 us with full blocks on 16 SMs and takes 288 us with
+// 4 warps on each of 125; 130 x 81: 401 and 375 us.  From 32 points per SM
+// on, the shape is that of full blocks, which no smaller block beat.
+struct PmShape {
+	int grid, block;
+};
+
+inline PmShape pm_shape(int V, long long nt, int num_sms)
+{
+	const int most = pm_threads(V) / 32;
+	const long long per_sm = (nt + num_sms - 1) / num_sms;
+	const int warps = (int)std::max(1LL, std::min((long long)most, per_sm));
+	return {(int)std::min((long long)num_sms, (nt + warps - 1) / warps), 32 * warps};
+}
+
 // Per-warp state of the staged path.
 struct TmaState {
 	const CUtensorMap *map;
@@ -1067,9 +1087,8 @@ static void launch_sweeps(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int 
                           int2 *nnf_x, float *dist_x, int2 *nnf_y, float *dist_y, unsigned long long *counter,
                           const PmMetrics &mt, const CUtensorMap &map, size_t smem)
 {
-	// persistent: one block per SM (fewer when there are fewer points)
-	const int block = pm_threads(V);
-	const int grid = (int)std::min<size_t>(((size_t)p.nt * 32 + block - 1) / block, (size_t)ctx->num_sms);
+	const PmShape shape = pm_shape(V, p.nt, ctx->num_sms);
+	const int block = shape.block, grid = shape.grid;
 	int *timeout = &ctx->status->timeout;
 	// The kernels' dynamic shared-memory limit is raised once per device, to
 	// the largest opt-in size (each launch passes the size it uses): a
@@ -1116,7 +1135,8 @@ static void run_sweeps(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int ite
 	std::memset(&map, 0, sizeof(map));
 	if constexpr (P > 0) {
 		if (ctx->tune_pm_variant == kPmStaged) {
-			const size_t smem = pm_smem_bytes_tma(taps, p.rows, p.L, p.K, pm_threads(kPmStaged) / 32);
+			const size_t smem = pm_smem_bytes_tma(taps, p.rows, p.L, p.K,
+			                                      pm_shape(kPmStaged, p.nt, ctx->num_sms).block / 32);
 			if (smem <= (size_t)ctx->max_smem_optin && encode_source_map(p, &map)) {
 				launch_sweeps<KIND, C, P, kPmStaged>(ctx, a, p, iterations, init, nnf_x, dist_x, nnf_y, dist_y,
 				                                     counter, mt, map, smem);
@@ -1124,12 +1144,15 @@ static void run_sweeps(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int ite
 			}
 		} else if (ctx->tune_pm_variant == kPmRegs) {
 			launch_sweeps<KIND, C, P, kPmRegs>(ctx, a, p, iterations, init, nnf_x, dist_x, nnf_y, dist_y, counter,
-			                                   mt, map, pm_smem_bytes(taps, p.rows, p.L, pm_threads(kPmRegs) / 32));
+			                                   mt, map,
+			                                   pm_smem_bytes(taps, p.rows, p.L,
+			                                                 pm_shape(kPmRegs, p.nt, ctx->num_sms).block / 32));
 			return;
 		}
 	}
 	launch_sweeps<KIND, C, P, kPmShared>(ctx, a, p, iterations, init, nnf_x, dist_x, nnf_y, dist_y, counter, mt, map,
-	                                     pm_smem_bytes(taps, p.rows, p.L, pm_threads(kPmShared) / 32));
+	                                     pm_smem_bytes(taps, p.rows, p.L,
+	                                                   pm_shape(kPmShared, p.nt, ctx->num_sms).block / 32));
 }
 
 static void sweep_energy(cudaStream_t s, const PmArgs &p, const float *dist, const PmMetrics &m, int sweep)
@@ -1328,9 +1351,10 @@ __global__ void k_copy_targets_batch(const __grid_constant__ PmBatchArgs B)
 }
 
 template <int KIND, int C, int P>
-static void run_batch_kernels(nli_ctx *ctx, const DistArgs &a, const PmBatchArgs &B, int iterations, size_t smem,
-                              unsigned long long *counter)
+static void run_batch_kernels(nli_ctx *ctx, const DistArgs &a, const PmBatchArgs &B, int iterations, PmShape shape,
+                              size_t smem, unsigned long long *counter)
 {
+	const int block = shape.block, grid = shape.grid;
 	// dynamic shared memory up to the opt-in limit less the kernels' static
 	// shared memory (the work-list prefix), raised once per device
 	static std::atomic<uint32_t> raised{0};  // one bit per device
@@ -1350,8 +1374,6 @@ static void run_batch_kernels(nli_ctx *ctx, const DistArgs &a, const PmBatchArgs
 	}
 	NLI_REQUIRE(smem <= (size_t)dyn_max[ctx->device & 31].load(std::memory_order_relaxed), NLI_E_UNSUPPORTED,
 	            "PatchMatch shared memory too large");
-	const int block = pm_threads(kPmShared);
-	const int grid = ctx->num_sms;
 	{
 		ProfScope ps(ctx, "pm_init");
 		k_pm_init_batch<KIND, C, P><<<grid, block, smem, ctx->stream>>>(a, B, counter);
@@ -1377,6 +1399,7 @@ void patchmatch_batch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli
 	B.active = active;
 	B.tile = ctx->tune_pm_tile;
 	int maxpix = 0, maxpad = 0, maxnt = 0;
+	long long total = 0;  // target points of all images
 	for (int i = 0; i < n; i++) {
 		const PmBatchItem &it = items[i];
 		NLI_REQUIRE(it.W < 32768 && it.H < 32768, NLI_E_UNSUPPORTED, "PatchMatch source sides must be below 32768");
@@ -1420,6 +1443,7 @@ void patchmatch_batch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli
 		maxpix = max(maxpix, it.W * it.H);
 		maxpad = max(maxpad, (it.W + 1) * (it.H + 1));
 		maxnt = max(maxnt, it.nt);
+		total += it.nt;
 	}
 	cudaStream_t s = ctx->stream;
 	const int per = 256;
@@ -1440,16 +1464,17 @@ void patchmatch_batch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli
 		NLI_CUDA(cudaMemsetAsync(B.queue, 0, sizeof(unsigned) * slots, s));
 	}
 	const int taps = a.px * a.py;
-	const size_t smem = pm_smem_bytes(taps, B.t[0].p.rows, B.t[0].p.L, pm_threads(kPmShared) / 32);
+	const PmShape shape = pm_shape(kPmShared, total, ctx->num_sms);
+	const size_t smem = pm_smem_bytes(taps, B.t[0].p.rows, B.t[0].p.L, shape.block / 32);
 	NLI_REQUIRE(smem <= (size_t)ctx->max_smem_optin, NLI_E_UNSUPPORTED, "PatchMatch shared memory too large");
 	const bool p9 = a.px == 9 && a.py == 9;
 	bool handled = false;
 #define NLI_PMB_CASE(KIND, CC)                                                                  \
 	if (dp.kind == KIND && C == CC) {                                                           \
 		if (p9)                                                                                 \
-			run_batch_kernels<KIND, CC, 9>(ctx, a, B, pm.iterations, smem, counter);          \
+			run_batch_kernels<KIND, CC, 9>(ctx, a, B, pm.iterations, shape, smem, counter);   \
 		else                                                                                    \
-			run_batch_kernels<KIND, CC, 0>(ctx, a, B, pm.iterations, smem, counter);          \
+			run_batch_kernels<KIND, CC, 0>(ctx, a, B, pm.iterations, shape, smem, counter);   \
 		handled = true;                                                                         \
 	}
 	NLI_PMB_CASE(NLI_DIST_L2_COMBINED, 3)
