@@ -295,6 +295,7 @@ struct PmBatchItem {
 	float4 *pad;          // (W + 1) * (H + 1) padded pixels
 	int32_t *nnf_y;       // W * H int2
 	float *dist_x, *dist_y;  // W * H
+	uint8_t *hist_x, *hist_y;  // W * H change histories
 	uint64_t seed;
 	unsigned long long *calls;    // the image's PatchMatch call index (device)
 	unsigned long long *counter;  // the image's candidate counters (2, device) or null

@@ -602,6 +602,7 @@ struct LkImage {
 	int32_t *A = nullptr, *B = nullptr, *nnf_l = nullptr, *scaled = nullptr, *nnf_y = nullptr;
 	float4 *pad = nullptr, *mom = nullptr;
 	float *dist_x = nullptr, *dist_y = nullptr;
+	uint8_t *hist_x = nullptr, *hist_y = nullptr;
 	unsigned *vmax = nullptr;
 	int64_t pm_calls = 0, upd_calls = 0, graph_iters = 0;
 	bool ok() const { return status == NLI_OK; }
@@ -689,6 +690,8 @@ class Lockstep {
 			m.mom = a.take<float4>((size_t)(m.W + 1) * (m.H + 1) * 4);
 			m.dist_x = a.take<float>(n0);
 			m.dist_y = a.take<float>(n0);
+			m.hist_x = a.take<uint8_t>(n0);
+			m.hist_y = a.take<uint8_t>(n0);
 			m.vmax = a.take<unsigned>(1);
 			if (pass == 0) arena_size[g] = a.off + 256;
 		}
@@ -765,6 +768,8 @@ class Lockstep {
 		it.nnf_y = m.nnf_y;
 		it.dist_x = m.dist_x;
 		it.dist_y = m.dist_y;
+		it.hist_x = m.hist_x;
+		it.hist_y = m.hist_y;
 		it.seed = m.seed;
 		it.calls = &dev->calls[g];
 		it.counter = dev->cand[g];
