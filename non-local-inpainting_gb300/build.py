@@ -14,7 +14,8 @@ LIB = os.path.join(HERE, "libnli_gb300.so")
 DROPIN = os.path.join(HERE, "libnli_dropin.so")
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 
-SOURCES = ["api.cu", "gradient.cu", "distance.cu", "patchmatch.cu", "update.cu", "pyramid.cu", "process.cu",
+SOURCES = ["api.cu", "gradient.cu", "distance.cu", "patchmatch.cu", "pm_combined.cu",
+           "pm_combined_rgb.cu", "pm_rgbd.cu", "pm_l2.cu", "pm_l1.cu", "update.cu", "pyramid.cu", "process.cu",
            "batch.cu", "color.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
