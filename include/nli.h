@@ -134,8 +134,8 @@ typedef struct nli_process_stats {
 	int32_t targets[NLI_MAX_SCALES];     /* PatchMatch target points per scale (the
 	                                        extended domain minus the margin) */
 	int32_t holes[NLI_MAX_SCALES];       /* hole pixels per scale (the CG's unknowns) */
-	int64_t candidates_partial;          /* of the candidates, those stopped after the
-	                                        early-termination test */
+	int64_t candidates_partial;          /* of the candidates, those that had reached
+	                                        the match at the early-termination test */
 } nli_process_stats;
 
 typedef struct nli_ctx nli_ctx;
@@ -168,8 +168,8 @@ int nli_ctx_set_profiling(nli_ctx *ctx, int enable);
  * kernel name, launches and total milliseconds.  NLI_E_INVALID past the end. */
 int nli_ctx_profile_entry(nli_ctx *ctx, int index, char *name, int name_len, int64_t *launches, double *ms);
 /* Running totals of this context: PatchMatch distance evaluations counted
- * on the device, the part of them stopped early (after the first 32 taps
- * their partial sum already exceeded the current match), conjugate-gradient
+ * on the device, the part of them whose partial sum had already reached the
+ * point's match at the early-termination test, conjugate-gradient
  * iterations (summed over channels) and the same weighted by the number of
  * unknowns of each solve.  Any pointer may be NULL. */
 int nli_ctx_counters(nli_ctx *ctx, int64_t *candidates, int64_t *candidates_partial, int64_t *cg_iterations,
@@ -406,12 +406,14 @@ int nli_ctx_set_batch_width(nli_ctx *ctx, int width);
  *   NLI_TUNE_CG_CLUSTER_CAP        CTAs per CG cluster at most (1..16, default 16)
  *   NLI_TUNE_CG_UNKNOWNS_PER_CTA   unknowns per CG CTA at least (default 1024)
  *   NLI_TUNE_BATCH_WIDTH           as nli_ctx_set_batch_width
- *   NLI_TUNE_PM_VARIANT            how 9x9 PatchMatch reads candidate windows:
- *                                  0 (default) target window in shared memory,
- *                                  source rows by plain loads; 1 source windows
- *                                  staged in shared memory by tensor copies;
- *                                  2 target window in registers.  The fields
- *                                  are identical for all three.
+ *   NLI_TUNE_PM_VARIANT            how 9x9 PatchMatch works: 0 (default) groups
+ *                                  of up to three target points per warp, both
+ *                                  windows by plain loads; 1 one point per
+ *                                  warp, its window in shared memory and
+ *                                  source windows staged there by tensor
+ *                                  copies; 2 one point per warp, its window in
+ *                                  registers.  The fields are identical for
+ *                                  all three.
  *   NLI_TUNE_CG_PRECOND            NL-Poisson / NL-depth conjugate gradient:
  *                                  0 (default) plain CG as the reference
  *                                  (patch_non_local_poisson.cpp:387-477);
@@ -471,7 +473,8 @@ int nli_ctx_set_batch_width(nli_ctx *ctx, int width);
  *   NLI_TUNE_PM_TILE               how the persistent PatchMatch kernels
  *                                  share out the target points: n > 0 a
  *                                  device work queue from which each warp
- *                                  takes n consecutive points per atomic
+ *                                  takes n consecutive groups of points
+ *                                  (variants 1 and 2: points) per atomic
  *                                  grab (1..1024, default 1); 0 static
  *                                  ranges (block b takes the b-th contiguous
  *                                  range).  Identical fields.

@@ -94,6 +94,12 @@ struct Rng {
 	    : key(k), pixel(p), sweep(s), block(0), tag(0x6e6c6900u ^ (stream << 16)), used(4)
 	{
 	}
+	// block `block` of a stream: its draws 4 block .. 4 block + 3
+	static __device__ __forceinline__ uint4 block_of(uint2 key, uint32_t pixel, uint32_t sweep, uint32_t stream,
+	                                                 uint32_t block)
+	{
+		return philox(make_uint4(pixel, sweep, block, 0x6e6c6900u ^ (stream << 16)), key);
+	}
 	__device__ __forceinline__ uint32_t next()
 	{
 		if (used == 4) {

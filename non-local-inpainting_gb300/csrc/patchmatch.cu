@@ -134,7 +134,7 @@ __global__ void k_copy_targets_batch(const __grid_constant__ PmBatchArgs B)
 	if (!batch_on(B.active, T.flag)) return;
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < T.p.nt; i += gridDim.x * blockDim.x) {
 		const int pix = T.p.tlist[i];
-		T.nnf_x[pix] = T.nnf_y[pix];
+		T.nnf_x[pix] = T.io[0].nnf_out[pix];
 	}
 }
 
@@ -152,6 +152,7 @@ void patchmatch_batch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli
 	B.tile = ctx->tune_pm_tile;
 	int maxpix = 0, maxpad = 0, maxnt = 0;
 	long long total = 0;  // target points of all images
+	int widest = 0;       // the largest random-search window (as unsigned)
 	for (int i = 0; i < n; i++) {
 		const PmBatchItem &it = items[i];
 		NLI_REQUIRE(it.W < 32768 && it.H < 32768, NLI_E_UNSUPPORTED, "PatchMatch source sides must be below 32768");
@@ -189,15 +190,14 @@ void patchmatch_batch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli
 		T.img = it.img;
 		T.init = reinterpret_cast<const int2 *>(it.init);
 		T.nnf_x = reinterpret_cast<int2 *>(it.out);
-		T.nnf_y = reinterpret_cast<int2 *>(it.nnf_y);
-		T.dist_x = it.dist_x;
-		T.dist_y = it.dist_y;
-		T.hist_x = it.hist_x;
-		T.hist_y = it.hist_y;
+		const PmFields f = {T.nnf_x,   reinterpret_cast<int2 *>(it.nnf_y), it.dist_x, it.dist_y, it.hist_x, it.hist_y};
+		T.io[0] = f.io(0);
+		T.io[1] = f.io(1);
 		maxpix = max(maxpix, it.W * it.H);
 		maxpad = max(maxpad, (it.W + 1) * (it.H + 1));
 		maxnt = max(maxnt, it.nt);
 		total += it.nt;
+		widest = (int)std::max((unsigned)widest, (unsigned)p.max_window);
 	}
 	cudaStream_t s = ctx->stream;
 	const int per = 256;
@@ -217,12 +217,14 @@ void patchmatch_batch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli
 		B.queue = ctx->buf<unsigned>("pm.queue", slots);
 		NLI_CUDA(cudaMemsetAsync(B.queue, 0, sizeof(unsigned) * slots, s));
 	}
-	const int taps = a.px * a.py;
-	const PmShape shape = pm_shape(kPmShared, total, ctx->num_sms);
-	const size_t smem = pm_smem_bytes(taps, B.t[0].p.rows, B.t[0].p.L, shape.block / 32);
-	NLI_REQUIRE(smem <= (size_t)ctx->max_smem_optin, NLI_E_UNSUPPORTED, "PatchMatch shared memory too large");
+	B.group = pm_group(total, widest, ctx->num_sms);
+	long long groups = 0;
+	for (int i = 0; i < n; i++) {
+		B.t[i].p.group = B.group;
+		groups += (B.t[i].p.nt + B.group.points - 1) / B.group.points;
+	}
 	const bool handled = pm_dispatch(dp.kind, C, [&](auto d) {
-		d.batch(ctx, a, B, pm.iterations, shape, smem, counter);
+		d.batch(ctx, a, B, pm.iterations, groups, counter);
 	});
 	NLI_REQUIRE(handled, NLI_E_UNSUPPORTED, "no PatchMatch kernel for this distance / channel count");
 	if (pm.iterations % 2 == 1) {
@@ -339,6 +341,7 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 		p.dev = smom ? dev : 0;
 		p.queue = nullptr;
 		p.tile = ctx->tune_pm_tile;
+		p.group = {32, 1};  // run_sweeps chooses
 		if (p.tile > 0) {
 			const int slots = std::max(pm.iterations, 0) + 1;
 			p.queue = ctx->buf<unsigned>("pm.queue", slots);

@@ -20,20 +20,34 @@
 // channels, zero-filled), with one extra column and row that repeat the
 // last ones, so the forward differences u(x+1) - u(x) and u(y+1) - u(y) are
 // exactly 0 on the last column / row, as Gradient::calculate sets them
-// (gradient.cpp:37-63).  One warp works on one target point at a time
-// (persistent warps); its target window (patch + 1 column + 1 row) sits in
-// shared memory.  The warp's lanes are split into K = 32 / L sub-warps of
-// L = patch width + 1 lanes (3 sub-warps of 10 lanes for 9x9 patches); each
-// sub-warp evaluates one candidate, lane c walking down column c of the
-// candidate's window.  Per row a lane loads one float4, forms the colour
-// difference d = u_s - u_t, gets d of column c + 1 by a shuffle (x gradient
-// difference) and keeps the previous row's d in registers (y gradient
-// difference).  The gradient difference of the two patches is formed as a
-// difference of colour differences, (u_s(x+1) - u_t(x+1)) - (u_s(x) - u_t(x)),
-// which equals (gx_s - gx_t) up to float rounding.  The candidates of one
-// step (propagation, then random search) are gathered first, one per lane,
-// then evaluated K at a time and accepted in their sequential order with a
-// strict "<", so the result equals evaluating them one after the other.
+// (gradient.cpp:37-63).
+//
+// A warp works on a group of up to three target points at a time.  To
+// propose, its lanes are split evenly over the points (10, 16 or 32 lanes
+// each): a point's lanes each fetch one neighbour's match, or draw in one
+// random-search window, test it and drop it where the lower bound below
+// rules it out.  What survives goes into one list for the whole warp, in
+// the order of points and proposals.  To evaluate, the lanes are split into
+// K = 32 / L sub-warps of L = patch width + 1 lanes (3 sub-warps of 10 lanes
+// for 9x9 patches), and each round takes the next K entries of the list,
+// whichever points they belong to.  In a sub-warp lane c walks down column c
+// of the candidate's and the target's window: per row it loads one float4
+// of each, forms the colour difference d = u_s - u_t, gets d of column c + 1
+// by a shuffle (x gradient difference) and keeps the previous row's d in
+// registers (y gradient difference).  The gradient difference of the two
+// patches is formed as a difference of colour differences,
+// (u_s(x+1) - u_t(x+1)) - (u_s(x) - u_t(x)), which equals (gx_s - gx_t) up to
+// float rounding.  Results are accepted in the list's order with a strict
+// "<", so the field equals evaluating each point's candidates one after the
+// other, whatever the grouping.
+//
+// Why groups: in a run whose field has converged about two of a point's
+// eighteen proposals survive the bound, so one point filled two of the three
+// sub-warps in a round of its own, and its proposing (the random draws, the
+// mask tests and the bound, over 500 instructions) kept 8 to 10 of 32 lanes
+// busy.  Three points share both: a call on
+// 512 x 512 takes 1466 us instead of 1567, on 1013 x 887 5720 instead of 6847,
+// on 640 x 480 RGB-D 1695 instead of 2035 (figures of the bound by means).
 #pragma once
 
 #include <cuda.h>  // CUtensorMap (the descriptor type; encoded through the runtime's driver entry point)
@@ -103,35 +117,58 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 	    : "memory");
 }
 
-// How the fixed-size (9 x 9) kernels read a candidate's two windows
-// (NLI_TUNE_PM_VARIANT): kPmShared keeps the target window in shared memory
-// and loads source rows from global memory (32 warps per SM); kPmStaged also
-// copies the source windows into shared memory by tensor copies; kPmRegs
-// holds the lane's column of the target window in registers (16 warps per
-// SM, twice the registers).  All three evaluate the same candidates with the
-// same arithmetic.  Runtime-sized patches always use kPmShared.
-enum PmVariant { kPmShared = 0, kPmStaged = 1, kPmRegs = 2 };
+// How the fixed-size (9 x 9) kernels work (NLI_TUNE_PM_VARIANT): kPmGrouped
+// (the default, described above) takes groups of points and loads both
+// windows' rows from global memory.  The other two take one point per warp:
+// kPmStaged keeps the target window in shared memory and copies the source
+// windows there by tensor copies; kPmRegs holds the lane's column of the
+// target window in registers (16 warps per SM, twice the registers).  All
+// three evaluate the same candidates with the same arithmetic.
+// Runtime-sized patches and batches always use kPmGrouped.
+enum PmVariant { kPmGrouped = 0, kPmStaged = 1, kPmRegs = 2 };
 
 __host__ __device__ constexpr int pm_threads(int V) { return V == kPmRegs ? 512 : 1024; }
 
-// Launch shape of the persistent kernels for nt target points: one block per
-// SM, with just enough warps that every point has one (up to the variant's
-// most).  A point is one warp's serial chain of loads and evaluations, and a
-// sweep of a coarse level is bound by the warps that share an SM, so the
-// points are spread over all SMs first: a PatchMatch call on a 64 x 48 level
-// (500 points) took 348 us with full blocks on 16 SMs and takes 288 us with
-// 4 warps on each of 125; 130 x 81: 401 and 375 us.  From 32 points per SM
-// on, the shape is that of full blocks, which no smaller block beat.
+// Lanes per target point and points per warp when a warp proposes: enough
+// lanes for a call's random-search windows (max_window, max_window / 2, ...,
+// 1: 10 up to sides of 1023) and for its 8 neighbours.
+struct PmGroup {
+	int lanes, points;
+};
+
+// Launch shape of the persistent kernels for `items` work items (groups of
+// points, or points): one block per SM, with just enough warps that every
+// item has one (up to the variant's most).  An item is one warp's serial
+// chain of loads and evaluations, and a sweep of a coarse level is bound by
+// the warps that share an SM, so the items are spread over all SMs first: a
+// PatchMatch call on a 64 x 48 level (500 points) took 348 us with full
+// blocks on 16 SMs and 288 us with 4 warps on each of 125.
 struct PmShape {
 	int grid, block;
 };
 
-inline PmShape pm_shape(int V, long long nt, int num_sms)
+inline PmShape pm_shape(int threads, long long items, int num_sms)
 {
-	const int most = pm_threads(V) / 32;
-	const long long per_sm = (nt + num_sms - 1) / num_sms;
+	const int most = threads / 32;
+	const long long per_sm = (items + num_sms - 1) / num_sms;
 	const int warps = (int)std::max(1LL, std::min((long long)most, per_sm));
-	return {(int)std::min((long long)num_sms, (nt + warps - 1) / warps), 32 * warps};
+	return {(int)std::min((long long)num_sms, (items + warps - 1) / warps), 32 * warps};
+}
+
+// Groups for a call of nt points in all.  Several points per group take
+// fewer instructions per point but make a warp's chain of rounds longer, so
+// they pay once every SM has 16 groups: 512 x 512 (50 000 points) 1715 us a
+// call with one point per group and 1466 us with three, 276 x 167 RGB-D
+// (11 000) 569 and 510 us, but 64 x 48 (750) 296 and 416 us, 190 x 107 (6500)
+// 457 and 542 us.  The line lies near 7300 points: 8 or 24 groups per SM are
+// slower on calls of 4000 to 11 000 points.
+inline PmGroup pm_group(long long nt, int max_window, int num_sms)
+{
+	int windows = 0;
+	for (unsigned w = (unsigned)max_window; w; w >>= 1) windows++;
+	PmGroup g = windows <= 10 ? PmGroup{10, 3} : windows <= 16 ? PmGroup{16, 2} : PmGroup{32, 1};
+	while (g.points > 1 && nt < 16LL * num_sms * g.points) g.points--;
+	return g;
 }
 
 // Per-warp state of the staged path.
@@ -173,6 +210,7 @@ struct PmArgs {
 	// a warp takes `tile` consecutive target points per grab
 	unsigned *queue;
 	int tile;
+	PmGroup group;  // kPmGrouped
 };
 
 // Philox key of this PatchMatch call: the seed mixed with the call's index
@@ -189,14 +227,16 @@ struct Kind {
 	static constexpr bool grad = KIND == NLI_DIST_L2_COMBINED || KIND == NLI_DIST_L2_RGBD;
 };
 
-// The work items [0, n) of a persistent PatchMatch launch, visited by the
+// The work items [0, n) of a persistent PatchMatch launch (groups of target
+// points, single points in the variants that take them one by one), visited by the
 // calling warp (f(i) for each of its items, in increasing order).  Without
 // a queue, block b takes the contiguous range [b * chunk, (b + 1) * chunk)
 // and its warps interleave over it, so the warps of an SM work on
 // neighbouring points and share source neighbourhoods in L1.  With a queue
-// (`queue` a counter zeroed before the launch), each warp takes `tile`
-// consecutive items per atomic grab until the list is exhausted, so warps
-// that drew cheap points take more and no SM idles while others finish.
+// (`queue` a counter zeroed before the launch), each warp starts on the `tile`
+// items of its own number and then takes `tile` consecutive items per atomic
+// grab until the list is exhausted, so warps that drew cheap points take
+// more and no SM idles while others finish.
 // Every item's computation is independent of which warp does it and when
 // (the sweeps read the previous field and the random streams are keyed by
 // point), so both give the same field.
@@ -205,13 +245,14 @@ __device__ __forceinline__ void pm_for_each(int n, unsigned *queue, int tile, F 
 {
 	if (queue) {
 		const int lane = threadIdx.x & 31;
-		for (;;) {
-			unsigned base = 0u;
-			if (lane == 0) base = atomicAdd(queue, (unsigned)tile);
-			base = __shfl_sync(kFull, base, 0);
-			if (base >= (unsigned)n) break;
+		const unsigned warps = gridDim.x * (blockDim.x >> 5), taken = warps * (unsigned)tile;
+		unsigned base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (unsigned)tile;
+		while (base < (unsigned)n) {
 			const int stop = min(n, (int)base + tile);
 			for (int i = (int)base; i < stop; i++) f(i);
+			if (taken >= (unsigned)n) break;  // every item had a warp
+			if (lane == 0) base = taken + atomicAdd(queue, (unsigned)tile);
+			base = __shfl_sync(kFull, base, 0);
 		}
 	} else {
 		const int chunk = (n + gridDim.x - 1) / gridDim.x;
@@ -223,30 +264,31 @@ __device__ __forceinline__ void pm_for_each(int n, unsigned *queue, int tile, F 
 // A source centre is usable when it is in the source mask and its whole
 // patch lies in the image (the masks of the inpainting driver guarantee the
 // latter through their margin; user masks may not).
-__device__ __forceinline__ bool src_ok(const PmArgs &p, int x, int y)
+__device__ __forceinline__ bool src_inside(const PmArgs &p, int x, int y)
 {
-	return x >= p.rx && y >= p.ry && x + p.ex <= p.sW && y + p.ey <= p.sH &&
-	       nli_in_bounds((long long)y * p.sW + x, (long long)p.sW * p.sH, kSitePmMask) && p.smask[y * p.sW + x];
+	return x >= p.rx && y >= p.ry && x + p.ex <= p.sW && y + p.ey <= p.sH;
 }
+
+__device__ __forceinline__ bool src_masked(const PmArgs &p, int x, int y)
+{
+	return nli_in_bounds((long long)y * p.sW + x, (long long)p.sW * p.sH, kSitePmMask) && p.smask[y * p.sW + x];
+}
+
+__device__ __forceinline__ bool src_ok(const PmArgs &p, int x, int y) { return src_inside(p, x, y) && src_masked(p, x, y); }
 
 __device__ __forceinline__ bool tgt_patch_inside(const PmArgs &p, int x, int y)
 {
 	return x >= p.rx && y >= p.ry && x + p.ex <= p.tW && y + p.ey <= p.tH;
 }
 
-__device__ __forceinline__ bool tgt_ok(const PmArgs &p, int x, int y)
-{
-	return (unsigned)x < (unsigned)p.tW && (unsigned)y < (unsigned)p.tH && p.tmask[y * p.tW + x];
-}
-
 // Shared memory: per-tap weights (divided by the patch area) for all warps,
-// padded to a float4 boundary, then one target window of rows x L float4
-// per warp, then one 32-entry candidate list per warp.
+// padded to a float4 boundary, then one 32-entry candidate list and its
+// counts per warp (the staged variant's layout: pm_smem_bytes_tma).
 __host__ __device__ inline int pm_weight_slots(int taps) { return (taps + 3) / 4; }
 
-__host__ __device__ inline size_t pm_smem_bytes(int taps, int rows, int L, int warps)
+__host__ __device__ inline size_t pm_smem_bytes(int taps, int warps)
 {
-	return sizeof(float4) * ((size_t)pm_weight_slots(taps) + (size_t)warps * rows * L) + sizeof(int) * 32 * warps;
+	return sizeof(float4) * (size_t)pm_weight_slots(taps) + sizeof(int) * 36 * warps;
 }
 
 __device__ __forceinline__ void load_weights(const DistArgs &a, float *s_w)
@@ -257,22 +299,20 @@ __device__ __forceinline__ void load_weights(const DistArgs &a, float *s_w)
 	__syncthreads();
 }
 
-// The warp's target window: rows x L pixels starting at the patch corner.
-// With up to 3 channels the unused fourth component carries the tap's
-// weight (0 outside the patch), so the distance reads one float4 per row.
+// kPmStaged: the warp's target window, rows x L pixels starting at the patch
+// corner.  With up to 3 channels the unused fourth component carries the
+// tap's weight (0 outside the patch), so the distance reads one float4 per
+// row.
 template <int KIND, int C, int P>
 __device__ __forceinline__ void load_window(const PmArgs &p, const float *s_w, int x, int y, float4 *s_t)
 {
 	const int lane = threadIdx.x & 31;
-	// compiled sizes for P x P patches (a division by a constant), else the call's
-	constexpr int LP = P ? P + (Kind<KIND>::grad ? 1 : 0) : 1;
-	const int L = P ? LP : p.L, rows = P ? LP : p.rows;
-	const int px = P ? P : p.rx + p.ex, py = P ? P : p.ry + p.ey;
+	constexpr int L = P + (Kind<KIND>::grad ? 1 : 0);
 	const float4 *T = p.tgt + (size_t)(y - p.ry) * p.tWp + (x - p.rx);
-	for (int e = lane; e < rows * L; e += 32) {
-		const int r = P ? e / LP : e / L, c = e - r * L;
+	for (int e = lane; e < L * L; e += 32) {
+		const int r = e / L, c = e - r * L;
 		float4 v = __ldg(T + (size_t)r * p.tWp + c);
-		if (C <= 3) v.w = (r < py && c < px) ? s_w[r * px + c] : 0.f;
+		if (C <= 3) v.w = (r < P && c < P) ? s_w[r * P + c] : 0.f;
 		s_t[e] = v;
 	}
 	__syncwarp();
@@ -565,25 +605,41 @@ __device__ __forceinline__ void moments_span(const DistArgs &a, const float4 *__
 	if ((threadIdx.x & 31) == 0 && vm > 0.f) atomicMax(vmax, __float_as_uint(vm));
 }
 
-// Evaluates the n candidates held one per lane (packed x | y << 16, lane i
-// holds candidate i) against the target window s_t, in steps of K, and
-// accepts each in order when strictly better than the current match.  All
-// lanes return the same best / bd.  Once the rows summed so far reach the
-// current distance for every candidate of a step, the rest of the step is
-// skipped (exact: all terms are non-negative).  P > 0: square P x P patch
-// known at compile time (rows unrolled); P == 0: sizes from the arguments.
-// kPmStaged: the step's source windows are copied into the warp's slots
-// first (one tensor copy per candidate) and the rows are read from there.
-// kPmRegs: the target rows come from tw (registers) instead of s_t.
-template <int KIND, int C, int P, int V = kPmShared>
-__device__ __forceinline__ void eval_candidates(const PmArgs &p, const float *s_w, const float4 *s_t, int mycand,
-                                                int n, int2 &best, float &bd, unsigned &partial,
-                                                TmaState *ts = nullptr, const float4 *tw = nullptr)
+// Rows after which an evaluation is tested for early termination (counted
+// from 0): every term is non-negative, so once the rows summed so far reach
+// the current distance for every candidate of a round, the rest of the round
+// is skipped (exact).  9 x 9 L2 combined: after 4 of 10 rows.  Over the
+// 512 x 512 NL-Poisson process() without the lower bound that stops 57.5 %
+// of the candidates and was 1.6 % faster than a test at half the window
+// (65 % stopped); two tests (rows 5 and 7, or 3 and 5 and 7) cost more than
+// they save.
+template <int P, int G>
+__device__ __forceinline__ constexpr int check_row()
 {
-	constexpr bool TMA = V == kPmStaged;
+	return (P + G) / 2 - 2;
+}
+
+// A warp's counts in shared memory (kept by lane 0): candidates evaluated, of
+// these at their point's distance by the early test, points that propagation
+// improved; registers are what limits the warps per SM.
+struct PmCount {
+	unsigned evals, partial, improved, pad;
+};
+
+// Evaluates the list's n entries (candidate x | y << 15 | group << 30), K at a
+// time, and accepts each in order when strictly better than the match of
+// the point it belongs to.  A lane holds its own point's state: group index
+// g, target position txy (x | y << 16), match (as the list's, without the
+// group) and distance bd; lane g * lanes speaks for group g.  count->partial
+// takes the candidates that had reached their point's distance of before
+// the call at the early test (independent of how points are grouped).
+// P > 0: square P x P patch known at compile time (rows unrolled); P == 0:
+// sizes from the arguments.
+template <int KIND, int C, int P>
+__device__ __forceinline__ void eval_list(const PmArgs &p, const float *s_w, const unsigned *list, int n, int g,
+                                          unsigned txy, unsigned &match, float &bd, PmCount *count)
+{
 	constexpr bool G = Kind<KIND>::grad;
-	constexpr int PF = (C == 4) ? 1 : 2;  // rows of loads in flight (fewer for 4 channels: registers)
-	if (TMA && ts->map == nullptr) return;  // this warp's staging gave up (timeout flagged)
 	const int L = P ? P + G : p.L;
 	const int K = P ? 32 / (P + G) : p.K;
 	const int rows = P ? P + G : p.rows;
@@ -592,7 +648,123 @@ __device__ __forceinline__ void eval_candidates(const PmArgs &p, const float *s_
 	const int lane = threadIdx.x & 31;
 	const int sw = lane / L, c = lane - sw * L;
 	const bool tapcol = c < px;
-	const int check_row = rows / 2;
+	const float *W = s_w + c;
+	const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+	const float bd0 = bd;
+#pragma unroll 1
+	for (int b = 0; b < n; b += K) {
+		const int idx = b + sw;
+		const bool active = sw < K && idx < n;
+		// idle lanes repeat the round's first entry; nothing reads their sums
+		const unsigned e = list[active ? idx : b];
+		const int speaker = (int)(e >> 30) * p.group.lanes;
+		const int cx = (int)(e & 0x7fffu), cy = (int)((e >> 15) & 0x7fffu);
+		const unsigned t = __shfl_sync(kFull, txy, speaker);
+		const float bound = __shfl_sync(kFull, bd, speaker);
+		// this lane's pixel of the next row to load (sides below 32768: 31 bits)
+		int so = (cy - p.ry) * p.sWp + (cx - p.rx) + c;
+		int to = ((int)(t >> 16) - p.ry) * p.tWp + ((int)(t & 0xffffu) - p.rx) + c;
+		const int s_n = p.sWp * (p.sH + 1);
+		auto load_s = [&](float4 &v) {
+			// the lanes left over hold no column of a window
+			if (sw < K && nli_in_bounds(so, s_n, kSitePmSource)) v = __ldg(p.src + so);
+			so += p.sWp;
+		};
+		auto load_t = [&](float4 &v) {
+			if (sw < K) v = __ldg(p.tgt + to);
+			to += p.tWp;
+		};
+		// source rows in flight (fewer for 4 channels: registers); the target's
+		// window is the warp's own and in L1 after the first candidate
+		constexpr int PF = C == 4 ? 1 : 2;
+		float4 v[PF], u = zero;
+#pragma unroll
+		for (int r = 0; r < PF; r++) {
+			v[r] = zero;
+			if (r < rows) load_s(v[r]);
+		}
+		load_t(u);
+		float4 dp = zero;
+		float wp = 0.f;
+		Acc A = {0.f, 0.f, 0.f, 0.f};
+		bool stop = false;
+		auto row = [&](int r, float4 &vr) {
+			const float4 d = subc<C>(vr, u);
+			const bool tap = tapcol && r < py;
+			const float w = tap ? W[r * px] : 0.f;
+			if (r + PF < rows) load_s(vr);
+			if (r + 1 < rows) load_t(u);
+			row_terms<KIND, C>(d, dp, w, wp, tap, G && tapcol && r > 0, A);
+			dp = d;
+			wp = w;
+		};
+		auto check = [&]() {
+			const float part = subwarp_sum(combine<KIND>(A, p), c, L);
+			const float start = __shfl_sync(kFull, bd0, speaker);
+			const unsigned reached = __ballot_sync(kFull, active && c == 0 && part >= start);
+			if (reached && lane == 0) count->partial += __popc(reached);
+			return __all_sync(kFull, !active || c != 0 || part >= bound);
+		};
+		if constexpr (P > 0) {
+#pragma unroll
+			for (int r = 0; r < P + G; r++) {
+				row(r, v[r % PF]);
+				if (r == check_row<P, G>() && check()) {
+					stop = true;
+					break;
+				}
+			}
+		} else {
+#pragma unroll 1
+			for (int r0 = 0; r0 < rows && !stop; r0 += PF) {
+#pragma unroll
+				for (int i = 0; i < PF; i++) {
+					const int r = r0 + i;
+					if (r >= rows) break;
+					row(r, v[i]);
+					if (r == rows / 2 && check()) {
+						stop = true;
+						break;
+					}
+				}
+			}
+		}
+		if (stop) continue;
+		const float sum = subwarp_sum(combine<KIND>(A, p), c, L);
+		const int in_round = min(K, n - b);
+#pragma unroll 1
+		for (int s = 0; s < in_round; s++) {
+			const float ds = __shfl_sync(kFull, sum, s * L);
+			const unsigned es = __shfl_sync(kFull, e, s * L);
+			if ((int)(es >> 30) == g && ds < bd) {
+				bd = ds;
+				match = es & 0x3fffffffu;
+			}
+		}
+	}
+}
+
+// The one-point variants: evaluates the n candidates held one per lane (packed
+// x | y << 16, lane i holds candidate i) in steps of K and accepts each in
+// order when strictly better than the current match.  All lanes return the
+// same best / bd.  kPmStaged: the step's source windows are copied into the
+// warp's slots first (one tensor copy per candidate) and the rows are read
+// from there, the target rows from s_t.  kPmRegs: the source rows are plain
+// loads and the target rows come from tw (registers).
+template <int KIND, int C, int P, int V>
+__device__ __forceinline__ void eval_candidates(const PmArgs &p, const float *s_w, const float4 *s_t, int mycand,
+                                                int n, int2 &best, float &bd, unsigned &partial, TmaState *ts,
+                                                const float4 *tw)
+{
+	static_assert(P > 0 && V != kPmGrouped, "compiled for fixed patch sizes");
+	constexpr bool TMA = V == kPmStaged;
+	constexpr bool G = Kind<KIND>::grad;
+	constexpr int PF = (C == 4) ? 1 : 2;
+	constexpr int L = P + G, K = 32 / L, rows = P + G;
+	if (TMA && ts->map == nullptr) return;  // this warp's staging gave up (timeout flagged)
+	const int lane = threadIdx.x & 31;
+	const int sw = lane / L, c = lane - sw * L;
+	const bool tapcol = c < P;
 	const size_t sWp = (size_t)p.sWp;
 	const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
@@ -615,18 +787,16 @@ __device__ __forceinline__ void eval_candidates(const PmArgs &p, const float *s_
 		const float *Wt = s_w + c;
 		const float4 *Sl = nullptr;  // this lane's column of its candidate's staged window
 		if constexpr (TMA) {
-			static_assert(P > 0, "the staged path is compiled for fixed patch sizes");
-			constexpr int KC = 32 / (P + G);
 			const int nact = min(K, n - b);
-			int cs[KC];
+			int cs[K];
 #pragma unroll
-			for (int s = 0; s < KC; s++) cs[s] = __shfl_sync(kFull, mycand, min(b + s, 31));
+			for (int s = 0; s < K; s++) cs[s] = __shfl_sync(kFull, mycand, min(b + s, 31));
 			__syncwarp();
 			if (lane == 0) {
 				fence_proxy_async();
 				mbar_expect_tx(ts->bar, (unsigned)(nact * rows * L * sizeof(float4)));
 #pragma unroll
-				for (int s = 0; s < KC; s++)
+				for (int s = 0; s < K; s++)
 					if (s < nact)
 						tma_load_2d(ts->slots + s * ts->slot_stride, ts->map, 4 * ((cs[s] & 0xffff) - p.rx),
 						            (cs[s] >> 16) - p.ry, ts->bar);
@@ -644,7 +814,7 @@ __device__ __forceinline__ void eval_candidates(const PmArgs &p, const float *s_
 			Sl = ts->slots + (active ? sw : 0) * ts->slot_stride + c;
 		}
 		float4 v0 = (!TMA && active) ? ldrow(0) : zero;
-		float4 v1 = (!TMA && PF == 2 && active && rows > 1) ? ldrow(1) : zero;
+		float4 v1 = (!TMA && PF == 2 && active) ? ldrow(1) : zero;
 		float4 dp = zero;
 		float wp = 0.f;
 		Acc A = {0.f, 0.f, 0.f, 0.f};
@@ -666,8 +836,8 @@ __device__ __forceinline__ void eval_candidates(const PmArgs &p, const float *s_
 			else
 				t = T[r * L];
 			const float4 d = subc<C>(v, t);
-			const bool tap = act_col && r < py;
-			const float w = (C <= 3) ? t.w : (tap ? Wt[r * px] : 0.f);
+			const bool tap = act_col && r < P;
+			const float w = (C <= 3) ? t.w : (tap ? Wt[r * P] : 0.f);
 			row_terms<KIND, C>(d, dp, w, wp, tap, G && act_col && r > 0, A);
 			dp = d;
 			wp = w;
@@ -676,31 +846,12 @@ __device__ __forceinline__ void eval_candidates(const PmArgs &p, const float *s_
 			const float part = subwarp_sum(combine<KIND>(A, p), c, L);
 			return __all_sync(kFull, !active || c != 0 || part >= bound);
 		};
-		if constexpr (P > 0) {
-			// one test after the first (P + G) / 2 - 1 rows (4 of 10 for 9x9
-			// L2 combined).  On the 512x512 benchmark without the lower bound
-			// it stops 57.5 % of the candidates and is 1.6 % faster than a
-			// test at half the window (65 % stopped); two tests (rows 5 and 7,
-			// or 3 and 5 and 7) cost more than they save.  With the bound,
-			// tests after rows 5, 6 or 7, or after 4 and 7, take the same
-			// time within 0.3 %
-			constexpr int kCheckRow = (P + G) / 2 - 2;
 #pragma unroll
-			for (int r = 0; r < P + G; r++) {
-				row(r);
-				if (r == kCheckRow && check()) {
-					stop = true;
-					break;
-				}
-			}
-		} else {
-#pragma unroll 1
-			for (int r = 0; r < rows; r++) {
-				row(r);
-				if (r == check_row && check()) {
-					stop = true;
-					break;
-				}
+		for (int r = 0; r < rows; r++) {
+			row(r);
+			if (r == check_row<P, G>() && check()) {
+				stop = true;
+				break;
 			}
 		}
 		const int in_step = min(K, n - b);
@@ -742,11 +893,11 @@ __device__ __forceinline__ int compact_candidates(bool valid, int packed, const 
 }
 
 // Shared memory of the PatchMatch kernels: per-tap weights, then per warp a
-// target window (rows x L float4) and a candidate list (32 ints).
+// candidate list (32 ints).
 struct PmSmem {
 	float *w;
-	float4 *t;
 	int *list;
+	float4 *t;      // staged path: the target window, rows x L float4
 	float4 *slots;  // staged path: K windows per warp
 	int slot_stride;
 	uint64_t *bar;
@@ -771,13 +922,13 @@ template <int V>
 __device__ __forceinline__ PmSmem pm_smem(const DistArgs &a, const PmArgs &p)
 {
 	extern __shared__ float4 s_pm[];
-	const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+	const int warp = threadIdx.x >> 5;
 	PmSmem m;
 	const int ws = pm_weight_slots(a.px * a.py);
 	if (V != kPmStaged) {
 		m.w = reinterpret_cast<float *>(s_pm);
-		m.t = s_pm + ws + warp * p.rows * p.L;
-		m.list = reinterpret_cast<int *>(s_pm + ws + warps * p.rows * p.L) + warp * 32;
+		m.t = nullptr;
+		m.list = reinterpret_cast<int *>(s_pm + ws) + warp * 36;
 		m.slots = nullptr;
 		m.slot_stride = 0;
 		m.bar = nullptr;
@@ -795,9 +946,25 @@ __device__ __forceinline__ PmSmem pm_smem(const DistArgs &a, const PmArgs &p)
 	return m;
 }
 
+// A target point's seed match (patch_match.cpp:341-381): the init field's
+// where it lies in the source, otherwise redrawn uniformly up to `shots`
+// times; (x, y) where !src_ok remains when the draws run out.
+__device__ __forceinline__ int2 seed_match(const PmArgs &p, const uint2 key, int pix, const int2 *__restrict__ init)
+{
+	Rng rng(key, (uint32_t)pix, 0xffffffffu);
+	int2 n = init ? init[pix] : make_int2(-1, -1);
+	int tries = 0;
+	while (!src_ok(p, n.x, n.y) && tries < p.shots) {
+		n.x = rng.below(p.sW);
+		n.y = rng.below(p.sH);
+		tries++;
+	}
+	return n;
+}
+
 // One target point of the initial field (patch_match.cpp:329-381): its
-// seed match (the init field's, else random draws), and that match's
-// distance.  Called by one whole warp; lane 0 writes the results.
+// seed match and that match's distance.  Called by one whole warp; lane 0
+// writes the results.
 template <int KIND, int C, int P, int V>
 __device__ __forceinline__ void pm_init_point(const PmArgs &p, const PmSmem &m, TmaState &ts, float4 *tw,
                                               const uint2 key, int pix, const int2 *__restrict__ init,
@@ -807,24 +974,7 @@ __device__ __forceinline__ void pm_init_point(const PmArgs &p, const PmSmem &m, 
 	const int lane = threadIdx.x & 31;
 	if (!nli_in_bounds(pix, (long long)p.tW * p.tH, kSitePmTarget)) return;
 	const int x = pix % p.tW, y = pix / p.tW;
-	Rng rng(key, (uint32_t)pix, 0xffffffffu);
-	int2 n = init ? init[pix] : make_int2(-1, -1);
-	int tries = 0;
-	// patch_match.cpp:341-381: keep a seed match that lies in the
-	// source, otherwise redraw it uniformly up to `shots` times
-	if (init) {
-		while (!src_ok(p, n.x, n.y) && tries < p.shots) {
-			n.x = rng.below(p.sW);
-			n.y = rng.below(p.sH);
-			tries++;
-		}
-	} else {
-		while ((n.x < 0 || !src_ok(p, n.x, n.y)) && tries < p.shots) {
-			n.x = rng.below(p.sW);
-			n.y = rng.below(p.sH);
-			tries++;
-		}
-	}
+	const int2 n = seed_match(p, key, pix, init);
 	float d = FLT_MAX;
 	int2 best = make_int2(-1, -1);
 	if (src_ok(p, n.x, n.y) && tgt_patch_inside(p, x, y)) {
@@ -865,6 +1015,29 @@ __global__ void __launch_bounds__(pm_threads(V), 1) k_pm_init(DistArgs a, PmArgs
 	}
 }
 
+// What one sweep reads and writes.
+struct PmIo {
+	const int2 *nnf_in;
+	const float *dist_in;
+	const uint8_t *hist_in;
+	int2 *nnf_out;
+	float *dist_out;
+	uint8_t *hist_out;
+};
+
+// A call's field, distances and change histories (seen_before), each twice:
+// sweep s reads x and writes y when s is even, the other way round when odd.
+struct PmFields {
+	int2 *nnf_x, *nnf_y;
+	float *dist_x, *dist_y;
+	uint8_t *hist_x, *hist_y;
+	PmIo io(int sweep) const
+	{
+		return (sweep % 2) == 0 ? PmIo{nnf_x, dist_x, hist_x, nnf_y, dist_y, hist_y}
+		                        : PmIo{nnf_y, dist_y, hist_y, nnf_x, dist_x, hist_x};
+	}
+};
+
 // Whether a neighbour's proposal needs no evaluation because the same
 // proposal was already tried for this point in this call.  Bit i of a
 // point's history says whether sweep s - 1 - i changed its match.  The
@@ -877,82 +1050,115 @@ __global__ void __launch_bounds__(pm_threads(V), 1) k_pm_init(DistArgs a, PmArgs
 // On the 512 x 512 NL-Poisson process() this takes the evaluations from 1.09
 // to 0.69 x 10^9 and the run from 724 to 657 ms; a first call from random
 // matches on 512 x 512 goes from 1706 to 1567 us.
-__device__ __forceinline__ bool seen_before(const uint8_t *__restrict__ hist, int neighbour, int sweep, bool at_jump)
+__device__ __forceinline__ bool seen_before(unsigned hist, int sweep, bool at_jump)
 {
-	if (at_jump) return sweep >= 4 && (hist[neighbour] & 15u) == 0u;
-	return sweep >= 1 && (hist[neighbour] & 1u) == 0u;
+	return at_jump ? sweep >= 4 && (hist & 15u) == 0u : sweep >= 1 && (hist & 1u) == 0u;
 }
 
-// One target point of a sweep: propagation from the previous sweep's
-// field, then random search around the best match.  Called by one whole
-// warp; lane 0 writes the results.
+// Whether (cx, cy) is a usable source centre that the lower bound does not
+// rule out for target (x, y).  Usable centres are nearly all of those
+// proposed, so the bound's loads are issued beside the mask's.
+template <int KIND, int C>
+__device__ __forceinline__ bool src_takes(const PmArgs &p, int x, int y, int cx, int cy, float bd)
+{
+	if (!src_inside(p, cx, cy)) return false;
+	const bool usable = src_masked(p, cx, cy);
+	const bool rejected = p.smom && bound_rejects<KIND, C>(p, x, y, cx, cy, bd);
+	return usable && !rejected;
+}
+
+// Proposal k (0-7) of a point's propagation step: the match of neighbour
+// k & 3 (left, right, up, down) at distance 1 (k < 4) or at the jump distance,
+// shifted back by the neighbour's offset.  False when there is none to
+// evaluate.
+template <int KIND, int C>
+__device__ __forceinline__ bool propagated(const PmArgs &p, int x, int y, int k, int sweep, int jump,
+                                           const PmIo &io, float bd, int &cx, int &cy)
+{
+	const int s = (k < 4) ? 1 : jump, side = k & 3;
+	const int nx = x + ((side == 0) ? -s : (side == 1) ? s : 0);
+	const int ny = y + ((side == 2) ? -s : (side == 3) ? s : 0);
+	// the loads of a step are issued together (a point is a chain of them):
+	// outside the image, where nothing is proposed, they read the point itself
+	const bool in = (unsigned)nx < (unsigned)p.tW && (unsigned)ny < (unsigned)p.tH;
+	const int at = in ? ny * p.tW + nx : y * p.tW + x;
+	if (!nli_in_bounds(at, (long long)p.tW * p.tH, kSitePmField)) return false;
+	const uint8_t target = p.tmask[at];
+	const int2 q = io.nnf_in[at];
+	const unsigned hist = sweep ? io.hist_in[at] : 0u;
+	if (!in || !target || q.x < 0 || seen_before(hist, sweep, k >= 4)) return false;
+	cx = q.x + (x - nx);
+	cy = q.y + (y - ny);
+	return src_takes<KIND, C>(p, x, y, cx, cy, bd);
+}
+
+// Proposal k of a point's random search around its match (bx, by): up to
+// `shots` draws in window max_window >> k from the proposal's own stream, the
+// first that lands in the source.  False when there is none to evaluate.
+// One Philox block holds two draws; which draw of its stream a proposal ends
+// on depends on the draws alone.
+template <int KIND, int C>
+__device__ __forceinline__ bool drawn(const PmArgs &p, const uint2 key, int pix, int x, int y, int bx, int by, int k,
+                                      int sweep, float bd, int &cx, int &cy, int &max_shot)
+{
+	const int w = p.max_window >> k;
+	const int x_min = max(bx - w, 0), y_min = max(by - w, 0);
+	const uint32_t nx = (uint32_t)(min(bx + w + 1, p.sW) - x_min), ny = (uint32_t)(min(by + w + 1, p.sH) - y_min);
+#pragma unroll 1
+	for (int t = 0; t < p.shots; t += 2) {
+		const uint4 u = Rng::block_of(key, (uint32_t)pix, (uint32_t)sweep, (uint32_t)k, (uint32_t)t >> 1);
+		cx = x_min + (int)__umulhi(u.x, nx);
+		cy = y_min + (int)__umulhi(u.y, ny);
+		bool ok = src_ok(p, cx, cy);
+		int shot = t;
+		if (!ok && t + 1 < p.shots) {
+			cx = x_min + (int)__umulhi(u.z, nx);
+			cy = y_min + (int)__umulhi(u.w, ny);
+			ok = src_ok(p, cx, cy);
+			shot = t + 1;
+		}
+		if (ok) {
+			max_shot = max(max_shot, shot);
+			return !(p.smom && bound_rejects<KIND, C>(p, x, y, cx, cy, bd));
+		}
+	}
+	return false;
+}
+
+// The one-point variants' target point of a sweep: propagation from the
+// previous sweep's field, then random search around the best match.  Called
+// by one whole warp; lane 0 writes the results.
 template <int KIND, int C, int P, int V>
 __device__ __forceinline__ void pm_sweep_point(const PmArgs &p, const PmSmem &m, TmaState &ts, float4 *tw,
                                                const uint2 key, int windows, int pix, int sweep, int jump,
-                                               const int2 *__restrict__ nnf_in, const float *__restrict__ dist_in,
-                                               const uint8_t *__restrict__ hist_in, int2 *__restrict__ nnf_out,
-                                               float *__restrict__ dist_out, uint8_t *__restrict__ hist_out,
+                                               const PmIo &io,
                                                unsigned &evals, unsigned &partial, unsigned &improved, int &max_shot)
 {
 	const int lane = threadIdx.x & 31;
 	if (!nli_in_bounds(pix, (long long)p.tW * p.tH, kSitePmTarget)) return;
 	const int x = pix % p.tW, y = pix / p.tW;
-	int2 best = nnf_in[pix];
-	float bd = dist_in[pix];
+	int2 best = io.nnf_in[pix];
+	float bd = io.dist_in[pix];
 	const float bd_in = bd;
-	const unsigned hist = sweep ? hist_in[pix] : 0u;
+	const unsigned hist = sweep ? io.hist_in[pix] : 0u;
 	if (tgt_patch_inside(p, x, y)) {
 		if constexpr (V == kPmRegs)
 			load_window_regs<KIND, C, P>(p, m.w, x, y, tw);
 		else
 			load_window<KIND, C, P>(p, m.w, x, y, m.t);
-		const bool bounded = p.smom != nullptr;
-		// propagation: lane 4s + k proposes the match of neighbour k
-		// (left, right, up, down) at distance 1 (s = 0) or at the jump
-		// distance (s = 1), shifted back by the neighbour's offset
-		bool valid = false;
-		int packed = 0;
-		if (lane < (jump > 1 ? 8 : 4)) {
-			const int s = (lane < 4) ? 1 : jump, k = lane & 3;
-			const int nx = x + ((k == 0) ? -s : (k == 1) ? s : 0);
-			const int ny = y + ((k == 2) ? -s : (k == 3) ? s : 0);
-			if (tgt_ok(p, nx, ny) && nli_in_bounds((long long)ny * p.tW + nx, (long long)p.tW * p.tH, kSitePmField)) {
-				const int2 q = nnf_in[ny * p.tW + nx];
-				if (q.x >= 0 && !seen_before(hist_in, ny * p.tW + nx, sweep, lane >= 4)) {
-					const int cx = q.x + (x - nx), cy = q.y + (y - ny);
-					valid = src_ok(p, cx, cy) && !(bounded && bound_rejects<KIND, C>(p, x, y, cx, cy, bd));
-					packed = cx | (cy << 16);
-				}
-			}
-		}
+		int cx = 0, cy = 0;
+		bool valid = lane < (jump > 1 ? 8 : 4) &&
+		             propagated<KIND, C>(p, x, y, lane, sweep, jump, io, bd, cx, cy);
 		int mycand;
-		int n = compact_candidates(valid, packed, best, m.list, mycand);
+		int n = compact_candidates(valid, cx | (cy << 16), best, m.list, mycand);
 		evals += n;
 		const float bd_before = bd;
 		eval_candidates<KIND, C, P, V>(p, m.w, m.t, mycand, n, best, bd, partial, &ts, tw);
 		if (bd < bd_before) improved++;
-		// random search around the match after propagation: lane k draws
-		// in window max_window >> k from its own stream, up to `shots`
-		// draws, and proposes the first that lands in the source
-		valid = false;
-		if (lane < windows) {
-			const int w = p.max_window >> lane;
-			const int x_min = max(best.x - w, 0), y_min = max(best.y - w, 0);
-			const int x_max = min(best.x + w + 1, p.sW), y_max = min(best.y + w + 1, p.sH);
-			Rng rng(key, (uint32_t)pix, (uint32_t)sweep, (uint32_t)lane);
-#pragma unroll 1
-			for (int t = 0; t < p.shots; t++) {
-				const int rx = x_min + rng.below(x_max - x_min);
-				const int ry = y_min + rng.below(y_max - y_min);
-				if (src_ok(p, rx, ry)) {
-					valid = !(bounded && bound_rejects<KIND, C>(p, x, y, rx, ry, bd));
-					packed = rx | (ry << 16);
-					max_shot = max(max_shot, t);
-					break;
-				}
-			}
-		}
-		n = compact_candidates(valid, packed, best, m.list, mycand);
+		cx = cy = 0;
+		valid = lane < windows &&
+		        drawn<KIND, C>(p, key, pix, x, y, best.x, best.y, lane, sweep, bd, cx, cy, max_shot);
+		n = compact_candidates(valid, cx | (cy << 16), best, m.list, mycand);
 		evals += n;
 		eval_candidates<KIND, C, P, V>(p, m.w, m.t, mycand, n, best, bd, partial, &ts, tw);
 		__syncwarp();
@@ -961,10 +1167,192 @@ __device__ __forceinline__ void pm_sweep_point(const PmArgs &p, const PmSmem &m,
 		bd = FLT_MAX;
 	}
 	if (lane == 0) {
-		nnf_out[pix] = best;
-		dist_out[pix] = bd;
+		io.nnf_out[pix] = best;
+		io.dist_out[pix] = bd;
 		// a match changes only together with a strictly smaller distance
-		hist_out[pix] = (uint8_t)((hist << 1) | (bd < bd_in ? 1u : 0u));
+		io.hist_out[pix] = (uint8_t)((hist << 1) | (bd < bd_in ? 1u : 0u));
+	}
+}
+
+// ------------------------------------------------------ groups of points
+// A lane's place in its warp's group: point g, lane k of that point's.
+struct PmLane {
+	int g, k;
+};
+
+__device__ __forceinline__ PmLane pm_lane(const PmGroup &group)
+{
+	const int lane = threadIdx.x & 31;
+	const int g = lane / group.lanes;
+	return {g, lane - g * group.lanes};
+}
+
+constexpr unsigned kNoMatch = 0xffffffffu;
+
+// The counts behind a warp's list.
+__device__ __forceinline__ PmCount *pm_count(unsigned *list) { return reinterpret_cast<PmCount *>(list + 32); }
+
+__device__ __forceinline__ void pm_count_clear(unsigned *list)
+{
+	if ((threadIdx.x & 31) < 4) list[32 + (threadIdx.x & 31)] = 0u;
+	__syncwarp();
+}
+
+// The warp's list of proposals (one per lane at most, packed x | y << 15 with
+// the group above): those that are valid, differ from their point's match and
+// from every lower lane's for the same point.  Returns their number.
+__device__ __forceinline__ int list_proposals(bool valid, unsigned packed, unsigned match, int g, unsigned *list)
+{
+	const int lane = threadIdx.x & 31;
+	const unsigned below = (1u << lane) - 1u;
+	valid = valid && packed != match;
+	const unsigned entry = packed | ((unsigned)g << 30);
+	const unsigned vmask = __ballot_sync(kFull, valid);
+	if (vmask == 0) return 0;
+	const unsigned same = __match_any_sync(kFull, valid ? entry : kNoMatch);
+	const bool keep = valid && (same & vmask & below) == 0;
+	const unsigned kmask = __ballot_sync(kFull, keep);
+	__syncwarp();
+	if (keep) list[__popc(kmask & below)] = entry;
+	if (lane == 0) pm_count(list)->evals += __popc(kmask);
+	__syncwarp();
+	return __popc(kmask);
+}
+
+// Points [first, first + group.points) of the initial field.
+template <int KIND, int C, int P>
+__device__ __forceinline__ void pm_init_group(const PmArgs &p, const float *s_w, unsigned *list, const PmLane at,
+                                              const uint2 key, int first, const int2 *__restrict__ init,
+                                              int2 *__restrict__ nnf, float *__restrict__ dist)
+{
+	PmCount *count = pm_count(list);
+	bool has = at.g < p.group.points && first + at.g < p.nt;
+	const int pix = has ? p.tlist[first + at.g] : 0;
+	has = has && nli_in_bounds(pix, (long long)p.tW * p.tH, kSitePmTarget);
+	const int x = pix % p.tW, y = pix / p.tW;
+	int2 n = make_int2(0, 0);
+	bool valid = false;
+	if (has) {
+		n = seed_match(p, key, pix, init);
+		valid = src_ok(p, n.x, n.y) && tgt_patch_inside(p, x, y);
+	}
+	unsigned match = kNoMatch;
+	float d = FLT_MAX;
+	const int listed = list_proposals(valid && at.k == 0, (unsigned)n.x | ((unsigned)n.y << 15), match, at.g, list);
+	eval_list<KIND, C, P>(p, s_w, list, listed, at.g, (unsigned)x | ((unsigned)y << 16), match, d, count);
+	if (has && at.k == 0) {
+		nnf[pix] = match == kNoMatch ? make_int2(-1, -1) : make_int2(match & 0x7fffu, match >> 15);
+		dist[pix] = d;
+	}
+}
+
+// Points [first, first + group.points) of a sweep: propagation from the
+// previous sweep's field, then random search around each point's match.
+template <int KIND, int C, int P>
+__device__ __forceinline__ void pm_sweep_group(const PmArgs &p, const float *s_w, unsigned *list, const PmLane at,
+                                               const uint2 key, int windows, int first, int sweep, int jump,
+                                               const PmIo &io,
+                                               int &max_shot)
+{
+	PmCount *count = pm_count(list);
+	bool has = at.g < p.group.points && first + at.g < p.nt;
+	const int pix = has ? p.tlist[first + at.g] : 0;
+	has = has && nli_in_bounds(pix, (long long)p.tW * p.tH, kSitePmTarget);
+	const int x = pix % p.tW, y = pix / p.tW;
+	const unsigned txy = (unsigned)x | ((unsigned)y << 16);
+	const bool inside = has && tgt_patch_inside(p, x, y);
+	unsigned match = kNoMatch;
+	float bd = FLT_MAX;
+	if (inside) {
+		const int2 q = io.nnf_in[pix];
+		if (q.x >= 0) match = (unsigned)q.x | ((unsigned)q.y << 15);
+		bd = io.dist_in[pix];
+	}
+	const float bd_in = bd;
+	int cx = 0, cy = 0;
+	bool valid = inside && at.k < (jump > 1 ? 8 : 4) &&
+	             propagated<KIND, C>(p, x, y, at.k, sweep, jump, io, bd, cx, cy);
+	int n = list_proposals(valid, (unsigned)cx | ((unsigned)cy << 15), match, at.g, list);
+	if (n) {
+		eval_list<KIND, C, P>(p, s_w, list, n, at.g, txy, match, bd, count);
+		const unsigned better = __ballot_sync(kFull, at.k == 0 && bd < bd_in);
+		if (better && at.g == 0 && at.k == 0) count->improved += __popc(better);
+	}
+	const int bx = match == kNoMatch ? -1 : (int)(match & 0x7fffu), by = match == kNoMatch ? -1 : (int)(match >> 15);
+	cx = cy = 0;
+	valid = inside && at.k < windows &&
+	        drawn<KIND, C>(p, key, pix, x, y, bx, by, at.k, sweep, bd, cx, cy, max_shot);
+	n = list_proposals(valid, (unsigned)cx | ((unsigned)cy << 15), match, at.g, list);
+	eval_list<KIND, C, P>(p, s_w, list, n, at.g, txy, match, bd, count);
+	if (has && at.k == 0) {
+		io.nnf_out[pix] = match == kNoMatch ? make_int2(-1, -1) : make_int2(match & 0x7fffu, match >> 15);
+		io.dist_out[pix] = bd;
+		// a match changes only together with a strictly smaller distance
+		const unsigned hist = sweep ? io.hist_in[pix] : 0u;
+		io.hist_out[pix] = (uint8_t)((hist << 1) | (inside && bd < io.dist_in[pix] ? 1u : 0u));
+	}
+}
+
+// Adds a warp's candidate counts to `counter` (and to `image`'s, if given).
+__device__ __forceinline__ void pm_count_add(unsigned *list, unsigned long long *counter, unsigned long long *image)
+{
+	const PmCount *c = pm_count(list);
+	if ((threadIdx.x & 31) == 0 && c->evals) {
+		atomicAdd(counter, (unsigned long long)c->evals);
+		if (c->partial) atomicAdd(counter + 1, (unsigned long long)c->partial);
+		if (image) {
+			atomicAdd(image, (unsigned long long)c->evals);
+			if (c->partial) atomicAdd(image + 1, (unsigned long long)c->partial);
+		}
+	}
+	__syncwarp();
+}
+
+template <int KIND, int C, int P>
+__global__ void __launch_bounds__(pm_threads(kPmGrouped), 1)
+    k_pm_init_grouped(DistArgs a, PmArgs p, const int2 *__restrict__ init, int2 *__restrict__ nnf,
+                      float *__restrict__ dist, unsigned long long *counter)
+{
+	const PmSmem m = pm_smem<kPmGrouped>(a, p);
+	load_weights(a, m.w);
+	const uint2 key = pm_key(p);
+	const PmLane at = pm_lane(p.group);
+	unsigned *list = reinterpret_cast<unsigned *>(m.list);
+	pm_count_clear(list);
+	const int groups = (p.nt + p.group.points - 1) / p.group.points;
+	pm_for_each(groups, p.queue, p.tile, [&](int i) {
+		pm_init_group<KIND, C, P>(p, m.w, list, at, key, i * p.group.points, init, nnf, dist);
+	});
+	pm_count_add(list, counter, nullptr);
+}
+
+// metric_prop (may be NULL): this sweep's count of target points that the
+// propagation step improved; metric_shots (may be NULL): the largest index
+// of a first accepted random draw (patch_match.cpp:452-456, 481-485).
+template <int KIND, int C, int P>
+__global__ void __launch_bounds__(pm_threads(kPmGrouped), 1)
+    k_pm_sweep_grouped(DistArgs a, PmArgs p, int sweep, int jump, PmIo io, unsigned long long *counter, unsigned long long *metric_prop, int *metric_shots)
+{
+	const int lane = threadIdx.x & 31;
+	const PmSmem m = pm_smem<kPmGrouped>(a, p);
+	load_weights(a, m.w);
+	const uint2 key = pm_key(p);
+	const PmLane at = pm_lane(p.group);
+	unsigned *list = reinterpret_cast<unsigned *>(m.list);
+	pm_count_clear(list);
+	int max_shot = -1;
+	// number of random-search windows: max_window, max_window / 2, ..., 1
+	const int windows = 32 - __clz(p.max_window);
+	const int groups = (p.nt + p.group.points - 1) / p.group.points;
+	pm_for_each(groups, p.queue ? p.queue + 1 + sweep : nullptr, p.tile, [&](int i) {
+		pm_sweep_group<KIND, C, P>(p, m.w, list, at, key, windows, i * p.group.points, sweep, jump, io, max_shot);
+	});
+	pm_count_add(list, counter, nullptr);
+	if (metric_prop && lane == 0 && pm_count(list)->improved)
+		atomicAdd(metric_prop, (unsigned long long)pm_count(list)->improved);
+	if (metric_shots) {
+		max_shot = __reduce_max_sync(kFull, max_shot);
+		if (lane == 0 && max_shot >= 0) atomicMax(metric_shots, max_shot);
 	}
 }
 
@@ -973,10 +1361,7 @@ __device__ __forceinline__ void pm_sweep_point(const PmArgs &p, const PmSmem &m,
 // of a first accepted random draw (patch_match.cpp:452-456, 481-485).
 template <int KIND, int C, int P, int V>
 __global__ void __launch_bounds__(pm_threads(V), 1) k_pm_sweep(DistArgs a, PmArgs p, int sweep, int jump,
-                                                       const int2 *__restrict__ nnf_in, const float *__restrict__ dist_in,
-                                                       const uint8_t *__restrict__ hist_in, int2 *__restrict__ nnf_out,
-                                                       float *__restrict__ dist_out, uint8_t *__restrict__ hist_out,
-                                                       unsigned long long *counter, unsigned long long *metric_prop,
+                                                       PmIo io, unsigned long long *counter, unsigned long long *metric_prop,
                                                        int *metric_shots, const __grid_constant__ CUtensorMap tmap,
                                                        int *timeout)
 {
@@ -992,8 +1377,8 @@ __global__ void __launch_bounds__(pm_threads(V), 1) k_pm_sweep(DistArgs a, PmArg
 	// number of random-search windows: max_window, max_window / 2, ..., 1
 	const int windows = 32 - __clz(p.max_window);
 	pm_for_each(p.nt, p.queue ? p.queue + 1 + sweep : nullptr, p.tile, [&](int wi) {
-		pm_sweep_point<KIND, C, P, V>(p, m, ts, tw, key, windows, p.tlist[wi], sweep, jump, nnf_in, dist_in, hist_in,
-		                              nnf_out, dist_out, hist_out, evals, partial, improved, max_shot);
+		pm_sweep_point<KIND, C, P, V>(p, m, ts, tw, key, windows, p.tlist[wi], sweep, jump, io, evals, partial, improved,
+		                              max_shot);
 	});
 	if (lane == 0 && evals) {
 		atomicAdd(counter, (unsigned long long)evals);
@@ -1030,82 +1415,93 @@ void sweep_energy(cudaStream_t s, const PmArgs &p, const float *dist, const PmMe
 // The padded source as a tensor map of candidate windows (patchmatch.cu).
 bool encode_source_map(const PmArgs &p, CUtensorMap *map);
 
-// A call's field, distances and change histories (seen_before), each twice:
-// sweep s reads x and writes y when s is even, the other way round when odd.
-struct PmFields {
-	int2 *nnf_x, *nnf_y;
-	float *dist_x, *dist_y;
-	uint8_t *hist_x, *hist_y;
-};
+// The kernels' dynamic shared-memory limit is raised once per device, to the
+// largest opt-in size (each launch passes the size it uses): a function
+// attribute set on every call costs a driver call per PatchMatch call on
+// every batch worker thread.
+template <class Init, class Sweep>
+static void raise_smem(nli_ctx *ctx, std::atomic<uint32_t> &raised, Init *init, Sweep *sweep)
+{
+	const uint32_t bit = 1u << (ctx->device & 31);
+	if (raised.load(std::memory_order_acquire) & bit) return;
+	NLI_CUDA(cudaFuncSetAttribute(init, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin));
+	NLI_CUDA(cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin));
+	raised.fetch_or(bit, std::memory_order_release);
+}
 
+// The one-point variants of the 9 x 9 kernels.
 template <int KIND, int C, int P, int V>
 static void launch_sweeps(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int iterations, const int2 *init,
-                          const PmFields &b, unsigned long long *counter, const PmMetrics &mt, const CUtensorMap &map, size_t smem)
+                          const PmFields &b, unsigned long long *counter, const PmMetrics &mt,
+                          const CUtensorMap &map, size_t smem)
 {
-	const PmShape shape = pm_shape(V, p.nt, ctx->num_sms);
-	const int block = shape.block, grid = shape.grid;
+	const PmShape shape = pm_shape(pm_threads(V), p.nt, ctx->num_sms);
 	int *timeout = &ctx->status->timeout;
-	// The kernels' dynamic shared-memory limit is raised once per device, to
-	// the largest opt-in size (each launch passes the size it uses): a
-	// function attribute set on every call costs a driver call per PatchMatch
-	// call on every batch worker thread.
 	static std::atomic<uint32_t> raised{0};  // one bit per device
-	const uint32_t bit = 1u << (ctx->device & 31);
-	if (!(raised.load(std::memory_order_acquire) & bit)) {
-		NLI_REQUIRE(smem <= (size_t)ctx->max_smem_optin, NLI_E_UNSUPPORTED, "PatchMatch shared memory too large");
-		NLI_CUDA(cudaFuncSetAttribute(k_pm_init<KIND, C, P, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                              ctx->max_smem_optin));
-		NLI_CUDA(cudaFuncSetAttribute(k_pm_sweep<KIND, C, P, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                              ctx->max_smem_optin));
-		raised.fetch_or(bit, std::memory_order_release);
-	}
+	raise_smem(ctx, raised, k_pm_init<KIND, C, P, V>, k_pm_sweep<KIND, C, P, V>);
 	NLI_REQUIRE(smem <= (size_t)ctx->max_smem_optin, NLI_E_UNSUPPORTED, "PatchMatch shared memory too large");
 	{
 		ProfScope ps(ctx, "pm_init");
-		k_pm_init<KIND, C, P, V><<<grid, block, smem, ctx->stream>>>(a, p, init, b.nnf_x, b.dist_x, counter, map,
-		                                                              timeout);
+		k_pm_init<KIND, C, P, V><<<shape.grid, shape.block, smem, ctx->stream>>>(a, p, init, b.nnf_x, b.dist_x,
+		                                                                         counter, map, timeout);
 		NLI_CHECK_LAUNCH();
 	}
 	for (int it = 0; it < iterations; it++) {
-		const bool even = (it % 2) == 0;
 		ProfScope ps(ctx, "pm_sweep");
-		k_pm_sweep<KIND, C, P, V><<<grid, block, smem, ctx->stream>>>(
-		    a, p, it, jump_for(it, p.tW, p.tH), even ? b.nnf_x : b.nnf_y, even ? b.dist_x : b.dist_y,
-		    even ? b.hist_x : b.hist_y, even ? b.nnf_y : b.nnf_x, even ? b.dist_y : b.dist_x,
-		    even ? b.hist_y : b.hist_x, counter, mt.prop ? mt.prop + it : nullptr, mt.shots, map, timeout);
+		k_pm_sweep<KIND, C, P, V><<<shape.grid, shape.block, smem, ctx->stream>>>(
+		    a, p, it, jump_for(it, p.tW, p.tH), b.io(it), counter, mt.prop ? mt.prop + it : nullptr, mt.shots, map, timeout);
 		NLI_CHECK_LAUNCH();
-		if (mt.energy) sweep_energy(ctx->stream, p, even ? b.dist_y : b.dist_x, mt, it);
+		if (mt.energy) sweep_energy(ctx->stream, p, b.io(it).dist_out, mt, it);
+	}
+}
+
+template <int KIND, int C, int P>
+static void launch_grouped(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int iterations, const int2 *init,
+                           const PmFields &b, unsigned long long *counter, const PmMetrics &mt)
+{
+	const PmShape shape =
+	    pm_shape(pm_threads(kPmGrouped), (p.nt + p.group.points - 1) / p.group.points, ctx->num_sms);
+	const size_t smem = pm_smem_bytes(a.px * a.py, shape.block / 32);
+	{
+		ProfScope ps(ctx, "pm_init");
+		k_pm_init_grouped<KIND, C, P><<<shape.grid, shape.block, smem, ctx->stream>>>(a, p, init, b.nnf_x, b.dist_x,
+		                                                                              counter);
+		NLI_CHECK_LAUNCH();
+	}
+	for (int it = 0; it < iterations; it++) {
+		ProfScope ps(ctx, "pm_sweep");
+		k_pm_sweep_grouped<KIND, C, P><<<shape.grid, shape.block, smem, ctx->stream>>>(
+		    a, p, it, jump_for(it, p.tW, p.tH), b.io(it), counter, mt.prop ? mt.prop + it : nullptr, mt.shots);
+		NLI_CHECK_LAUNCH();
+		if (mt.energy) sweep_energy(ctx->stream, p, b.io(it).dist_out, mt, it);
 	}
 }
 
 // Fixed-size patches take the context's variant; the staged one only when
 // the tensor map encodes and its layout fits, else (and for runtime-sized
-// patches) kPmShared.
+// patches) kPmGrouped.
 template <int KIND, int C, int P>
-static void run_sweeps(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int iterations, const int2 *init,
+static void run_sweeps(nli_ctx *ctx, const DistArgs &a, PmArgs p, int iterations, const int2 *init,
                        const PmFields &b, unsigned long long *counter, const PmMetrics &mt)
 {
-	const int taps = a.px * a.py;
-	CUtensorMap map;
-	std::memset(&map, 0, sizeof(map));
 	if constexpr (P > 0) {
+		CUtensorMap map;
+		std::memset(&map, 0, sizeof(map));
+		const int taps = a.px * a.py, warps = pm_shape(pm_threads(ctx->tune_pm_variant), p.nt, ctx->num_sms).block / 32;
 		if (ctx->tune_pm_variant == kPmStaged) {
-			const size_t smem = pm_smem_bytes_tma(taps, p.rows, p.L, p.K,
-			                                      pm_shape(kPmStaged, p.nt, ctx->num_sms).block / 32);
+			const size_t smem = pm_smem_bytes_tma(taps, p.rows, p.L, p.K, warps);
 			if (smem <= (size_t)ctx->max_smem_optin && encode_source_map(p, &map)) {
 				launch_sweeps<KIND, C, P, kPmStaged>(ctx, a, p, iterations, init, b, counter, mt, map, smem);
 				return;
 			}
 		} else if (ctx->tune_pm_variant == kPmRegs) {
 			launch_sweeps<KIND, C, P, kPmRegs>(ctx, a, p, iterations, init, b, counter, mt, map,
-			                                   pm_smem_bytes(taps, p.rows, p.L,
-			                                                 pm_shape(kPmRegs, p.nt, ctx->num_sms).block / 32));
+			                                   pm_smem_bytes(taps, warps));
 			return;
 		}
 	}
-	launch_sweeps<KIND, C, P, kPmShared>(ctx, a, p, iterations, init, b, counter, mt, map,
-	                                     pm_smem_bytes(taps, p.rows, p.L,
-	                                                   pm_shape(kPmShared, p.nt, ctx->num_sms).block / 32));
+	p.group = pm_group(p.nt, p.max_window, ctx->num_sms);
+	launch_grouped<KIND, C, P>(ctx, a, p, iterations, init, b, counter, mt);
 }
 
 // ====================================================== batched launches
@@ -1122,18 +1518,17 @@ static void run_sweeps(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int ite
 // __grid_constant__ table read through the constant cache, not the L1 data
 // pipe that bounds the sweep).  The persistent kernels see the concatenated
 // target lists of the images still iterating (their `active` flag, written
-// on the device between iterations) as one work list, distributed as the
-// one-image kernels distribute theirs (pm_for_each: static block ranges or
-// the device work queue).
+// on the device between iterations) as one work list of groups (a group's
+// points are one image's), distributed as the one-image kernels distribute
+// theirs (pm_for_each: static block ranges or the device work queue).
 struct PmBatchTask {
 	PmArgs p;
 	int flag;            // index of the image's active flag
 	unsigned long long *counter;  // the image's candidate counters (2)
 	const float *img;    // the image (source = target), HWC float
 	const int2 *init;    // initial field or null
-	int2 *nnf_x, *nnf_y;  // result (x) and the sweeps' second buffer
-	float *dist_x, *dist_y;
-	uint8_t *hist_x, *hist_y;
+	int2 *nnf_x;         // result
+	PmIo io[2];          // even sweeps read x and write the second buffer, odd ones the other way round
 };
 
 struct PmBatchArgs {
@@ -1141,20 +1536,24 @@ struct PmBatchArgs {
 	const int *active;  // per image: still iterating (null: all)
 	unsigned *queue;    // device work queue as PmArgs::queue (null: static ranges)
 	int tile;
+	PmGroup group;      // as PmArgs::group, the same for every image
 	PmBatchTask t[kBatchMax];
 };
 
 __device__ __forceinline__ bool batch_on(const int *active, int t) { return !active || active[t] != 0; }
 
-// Exclusive prefix of the active images' target counts in s_pre[0..n]
+// Exclusive prefix of the active images' numbers of groups in s_pre[0..n]
 // (s_pre[n] is the total); the whole block calls it.
 __device__ __forceinline__ int pm_batch_prefix(const PmBatchArgs &B, int *s_pre)
 {
 	if (threadIdx.x < 32) {
 		const int lane = threadIdx.x;
 		const int t0 = 2 * lane, t1 = t0 + 1;
-		const int v0 = (t0 < B.n && batch_on(B.active, B.t[t0].flag)) ? B.t[t0].p.nt : 0;
-		const int v1 = (t1 < B.n && batch_on(B.active, B.t[t1].flag)) ? B.t[t1].p.nt : 0;
+		auto groups = [&](int t) {
+			return (t < B.n && batch_on(B.active, B.t[t].flag)) ? (B.t[t].p.nt + B.group.points - 1) / B.group.points
+			                                                    : 0;
+		};
+		const int v0 = groups(t0), v1 = groups(t1);
 		int incl = v0 + v1;
 #pragma unroll
 		for (int o = 1; o < 32; o <<= 1) {
@@ -1170,110 +1569,77 @@ __device__ __forceinline__ int pm_batch_prefix(const PmBatchArgs &B, int *s_pre)
 	return s_pre[B.n];
 }
 
-// Adds a warp's candidate counts to its image's counters and the launch's
-// total, and clears them.
-__device__ __forceinline__ void pm_batch_count(unsigned long long *image, unsigned long long *total, unsigned &evals,
-                                               unsigned &partial)
-{
-	if ((threadIdx.x & 31) == 0 && evals) {
-		atomicAdd(total, (unsigned long long)evals);
-		if (partial) atomicAdd(total + 1, (unsigned long long)partial);
-		if (image) {
-			atomicAdd(image, (unsigned long long)evals);
-			if (partial) atomicAdd(image + 1, (unsigned long long)partial);
-		}
-	}
-	evals = partial = 0;
-}
-
 template <int KIND, int C, int P>
-__global__ void __launch_bounds__(pm_threads(kPmShared), 1)
+__global__ void __launch_bounds__(pm_threads(kPmGrouped), 1)
     k_pm_init_batch(DistArgs a, const __grid_constant__ PmBatchArgs B, unsigned long long *counter)
 {
 	__shared__ int s_pre[kBatchMax + 1];
-	const int lane = threadIdx.x & 31;
-	const PmSmem m = pm_smem<kPmShared>(a, B.t[0].p);
-	TmaState ts = {nullptr, nullptr, 0, nullptr, 0u, nullptr};
-	float4 tw[1];
+	const PmSmem m = pm_smem<kPmGrouped>(a, B.t[0].p);
 	load_weights(a, m.w);
 	const int total = pm_batch_prefix(B, s_pre);
-	unsigned evals = 0, partial = 0;
+	const PmLane at = pm_lane(B.group);
+	unsigned *list = reinterpret_cast<unsigned *>(m.list);
+	pm_count_clear(list);
 	int t = 0, tk = -1;
 	uint2 key = make_uint2(0u, 0u);
 	// a warp's items increase, so its image index only moves forward
-	pm_for_each(total, B.queue, B.tile, [&](int wi) {
-		while (wi >= s_pre[t + 1]) t++;
+	pm_for_each(total, B.queue, B.tile, [&](int i) {
+		while (i >= s_pre[t + 1]) t++;
 		const PmBatchTask &T = B.t[t];
 		if (t != tk) {
-			if (tk >= 0) pm_batch_count(B.t[tk].counter, counter, evals, partial);
+			if (tk >= 0) {
+				pm_count_add(list, counter, B.t[tk].counter);
+				pm_count_clear(list);
+			}
 			key = pm_key(T.p);
 			tk = t;
 		}
-		pm_init_point<KIND, C, P, kPmShared>(T.p, m, ts, tw, key, T.p.tlist[wi - s_pre[t]], T.init, T.nnf_x,
-		                                     T.dist_x, evals, partial);
+		pm_init_group<KIND, C, P>(T.p, m.w, list, at, key, (i - s_pre[t]) * B.group.points, T.init, T.nnf_x,
+		                          T.io[1].dist_out);
 	});
-	if (tk >= 0) pm_batch_count(B.t[tk].counter, counter, evals, partial);
+	if (tk >= 0) pm_count_add(list, counter, B.t[tk].counter);
 }
 
 template <int KIND, int C, int P>
-__global__ void __launch_bounds__(pm_threads(kPmShared), 1)
+__global__ void __launch_bounds__(pm_threads(kPmGrouped), 1)
     k_pm_sweep_batch(DistArgs a, const __grid_constant__ PmBatchArgs B, int sweep, unsigned long long *counter)
 {
 	__shared__ int s_pre[kBatchMax + 1];
-	const int lane = threadIdx.x & 31;
-	const PmSmem m = pm_smem<kPmShared>(a, B.t[0].p);
-	TmaState ts = {nullptr, nullptr, 0, nullptr, 0u, nullptr};
-	float4 tw[1];
+	const PmSmem m = pm_smem<kPmGrouped>(a, B.t[0].p);
 	load_weights(a, m.w);
 	const int total = pm_batch_prefix(B, s_pre);
-	unsigned evals = 0, partial = 0, improved = 0;
+	const PmLane at = pm_lane(B.group);
+	unsigned *list = reinterpret_cast<unsigned *>(m.list);
+	pm_count_clear(list);
 	int max_shot = -1;
-	const bool even = (sweep % 2) == 0;
 	int t = 0, tk = -1, windows = 0, jump = 1;
 	uint2 key = make_uint2(0u, 0u);
-	pm_for_each(total, B.queue ? B.queue + 1 + sweep : nullptr, B.tile, [&](int wi) {
-		while (wi >= s_pre[t + 1]) t++;
+	pm_for_each(total, B.queue ? B.queue + 1 + sweep : nullptr, B.tile, [&](int i) {
+		while (i >= s_pre[t + 1]) t++;
 		const PmBatchTask &T = B.t[t];
 		if (t != tk) {
-			if (tk >= 0) pm_batch_count(B.t[tk].counter, counter, evals, partial);
+			if (tk >= 0) {
+				pm_count_add(list, counter, B.t[tk].counter);
+				pm_count_clear(list);
+			}
 			key = pm_key(T.p);
 			windows = 32 - __clz(T.p.max_window);
 			jump = jump_for(sweep, T.p.tW, T.p.tH);
 			tk = t;
 		}
-		pm_sweep_point<KIND, C, P, kPmShared>(T.p, m, ts, tw, key, windows, T.p.tlist[wi - s_pre[t]], sweep, jump,
-		                                      even ? T.nnf_x : T.nnf_y, even ? T.dist_x : T.dist_y,
-		                                      even ? T.hist_x : T.hist_y, even ? T.nnf_y : T.nnf_x,
-		                                      even ? T.dist_y : T.dist_x, even ? T.hist_y : T.hist_x, evals, partial,
-		                                      improved, max_shot);
+		pm_sweep_group<KIND, C, P>(T.p, m.w, list, at, key, windows, (i - s_pre[t]) * B.group.points, sweep, jump,
+		                           T.io[sweep & 1], max_shot);
 	});
-	if (tk >= 0) pm_batch_count(B.t[tk].counter, counter, evals, partial);
+	if (tk >= 0) pm_count_add(list, counter, B.t[tk].counter);
 }
 
 template <int KIND, int C, int P>
-static void run_batch_kernels(nli_ctx *ctx, const DistArgs &a, const PmBatchArgs &B, int iterations, PmShape shape,
-                              size_t smem, unsigned long long *counter)
+static void run_batch_kernels(nli_ctx *ctx, const DistArgs &a, const PmBatchArgs &B, int iterations, long long groups,
+                              unsigned long long *counter)
 {
+	const PmShape shape = pm_shape(pm_threads(kPmGrouped), groups, ctx->num_sms);
 	const int block = shape.block, grid = shape.grid;
-	// dynamic shared memory up to the opt-in limit less the kernels' static
-	// shared memory (the work-list prefix), raised once per device
-	static std::atomic<uint32_t> raised{0};  // one bit per device
-	// written by whichever thread raises the limit first (concurrent
-	// sub-groups may race to it with the same value)
-	static std::atomic<int> dyn_max[32];
-	const uint32_t bit = 1u << (ctx->device & 31);
-	if (!(raised.load(std::memory_order_acquire) & bit)) {
-		cudaFuncAttributes fa_init, fa_sweep;
-		NLI_CUDA(cudaFuncGetAttributes(&fa_init, k_pm_init_batch<KIND, C, P>));
-		NLI_CUDA(cudaFuncGetAttributes(&fa_sweep, k_pm_sweep_batch<KIND, C, P>));
-		const int dmax = ctx->max_smem_optin - (int)std::max(fa_init.sharedSizeBytes, fa_sweep.sharedSizeBytes);
-		NLI_CUDA(cudaFuncSetAttribute(k_pm_init_batch<KIND, C, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, dmax));
-		NLI_CUDA(cudaFuncSetAttribute(k_pm_sweep_batch<KIND, C, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, dmax));
-		dyn_max[ctx->device & 31].store(dmax, std::memory_order_relaxed);
-		raised.fetch_or(bit, std::memory_order_release);
-	}
-	NLI_REQUIRE(smem <= (size_t)dyn_max[ctx->device & 31].load(std::memory_order_relaxed), NLI_E_UNSUPPORTED,
-	            "PatchMatch shared memory too large");
+	const size_t smem = pm_smem_bytes(a.px * a.py, block / 32);
 	{
 		ProfScope ps(ctx, "pm_init");
 		k_pm_init_batch<KIND, C, P><<<grid, block, smem, ctx->stream>>>(a, B, counter);
@@ -1293,7 +1659,7 @@ template <int KIND, int C>
 struct PmKernels {
 	static void sweeps(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int iterations, const int2 *init,
 	                   const PmFields &b, unsigned long long *counter, const PmMetrics &mt);
-	static void batch(nli_ctx *ctx, const DistArgs &a, const PmBatchArgs &B, int iterations, PmShape shape, size_t smem,
+	static void batch(nli_ctx *ctx, const DistArgs &a, const PmBatchArgs &B, int iterations, long long groups,
 	                  unsigned long long *counter);
 };
 
@@ -1309,13 +1675,13 @@ void PmKernels<KIND, C>::sweeps(nli_ctx *ctx, const DistArgs &a, const PmArgs &p
 }
 
 template <int KIND, int C>
-void PmKernels<KIND, C>::batch(nli_ctx *ctx, const DistArgs &a, const PmBatchArgs &B, int iterations, PmShape shape,
-                               size_t smem, unsigned long long *counter)
+void PmKernels<KIND, C>::batch(nli_ctx *ctx, const DistArgs &a, const PmBatchArgs &B, int iterations, long long groups,
+                               unsigned long long *counter)
 {
 	if (a.px == 9 && a.py == 9)
-		run_batch_kernels<KIND, C, 9>(ctx, a, B, iterations, shape, smem, counter);
+		run_batch_kernels<KIND, C, 9>(ctx, a, B, iterations, groups, counter);
 	else
-		run_batch_kernels<KIND, C, 0>(ctx, a, B, iterations, shape, smem, counter);
+		run_batch_kernels<KIND, C, 0>(ctx, a, B, iterations, groups, counter);
 }
 #endif
 
