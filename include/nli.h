@@ -454,10 +454,12 @@ int nli_ctx_set_batch_width(nli_ctx *ctx, int width);
  *                                  enough that its distance provably cannot
  *                                  beat the current match: 1 (default) by
  *                                  the weighted means (Jensen's
- *                                  inequality); 2 by the means and the
- *                                  weighted standard deviations (L2 kinds;
- *                                  L1 uses the means): fewer candidates
- *                                  evaluated, but slower on the 512x512
+ *                                  inequality) and, for the L2 kinds on
+ *                                  large calls, the weighted slopes
+ *                                  (Bessel's inequality); 2 also by the
+ *                                  weighted standard deviations (L2 kinds):
+ *                                  fewer candidates evaluated, but slower
+ *                                  on the 512x512
  *                                  benchmark; 0 every candidate is
  *                                  evaluated.  The bound keeps a rounding
  *                                  margin, so fields and distances are

@@ -1,13 +1,165 @@
 // PatchMatch's entry points: buffers, tables and launches around the sweep
 // kernels of pm_kernels.cuh, which pm_*.cu instantiate.
+#include <cmath>
+
 #include "pm_kernels.cuh"
 
 namespace nli {
 
-__global__ void k_pm_moments(DistArgs a, const float4 *__restrict__ pad, int W, int H, float4 *__restrict__ mom,
-                             unsigned *vmax, int dev)
+// ------------------------------------------------------ bound tables
+// Factors of the patch weights along x and y and the slopes' weights: f_1 =
+// (x - mean x) / sigma_x under the weights, f_2 likewise in y (0 for a side of
+// one tap, whose slope says nothing).
+static void patch_factors(PmFactors &f, const DistArgs &a)
 {
-	moments_span(a, pad, W, H, mom, vmax, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, dev != 0);
+	std::memset(&f, 0, sizeof(f));
+	f.px = a.px;
+	f.py = a.py;
+	f.rx = a.rx;
+	f.ry = a.ry;
+	auto axis = [](const double *w, int n, float *ow, float *of) {
+		double mean = 0.0, var = 0.0;
+		for (int i = 0; i < n; i++) mean += w[i] * i;
+		for (int i = 0; i < n; i++) var += w[i] * (i - mean) * (i - mean);
+		for (int i = 0; i < n; i++) {
+			ow[i] = (float)w[i];
+			of[i] = var > 1e-9 ? (float)(w[i] * (i - mean) / std::sqrt(var)) : 0.f;
+		}
+	};
+	double wx[NLI_MAX_PATCH] = {}, wy[NLI_MAX_PATCH] = {};
+	for (int y = 0; y < a.py; y++)
+		for (int x = 0; x < a.px; x++) {
+			wx[x] += a.weights[y * a.px + x];
+			wy[y] += a.weights[y * a.px + x];
+		}
+	axis(wx, a.px, f.wx, f.fx);
+	axis(wy, a.py, f.wy, f.fy);
+}
+
+// Whether the L2 kinds' bound uses the slopes for an image of nt target points:
+// the terms it bounds have non-negative factors, and the call is one whose
+// points come in groups (pm_group) -- there a candidate less is a part of a
+// round less, while a small call waits longer for the second test than for
+// the evaluations it saves (64 x 48: 296 us without, 317 with; 130 x 81: 355
+// and 373; 512 x 512: 1466 and 1382).  By the image's own size, so that a
+// batch tests as the image alone does.
+static int bound_slopes(const nli_distance_params &d, int nt, int num_sms)
+{
+	if (nt < 48 * num_sms) return 0;
+	auto share = [](float v) { return v >= 0.f && v <= 1.f; };
+	if (d.kind == NLI_DIST_L1_NORM) return 0;
+	if (d.kind == NLI_DIST_L2_NORM) return 1;
+	return share(d.lambda) && (d.kind != NLI_DIST_L2_RGBD || share(d.lambda_d));
+}
+
+// Means and slopes of every position of the padded (W + 1) x (H + 1) grid
+// (window clamped to the grid), and the largest absolute pixel value (atomicMax
+// on the float bits of non-negative values).  The weights are a product of
+// factors, so a tile of kMomW x kMomH positions sums along x (w and w f_1)
+// over its rows and the window's, then along y: 2 x 9 + 3 x 9 products per
+// position instead of 3 x 81, every pixel read about 2.7 times instead of
+// 81.  The one-pass form took 25.4 us for the means alone at 512 x 512 (bound
+// by the L1 data pipe), this takes 13.1 us for means and slopes (15 MB written:
+// 1.2 TB/s); 64 x 48: 8.9 and 4.8 us.
+constexpr int kMomW = 32, kMomH = 8;
+
+__device__ __forceinline__ void moments_tile(const PmFactors &f, const float4 *__restrict__ pad, int W, int H,
+                                             float4 *__restrict__ mom, unsigned *vmax, int slopes, int tile)
+{
+	__shared__ float4 s_in[kMomH + NLI_MAX_PATCH - 1][kMomW + NLI_MAX_PATCH - 1];
+	__shared__ float4 s_w[kMomH + NLI_MAX_PATCH - 1][kMomW], s_f[kMomH + NLI_MAX_PATCH - 1][kMomW];
+	const int Wp = W + 1, tiles_x = (Wp + kMomW - 1) / kMomW;
+	const int x0 = (tile % tiles_x) * kMomW, y0 = (tile / tiles_x) * kMomH;
+	const int cols = kMomW + f.px - 1, rows = kMomH + f.py - 1;
+	for (int e = threadIdx.x; e < rows * cols; e += blockDim.x) {
+		const int r = e / cols, c = e - r * cols;
+		const int y = min(max(y0 - f.ry + r, 0), H), x = min(max(x0 - f.rx + c, 0), W);
+		s_in[r][c] = __ldg(pad + (size_t)y * Wp + x);
+	}
+	__syncthreads();
+	const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+	for (int e = threadIdx.x; e < rows * kMomW; e += blockDim.x) {
+		const int r = e / kMomW, c = e - r * kMomW;
+		float4 a = zero, b = zero;
+		for (int i = 0; i < f.px; i++) {
+			const float4 v = s_in[r][c + i];
+			a = f4_fma(f.wx[i], v, a);
+			b = f4_fma(f.fx[i], v, b);
+		}
+		s_w[r][c] = a;
+		s_f[r][c] = b;
+	}
+	__syncthreads();
+	const int c = threadIdx.x % kMomW, r = threadIdx.x / kMomW;
+	const int x = x0 + c, y = y0 + r;
+	float vm = 0.f;
+	if (x <= W && y <= H) {
+		float4 m = zero, sx = zero, sy = zero;
+		for (int j = 0; j < f.py; j++) {
+			const float4 a = s_w[r + j][c];
+			m = f4_fma(f.wy[j], a, m);
+			sx = f4_fma(f.wy[j], s_f[r + j][c], sx);
+			sy = f4_fma(f.fy[j], a, sy);
+		}
+		const size_t i = (size_t)y * Wp + x, n = (size_t)Wp * (H + 1);
+		mom[i] = m;
+		if (slopes) {
+			mom[n + 2 * i] = sx;
+			mom[n + 2 * i + 1] = sy;
+		}
+		const float4 v = s_in[r + f.ry][c + f.rx];
+		vm = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+	}
+	for (int o = 16; o > 0; o >>= 1) vm = fmaxf(vm, __shfl_xor_sync(kFull, vm, o));
+	if ((threadIdx.x & 31) == 0 && vm > 0.f) atomicMax(vmax, __float_as_uint(vm));
+}
+
+static int moment_tiles(int W, int H) { return ((W + 1 + kMomW - 1) / kMomW) * ((H + 1 + kMomH - 1) / kMomH); }
+
+__global__ void __launch_bounds__(kMomW * kMomH)
+    k_pm_moments(const __grid_constant__ PmFactors f, const float4 *__restrict__ pad, int W, int H,
+                 float4 *__restrict__ mom, unsigned *vmax, int slopes)
+{
+	moments_tile(f, pad, W, H, mom, vmax, slopes, blockIdx.x);
+}
+
+// The weighted standard deviations of the image and of its forward
+// differences in x and in y (NLI_TUNE_PM_BOUND 2), tables 3 to 5 of n = (W +
+// 1)(H + 1) float4: sqrt(sum_k w_k (v_k - mean)^2) from a second, centred pass.
+__device__ __forceinline__ void deviations_span(const DistArgs &a, const float4 *__restrict__ pad, int W, int H,
+                                                float4 *__restrict__ mom, int first, int stride)
+{
+	const int Wp = W + 1, n = Wp * (H + 1);
+	const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+	for (int i = first; i < n; i += stride) {
+		const int y = i / Wp, x = i - y * Wp;
+		float4 mean[3] = {zero, zero, zero}, s[3] = {zero, zero, zero};
+		for (int pass = 0; pass < 2; pass++)
+			for (int dy = 0; dy < a.py; dy++) {
+				const int yy = min(max(y - a.ry + dy, 0), H);
+				const float4 *row = pad + (size_t)yy * Wp, *below = pad + (size_t)min(yy + 1, H) * Wp;
+				for (int dx = 0; dx < a.px; dx++) {
+					const int xx = min(max(x - a.rx + dx, 0), W);
+					const float4 v = __ldg(row + xx);
+					const float w = a.weights[dy * a.px + dx];
+					const float4 d[3] = {v, f4_sub(__ldg(row + min(xx + 1, W)), v), f4_sub(__ldg(below + xx), v)};
+#pragma unroll
+					for (int k = 0; k < 3; k++) {
+						if (pass == 0)
+							mean[k] = f4_fma(w, d[k], mean[k]);
+						else
+							s[k] = f4_wsq(w, f4_sub(d[k], mean[k]), s[k]);
+					}
+				}
+			}
+#pragma unroll
+		for (int k = 0; k < 3; k++) mom[(size_t)(3 + k) * n + i] = f4_sqrt(s[k]);
+	}
+}
+
+__global__ void k_pm_deviations(DistArgs a, const float4 *__restrict__ pad, int W, int H, float4 *__restrict__ mom)
+{
+	deviations_span(a, pad, W, H, mom, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // Also advances the context's PatchMatch call index when `calls` is set.
@@ -102,14 +254,24 @@ __global__ void k_pad4_batch(const __grid_constant__ PmBatchArgs B, int C)
 	          gridDim.x * blockDim.x);
 }
 
-// The patch means of every active image (k_pm_moments per image).
-__global__ void k_pm_moments_batch(DistArgs a, const __grid_constant__ PmBatchArgs B)
+// k_pm_moments and k_pm_deviations per active image.
+__global__ void __launch_bounds__(kMomW * kMomH)
+    k_pm_moments_batch(const __grid_constant__ PmFactors f, const __grid_constant__ PmBatchArgs B)
 {
 	const int t = blockIdx.y;
 	const PmBatchTask &T = B.t[t];
-	if (!batch_on(B.active, T.flag) || !T.p.smom) return;
-	moments_span(a, T.p.src, T.p.sW, T.p.sH, const_cast<float4 *>(T.p.smom), const_cast<unsigned *>(T.p.vmax),
-	             blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, T.p.dev != 0);
+	if (!batch_on(B.active, T.flag) || (int)blockIdx.x >= T.moment_tiles) return;
+	moments_tile(f, T.p.src, T.p.sW, T.p.sH, const_cast<float4 *>(T.p.smom), const_cast<unsigned *>(T.p.vmax),
+	             T.p.slopes, blockIdx.x);
+}
+
+__global__ void k_pm_deviations_batch(DistArgs a, const __grid_constant__ PmBatchArgs B)
+{
+	const int t = blockIdx.y;
+	const PmBatchTask &T = B.t[t];
+	if (!batch_on(B.active, T.flag)) return;
+	deviations_span(a, T.p.src, T.p.sW, T.p.sH, const_cast<float4 *>(T.p.smom),
+	                blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // k_fill_nnf per active image: the result field to "none", and the image's
@@ -152,6 +314,7 @@ void patchmatch_batch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli
 	B.tile = ctx->tune_pm_tile;
 	int maxpix = 0, maxpad = 0, maxnt = 0;
 	long long total = 0;  // target points of all images
+	int maxtiles = 0;
 	int widest = 0;       // the largest random-search window (as unsigned)
 	for (int i = 0; i < n; i++) {
 		const PmBatchItem &it = items[i];
@@ -181,7 +344,10 @@ void patchmatch_batch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli
 		p.calls = it.calls;
 		p.smom = p.tmom = it.mom;
 		p.vmax = it.mom ? it.vmax : nullptr;
-		// the item's table holds room for the deviations (4 tables)
+		// the item's buffer holds room for every table (kPmMomentTables)
+		p.slopes = it.mom ? bound_slopes(dp, it.nt, ctx->num_sms) : 0;
+		T.moment_tiles = moment_tiles(it.W, it.H);
+		maxtiles = std::max(maxtiles, T.moment_tiles);
 		p.dev = (it.mom && ctx->tune_pm_bound == 2 && dp.kind != NLI_DIST_L1_NORM) ? 1 : 0;
 		p.queue = nullptr;  // the launch's queue is B.queue
 		p.tile = 0;
@@ -206,9 +372,15 @@ void patchmatch_batch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli
 	k_fill_nnf_batch<<<dim3((unsigned)std::min((maxpix + per - 1) / per, 1024), (unsigned)n), per, 0, s>>>(B);
 	NLI_CHECK_LAUNCH();
 	if (B.t[0].p.smom) {
-		k_pm_moments_batch<<<dim3((unsigned)std::min((maxpad + per - 1) / per, 1024), (unsigned)n), per, 0, s>>>(a,
-		                                                                                                       B);
+		PmFactors f;
+		patch_factors(f, a);
+		k_pm_moments_batch<<<dim3((unsigned)maxtiles, (unsigned)n), kMomW * kMomH, 0, s>>>(f, B);
 		NLI_CHECK_LAUNCH();
+		if (B.t[0].p.dev) {
+			k_pm_deviations_batch<<<dim3((unsigned)std::min((maxpad + per - 1) / per, 1024), (unsigned)n), per, 0,
+			                        s>>>(a, B);
+			NLI_CHECK_LAUNCH();
+		}
 	}
 	if (maxnt == 0) return;
 	unsigned long long *counter = ctx->buf<unsigned long long>("pm.counter", 2);
@@ -261,33 +433,36 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 		launch_pad4(s, tgt, tW, tH, C, t4);
 	}
 
-	// patch means for the lower bound (NLI_TUNE_PM_BOUND)
-	float4 *smom = nullptr, *tmom = nullptr;
-	unsigned *vmax = nullptr;
-	// the deviation tables serve the L2 kinds (NLI_TUNE_PM_BOUND 2)
-	const int dev = (ctx->tune_pm_bound == 2 && dp.kind != NLI_DIST_L1_NORM) ? 1 : 0;
-	if (ctx->tune_pm_bound) {
-		DistArgs da;
-		fill_dist_args(da, dp, C);
-		vmax = ctx->buf<unsigned>("pm.vmax", 1);
-		NLI_CUDA(cudaMemsetAsync(vmax, 0, sizeof(unsigned), s));
-		const int ns = (sW + 1) * (sH + 1);
-		smom = ctx->buf<float4>("pm.smom", (size_t)ns * (dev ? 4 : 1));
-		k_pm_moments<<<(ns + 255) / 256, 256, 0, s>>>(da, s4, sW, sH, smom, vmax, dev);
-		NLI_CHECK_LAUNCH();
-		tmom = smom;
-		if (t4 != s4) {
-			const int nt4 = (tW + 1) * (tH + 1);
-			tmom = ctx->buf<float4>("pm.tmom", (size_t)nt4 * (dev ? 4 : 1));
-			k_pm_moments<<<(nt4 + 255) / 256, 256, 0, s>>>(da, t4, tW, tH, tmom, vmax, dev);
-			NLI_CHECK_LAUNCH();
-		}
-	}
-
 	if (!tlist) {
 		int32_t *l = ctx->buf<int32_t>("pm.tlist", nT);
 		n_target = compact_mask(ctx, tmask, tW, tH, l, "pm");
 		tlist = l;
+	}
+
+	// tables of the lower bound (NLI_TUNE_PM_BOUND)
+	float4 *smom = nullptr, *tmom = nullptr;
+	unsigned *vmax = nullptr;
+	// the deviation tables serve the L2 kinds (NLI_TUNE_PM_BOUND 2)
+	const int dev = (ctx->tune_pm_bound == 2 && dp.kind != NLI_DIST_L1_NORM) ? 1 : 0;
+	const int slopes = ctx->tune_pm_bound ? bound_slopes(dp, n_target, ctx->num_sms) : 0;
+	if (ctx->tune_pm_bound) {
+		PmFactors f;
+		patch_factors(f, a);
+		vmax = ctx->buf<unsigned>("pm.vmax", 1);
+		NLI_CUDA(cudaMemsetAsync(vmax, 0, sizeof(unsigned), s));
+		auto tables = [&](const char *name, const float4 *pad, int W, int H) {
+			const size_t n = (size_t)(W + 1) * (H + 1);
+			float4 *mom = ctx->buf<float4>(name, n * (dev ? 6 : slopes ? 3 : 1));
+			k_pm_moments<<<moment_tiles(W, H), kMomW * kMomH, 0, s>>>(f, pad, W, H, mom, vmax, slopes);
+			NLI_CHECK_LAUNCH();
+			if (dev) {
+				k_pm_deviations<<<(int)((n + 255) / 256), 256, 0, s>>>(a, pad, W, H, mom);
+				NLI_CHECK_LAUNCH();
+			}
+			return mom;
+		};
+		smom = tables("pm.smom", s4, sW, sH);
+		tmom = t4 != s4 ? tables("pm.tmom", t4, tW, tH) : smom;
 	}
 	const int2 *init = reinterpret_cast<const int2 *>(init_nnf);
 	if (init_nnf && init_nnf == out_nnf) {
@@ -338,6 +513,7 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 		p.smom = smom;
 		p.tmom = tmom;
 		p.vmax = vmax;
+		p.slopes = slopes;
 		p.dev = smom ? dev : 0;
 		p.queue = nullptr;
 		p.tile = ctx->tune_pm_tile;

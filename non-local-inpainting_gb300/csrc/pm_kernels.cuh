@@ -197,14 +197,16 @@ struct PmArgs {
 	// lanes per candidate, candidates per warp step, window rows
 	int L, K, rows;
 	float lambda, lambda_d;
-	// patch-mean lower bound (null: off): the weighted patch means of the
-	// padded source and target, one float4 per (W + 1) x (H + 1) position,
-	// and the largest absolute pixel value of the images (as float bits)
+	// patch-statistics lower bound (null: off): the tables of the padded
+	// source and target (n = (W + 1)(H + 1) positions: n float4 of weighted
+	// patch means, then n pairs of weighted slopes in x and y), and the
+	// largest absolute pixel value of the images (as float bits)
 	const float4 *smom, *tmom;
 	const unsigned *vmax;
-	// 1: the tables also hold the weighted standard deviations (of the
-	// image and of its forward differences), and the bound uses them
-	int dev;
+	// 1: the bound uses the slopes; 1: behind them follow the weighted
+	// standard deviations (of the image and of its forward differences),
+	// and the bound uses them too
+	int slopes, dev;
 	// device work queue (null: static ranges): the call's counters, one
 	// per launch (init, then each sweep), zeroed before the init launch;
 	// a warp takes `tile` consecutive target points per grab
@@ -470,7 +472,7 @@ __device__ __forceinline__ float4 f4_sqrt(float4 a)
 	return make_float4(sqrtf(a.x), sqrtf(a.y), sqrtf(a.z), sqrtf(a.w));
 }
 
-// ------------------------------------------------ patch-mean lower bound
+// ------------------------------------------------ lower bound
 // Jensen's inequality gives, for weights v_k >= 0 summing to V,
 //   sum_k v_k |d_k|^2 >= |sum_k v_k d_k|^2 / V,   sum_k v_k |d_k|_1 >= |sum_k v_k d_k|_1.
 // With the kernel's tap weights v_k = w_k / P (sum 1 / P) and d_k the colour
@@ -480,23 +482,36 @@ __device__ __forceinline__ float4 f4_sqrt(float4 a)
 // apart.  So a candidate whose patch means differ enough from the target's
 // cannot beat the current match and is not evaluated.
 //
+// The means are the first of an orthonormal set: with f_0 = 1 and f_1, f_2 the
+// centred tap positions in x and y, scaled so that sum_k w_k f_i f_j = (i == j)
+// (they are orthogonal because the weights are a product of one factor in x
+// and one in y), Bessel's inequality gives
+//   sum_k w_k d_k^2 >= sum_j (sum_k w_k f_j d_k)^2.
+// The sums of f_1 and f_2, the patch's slopes, are two more linear tables, and
+// those of the forward differences are again differences of entries one
+// column (row) apart.  The L2 kinds test them (PmArgs::slopes) on what the
+// means let through: 686 -> 438 million evaluations in a 512 x 512 NL-Poisson
+// process() (590 -> 582 ms), and a first call on 512 x 512 takes 1383 us instead
+// of 1466, on 1013 x 887 5385 instead of 5732.
+//
 // With the weighted standard deviations as well (PmArgs::dev, the L2
-// kinds), the bound is tighter: for weights summing to 1,
+// kinds): for weights summing to 1,
 //   sum_k w_k d_k^2 = (sum_k w_k d_k)^2 + sum_k w_k (d_k - mean d)^2,
 // and with d = s - t the centred part is the squared weighted L2 distance of
 // the centred patches, at least (sigma_s - sigma_t)^2 by the reverse
 // triangle inequality.  So each channel's colour term is bounded by the
 // squared mean difference plus the squared difference of standard
 // deviations, and each gradient term likewise with the deviations of the
-// forward differences.
+// forward differences: a second bound beside that of the slopes.
 //
-// Exactness: every mean and deviation difference is shrunk by a slack (2e-4
-// of the largest pixel value) that covers the float rounding of the tables
-// (sums of 81 products: a few 1e-6 of the largest value) and of the
-// kernel's per-tap differences, and the bound must exceed the current
-// distance by a 1e-4 relative margin that covers the rounding of the
-// kernel's sums; the field and distances are those of evaluating every
-// candidate.
+// Exactness: every difference of means, slopes and deviations is shrunk by a
+// slack (2e-4 of the largest pixel value) that covers the float rounding of
+// the tables (sums of 81 products whose weights w_k |f_j| add up to at most
+// 1: a few 1e-6 of the largest value) and of the kernel's per-tap
+// differences, and the bound must exceed the current distance by a 1e-4
+// relative margin that covers the rounding of the kernel's sums and of the
+// set's orthonormality; the field and distances are those of evaluating
+// every candidate.
 __device__ __forceinline__ float shrink(float v, float slack) { return fmaxf(fabsf(v) - slack, 0.f); }
 
 // True when candidate (cx, cy) for target (x, y) provably cannot reach a
@@ -525,85 +540,54 @@ __device__ __forceinline__ bool bound_rejects(const PmArgs &p, int x, int y, int
 				(g ? grad : col) += e * e;
 		}
 	};
-	const float4 m0 = __ldg(M), t0 = __ldg(T);
-	add(f4_sub(m0, t0), false);
+	const float P = (float)((p.rx + p.ex) * (p.ry + p.ey));
+	auto exceeds = [&]() {
+		float lb = col;
+		if (Kind<KIND>::grad) lb = fmaf(p.lambda, col, (1.0f - p.lambda) * grad);
+		if (KIND == NLI_DIST_L2_RGBD) lb = fmaf(p.lambda_d, dcol, fmaf(1.0f - p.lambda_d, dgrad, lb));
+		return lb * (1.0f - 1e-4f) >= bd * P;
+	};
+	const float4 m0 = f4_sub(__ldg(M), __ldg(T));
+	add(m0, false);
 	if (Kind<KIND>::grad) {
 		// the mean of the forward differences: means one column (row) apart
-		add(f4_sub(f4_sub(__ldg(M + 1), m0), f4_sub(__ldg(T + 1), t0)), true);
-		add(f4_sub(f4_sub(__ldg(M + p.sWp), m0), f4_sub(__ldg(T + p.tWp), t0)), true);
+		add(f4_sub(f4_sub(__ldg(M + 1), __ldg(T + 1)), m0), true);
+		add(f4_sub(f4_sub(__ldg(M + p.sWp), __ldg(T + p.tWp)), m0), true);
 	}
-	if (KIND != NLI_DIST_L1_NORM && p.dev) {
+	if (exceeds()) return true;
+	if (KIND == NLI_DIST_L1_NORM) return false;
+	const size_t sn = (size_t)p.sWp * (p.sH + 1), tn = (size_t)p.tWp * (p.tH + 1);
+	if (p.dev) {
 		// weighted standard deviations: of the image, of its x and y differences
-		const size_t sn = (size_t)p.sWp * (p.sH + 1), tn = (size_t)p.tWp * (p.tH + 1);
-		add(f4_sub(__ldg(M + sn), __ldg(T + tn)), false);
+		const float c0 = col, g0 = grad, d0 = dcol, e0 = dgrad;
+		add(f4_sub(__ldg(M + 3 * sn), __ldg(T + 3 * tn)), false);
 		if (Kind<KIND>::grad) {
-			add(f4_sub(__ldg(M + 2 * sn), __ldg(T + 2 * tn)), true);
-			add(f4_sub(__ldg(M + 3 * sn), __ldg(T + 3 * tn)), true);
+			add(f4_sub(__ldg(M + 4 * sn), __ldg(T + 4 * tn)), true);
+			add(f4_sub(__ldg(M + 5 * sn), __ldg(T + 5 * tn)), true);
+		}
+		if (exceeds()) return true;
+		col = c0, grad = g0, dcol = d0, dgrad = e0;
+	}
+	if (!p.slopes) return false;
+	const float4 *MS = p.smom + sn + 2 * ((size_t)cy * p.sWp + cx), *TS = p.tmom + tn + 2 * ((size_t)y * p.tWp + x);
+#pragma unroll
+	for (int j = 0; j < 2; j++) {
+		const float4 f0 = f4_sub(__ldg(MS + j), __ldg(TS + j));
+		add(f0, false);
+		if (Kind<KIND>::grad) {
+			add(f4_sub(f4_sub(__ldg(MS + 2 + j), __ldg(TS + 2 + j)), f0), true);
+			add(f4_sub(f4_sub(__ldg(MS + 2 * p.sWp + j), __ldg(TS + 2 * p.tWp + j)), f0), true);
 		}
 	}
-	float lb = col;
-	if (Kind<KIND>::grad) lb = fmaf(p.lambda, col, (1.0f - p.lambda) * grad);
-	if (KIND == NLI_DIST_L2_RGBD) lb = fmaf(p.lambda_d, dcol, fmaf(1.0f - p.lambda_d, dgrad, lb));
-	const float P = (float)((p.rx + p.ex) * (p.ry + p.ey));
-	return lb * (1.0f - 1e-4f) >= bd * P;
+	return exceeds();
 }
 
-// Weighted patch statistics of the padded image at every position of the
-// (W + 1) x (H + 1) grid (window clamped to the grid): table 0 the weighted
-// means; with `dev`, tables 1-3 (each n = (W + 1)(H + 1) float4 further) the
-// weighted standard deviations of the image and of its forward differences
-// in x and in y, sqrt(sum_k w_k (v_k - mean)^2), from a second, centred
-// pass.  Also the largest absolute pixel value (atomicMax on the float bits
-// of non-negative values).
-__device__ __forceinline__ void moments_span(const DistArgs &a, const float4 *__restrict__ pad, int W, int H,
-                                             float4 *__restrict__ mom, unsigned *vmax, int first, int stride,
-                                             bool dev)
-{
-	const int Wp = W + 1, n = Wp * (H + 1);
-	float vm = 0.f;
-	const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-	for (int i = first; i < n; i += stride) {
-		const int y = i / Wp, x = i - y * Wp;
-		float4 acc = zero, ax = zero, ay = zero;
-		for (int dy = 0; dy < a.py; dy++) {
-			const int yy = min(max(y - a.ry + dy, 0), H);
-			const float4 *row = pad + (size_t)yy * Wp, *below = pad + (size_t)min(yy + 1, H) * Wp;
-			for (int dx = 0; dx < a.px; dx++) {
-				const int xx = min(max(x - a.rx + dx, 0), W);
-				const float4 v = __ldg(row + xx);
-				const float w = a.weights[dy * a.px + dx];
-				acc = f4_fma(w, v, acc);
-				if (dev) {
-					ax = f4_fma(w, f4_sub(__ldg(row + min(xx + 1, W)), v), ax);
-					ay = f4_fma(w, f4_sub(__ldg(below + xx), v), ay);
-				}
-			}
-		}
-		mom[i] = acc;
-		if (dev) {
-			float4 s = zero, sx = zero, sy = zero;
-			for (int dy = 0; dy < a.py; dy++) {
-				const int yy = min(max(y - a.ry + dy, 0), H);
-				const float4 *row = pad + (size_t)yy * Wp, *below = pad + (size_t)min(yy + 1, H) * Wp;
-				for (int dx = 0; dx < a.px; dx++) {
-					const int xx = min(max(x - a.rx + dx, 0), W);
-					const float4 v = __ldg(row + xx);
-					const float w = a.weights[dy * a.px + dx];
-					s = f4_wsq(w, f4_sub(v, acc), s);
-					sx = f4_wsq(w, f4_sub(f4_sub(__ldg(row + min(xx + 1, W)), v), ax), sx);
-					sy = f4_wsq(w, f4_sub(f4_sub(__ldg(below + xx), v), ay), sy);
-				}
-			}
-			mom[(size_t)n + i] = f4_sqrt(s);
-			mom[2 * (size_t)n + i] = f4_sqrt(sx);
-			mom[3 * (size_t)n + i] = f4_sqrt(sy);
-		}
-		const float4 v = __ldg(pad + i);
-		vm = fmaxf(vm, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-	}
-	for (int o = 16; o > 0; o >>= 1) vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, o));
-	if ((threadIdx.x & 31) == 0 && vm > 0.f) atomicMax(vmax, __float_as_uint(vm));
-}
+// The tables' tap weights, one factor per axis: w and w f (f_1 along x, f_2
+// along y; patch_factors in patchmatch.cu).
+struct PmFactors {
+	int px, py, rx, ry;
+	float wx[NLI_MAX_PATCH], wy[NLI_MAX_PATCH], fx[NLI_MAX_PATCH], fy[NLI_MAX_PATCH];
+};
 
 // Rows after which an evaluation is tested for early termination (counted
 // from 0): every term is non-negative, so once the rows summed so far reach
@@ -1524,6 +1508,7 @@ static void run_sweeps(nli_ctx *ctx, const DistArgs &a, PmArgs p, int iterations
 struct PmBatchTask {
 	PmArgs p;
 	int flag;            // index of the image's active flag
+	int moment_tiles;    // blocks of the image's bound tables
 	unsigned long long *counter;  // the image's candidate counters (2)
 	const float *img;    // the image (source = target), HWC float
 	const int2 *init;    // initial field or null
