@@ -712,35 +712,53 @@ __global__ void __launch_bounds__(kCgBlock) k_poisson_cg(PoissonArgs a, const Un
 	if (threadIdx.x == 0) diff_part[blockIdx.x] = dacc;
 }
 
-// Conjugate gradient on thread-block clusters with every vector and the
-// system itself in shared memory.  Cluster g of the grid solves channels
-// [g * C, (g + 1) * C) of the Ctot-channel image; the channels are
-// independent systems (the reference solves them one after the other), so
-// one cluster per channel (C = 1) spreads the solve over more SMs and lets
-// each channel stop at its own convergence.
+// Conjugate gradient on thread-block clusters with the vectors in registers
+// and shared memory.  Cluster g of the grid solves channel g of the image;
+// the channels are independent systems (the reference solves them one
+// after the other), so one cluster per channel spreads the solve over more
+// SMs and lets each channel stop at its own convergence.
 //
 // CTA `rank` of the cluster (up to 16 CTAs of 512 threads) owns the
-// contiguous unknown range [rank * chunk, (rank + 1) * chunk), chunk <=
-// 4096, and keeps in its shared memory the residual r, two alternating
-// direction buffers, the solution x and a compact 24-byte record per
-// unknown (its coefficients and 16-bit neighbour codes: owning CTA << 12 |
-// index); q = A d stays in registers.  Neighbours owned by another CTA are
-// read through distributed shared memory.  Iteration (as the reference's
-// conjugte_gradient, patch_non_local_poisson.cpp:387-477, with the
-// residual updated by recurrence): d = r + beta d_old (folded into the
-// stencil phase, formed at the neighbours from r and d_old), q = A d,
-// alpha = |r|^2 / <r, q>, x += alpha d, r -= alpha q, beta = |r'|^2 / |r|^2.
-// Two cluster barriers per iteration; block partial sums are exchanged
-// through distributed shared memory and added in rank order by one warp,
-// so every CTA holds the same totals.  alpha and beta are formed once per
-// CTA in double precision by that warp and published with one block
-// barrier.  (Pushing the partials into every CTA before the barrier, so
-// that the totals are read locally, measured no faster.)
+// contiguous unknown range [rank * chunk, (rank + 1) * chunk), chunk <= 4096;
+// thread t of it owns unknowns t, t + 512, ... and keeps their rows of the
+// system, r, x, d and q in registers.  Iteration (as the reference's
+// conjugte_gradient, patch_non_local_poisson.cpp:387-477, with the residual
+// updated by recurrence): d = r + beta d_old (folded into the stencil phase,
+// formed at the neighbours from r and d_old), q = A d, alpha = |r|^2 / <r, q>,
+// x += alpha d, r -= alpha q, beta = |r'|^2 / |r|^2.
+//
+// What a neighbour needs, the pair (r, d), is one float2 in shared memory, in
+// two alternating buffers: the update phase writes the new pair of every own
+// unknown with one store, and pushes it to the CTAs that have a neighbour of
+// it (the first and last pixel rows of a range), which hold a slot per such
+// neighbour; so the stencil reads four local float2 and nothing remote.
+//
+// An iteration is two exchanges between the CTAs and little else: everything
+// that crosses goes by asynchronous stores that complete on the receiver's
+// mbarrier, which warp 0 waits on.  At 16 CTAs, in cycles: exchanging one sum
+// per CTA so takes 449 (both block barriers included), with 512 pairs pushed
+// as well 745; a cluster barrier alone takes 522 (its release fence: 137
+// without), plain remote stores and a cluster barrier 1278, remote loads
+// instead of pushes 1373, and every warp pushing its own sum 2233.
+//
+// The sums.  Per thread in float, per warp in float, then in double over the
+// CTA's warps and over the CTAs, and alpha and beta are rounded quotients of
+// two such sums.  FP64 is slow here (62 cycles an addition, 562 a division: 1400
+// per exchange in its dependent chain), so what is formed is the sum as an
+// unevaluated pair of floats (Knuth's two-sum), exact to 2^-43, and the quotient
+// as such a pair.  Where every value within its error bound rounds to the same
+// float, that float is the quotient of the double sums; in the few cases
+// where it is not (about one in 16 000, and sums outside 1e-18 .. 1e18) the double
+// sums are formed (cg_double_total).  So are the stopping test's.
+//
+// 512 x 512 (39 000 unknowns, 3 x 16 CTAs, 73 iterations a channel, ncu): 185
+// us, 2.3 us an iteration, bound by the two exchanges and the block barriers
+// around them; 472 us with the rows and vectors in shared memory, remote
+// loads, two cluster barriers and double sums.
 constexpr int kClusterBlock = 512;
 constexpr int kClusterMax = 16;
 constexpr int kClusterMaxChunk = 4096;
 constexpr int kClusterPerThread = kClusterMaxChunk / kClusterBlock;  // unknowns per thread
-constexpr int kClusterVectors = 4;  // r, d (twice), x
 constexpr int kNoNb = 0xFFFF;
 
 struct UnkC {
@@ -790,333 +808,493 @@ __device__ __forceinline__ float jacobi_inv(const UnkC &n, float lam)
 // true residual, so the solve ends at the same residual as the plain CG,
 // in fewer iterations.  Without PRE, z is r itself and the iteration is the
 // reference's.
-// The CTAs that solve one system: a thread-block cluster (barriers and
-// distributed shared memory), or one CTA on its own (block barriers, its
-// own shared memory) for systems of at most kClusterMaxChunk unknowns.  The
-// one-CTA form performs the same arithmetic in the same order as a
-// cluster of one CTA.
-template <bool SINGLE>
-struct CgTeam;
+// Slots of a buffer of (r, d) pairs for ranges of `chunk` unknowns: the own
+// unknowns, then for each the slot of its upper and of its lower neighbour
+// where another CTA owns it, those of the range's left and right neighbour,
+// and one that stays zero for neighbours outside the hole.
+__host__ __device__ inline int cg_slots(int chunk) { return 3 * chunk + 3; }
 
-template <>
-struct CgTeam<true> {
-	__device__ int rank() const { return 0; }
-	__device__ int size() const { return 1; }
-	__device__ void sync() { __syncthreads(); }
-	template <class T>
-	__device__ T *map(T *p, int) const
-	{
-		return p;
-	}
+__host__ inline size_t cg_smem_bytes(int chunk) { return 2 * sizeof(float2) * (size_t)cg_slots(chunk); }
+
+// A sum as an unevaluated pair h + l, with the sum of its terms' magnitudes
+// (what its error is measured by: below 2^-43 a).
+struct Sum2 {
+	float h, l, a;
 };
 
-template <>
-struct CgTeam<false> {
-	cooperative_groups::cluster_group c;
-	__device__ CgTeam() : c(cooperative_groups::this_cluster()) {}
-	__device__ int rank() const { return (int)c.block_rank(); }
-	__device__ int size() const { return (int)c.num_blocks(); }
-	__device__ void sync() { c.sync(); }
-	template <class T>
-	__device__ T *map(T *p, int r)
-	{
-		return c.map_shared_rank(p, r);
-	}
+__device__ __forceinline__ Sum2 sum2(float v) { return {v, 0.f, fabsf(v)}; }
+
+__device__ __forceinline__ Sum2 sum2_add(Sum2 x, Sum2 y)
+{
+	const float s = x.h + y.h, t = s - x.h;
+	float e = (x.h - (s - t)) + (y.h - t);  // exact (two-sum)
+	e += x.l + y.l;
+	const float h = s + e;
+	return {h, e - (h - s), x.a + y.a};
+}
+
+__device__ __forceinline__ Sum2 sum2_shfl(Sum2 x, int o)
+{
+	return {__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o),
+	        __shfl_xor_sync(0xffffffffu, x.a, o)};
+}
+
+// The sum over 16 lanes, of which the warp's halves hold the same: every lane
+// of the warp ends with the same total.
+__device__ __forceinline__ Sum2 sum2_16(Sum2 x)
+{
+#pragma unroll
+	for (int o = 8; o > 0; o >>= 1) x = sum2_add(x, sum2_shfl(x, o));
+	return x;
+}
+
+// Bounds of what the pair arithmetic takes: nothing in it can over- or
+// underflow.
+__device__ __forceinline__ bool sum2_safe(float v) { return fabsf(v) >= 1e-18f && fabsf(v) <= 1e18f; }
+
+// float(n / d) of the double sums that n and d approximate; false where the
+// pairs do not decide it.
+__device__ __forceinline__ bool sum2_quotient(Sum2 n, Sum2 d, float &q)
+{
+	const float y = __fdividef(1.0f, d.h);
+	const float q0 = n.h * y;
+	const float rem = fmaf(-q0, d.l, fmaf(-q0, d.h, n.h) + n.l);
+	const float q1 = rem * y;
+	const float m = fabsf(q0) * 0x1p-40f * (2.0f + d.a * fabsf(y));
+	const float lo = q0 + (q1 - m), hi = q0 + (q1 + m);
+	q = lo;
+	return lo == hi && sum2_safe(n.h) && sum2_safe(d.h) && sum2_safe(q0) && d.a <= 1e18f;
+}
+
+__device__ __forceinline__ uint32_t cg_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ uint32_t cg_remote(uint32_t addr, int rank)
+{
+	uint32_t a;
+	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+	return a;
+}
+
+// Asynchronous stores into a CTA of the cluster (addresses from cg_remote)
+// that complete on its mbarrier.
+__device__ __forceinline__ void cg_send(uint32_t dst, float2 v, uint32_t bar)
+{
+	asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(dst),
+	             "f"(v.x), "f"(v.y), "r"(bar)
+	             : "memory");
+}
+
+__device__ __forceinline__ void cg_send(uint32_t dst, float4 v, uint32_t bar)
+{
+	asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+	             "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
+	             : "memory");
+}
+
+__device__ __forceinline__ void cg_send(uint32_t dst, double v, uint32_t bar)
+{
+	asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+	             "l"(__double_as_longlong(v)), "r"(bar)
+	             : "memory");
+}
+
+// One arrival and `bytes` to come for the barrier's current phase.
+__device__ __forceinline__ void cg_expect(uint32_t bar, uint32_t bytes)
+{
+	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+// Waits for phase `parity`; false when the bounded wait ran out (each poll
+// suspends for a microsecond at most: about a second in all).
+__device__ __forceinline__ bool cg_wait(uint32_t bar, uint32_t parity)
+{
+	constexpr uint32_t kPolls = 1u << 20, kPollNs = 1000u;
+	uint32_t ok = 0;
+	for (uint32_t i = 0; i < kPolls && !ok; i++)
+		asm volatile(
+		    "{\n\t.reg .pred p;\n\t"
+		    "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+		    "selp.u32 %0, 1, 0, p;\n\t}"
+		    : "=r"(ok)
+		    : "r"(bar), "r"(parity), "r"(kPollNs)
+		    : "memory");
+	return ok != 0;
+}
+
+// Shared memory of a solve beside the pairs.
+enum CgBar { kBarStencil = 0, kBarUpdate = 1, kBarDouble = 2 };
+
+template <bool PRE>
+struct CgShared {
+	static constexpr int NV = PRE ? 2 : 1;  // sums of the update phase: |r|^2 (and <r, z>)
+	float4 sumA[kClusterMax], sumB[NV][kClusterMax];  // every CTA's, by rank
+	double dbl[2][kClusterMax];
+	uint64_t bar[3];
+	float redA[16], redB[2][NV][16];  // this CTA's warps'; the update phase's last two
+	double red[kClusterBlock / 32];
+	float coef;
+	int active, ghosts;
+	uint32_t doubles;  // exchanges on kBarDouble so far
+	int failed;        // a wait ran out
 };
 
-// The solve of channel group `group` (channels [group * C, (group + 1) * C)
-// of the a.C-channel image) by the team's CTAs.
-template <int C, bool PRE, bool SINGLE>
+// The sum over the cluster in double, of warp sums red (16 per CTA): per CTA a
+// shuffle tree over its warps, then one over the CTAs.  Called by warp 0 of
+// every CTA alike; every lane returns the total.
+template <bool PRE, bool SINGLE>
+__device__ __noinline__ double cg_double_total(CgShared<PRE> &sh, const float *red, int rank, int ncta)
+{
+	const int lane = threadIdx.x & 31;
+	double v = warp_sum(lane < 16 ? (double)red[lane] : 0.0);
+	v = __shfl_sync(0xffffffffu, v, 0);
+	if (SINGLE) return v;
+	const uint32_t n = sh.doubles, bar = cg_u32(&sh.bar[kBarDouble]);
+	__syncwarp();
+	if (lane < ncta) cg_send(cg_remote(cg_u32(&sh.dbl[n & 1][rank]), lane), v, cg_remote(bar, lane));
+	const bool ok = __all_sync(0xffffffffu, cg_wait(bar, n & 1));
+	if (lane == 0) {
+		cg_expect(bar, ncta * (uint32_t)sizeof(double));
+		sh.doubles = n + 1;
+		if (!ok) sh.failed = 1;
+	}
+	__syncwarp();
+	v = warp_sum(lane < ncta ? sh.dbl[n & 1][lane] : 0.0);
+	return __shfl_sync(0xffffffffu, v, 0);
+}
+
+// The solve of channel ch of the a.C-channel image by a cluster's CTAs, or by
+// one CTA on its own (SINGLE; the arithmetic of a cluster of one); U: unknowns
+// per thread at most; timeout: the context's status word.
+template <bool PRE, bool SINGLE, int U>
 __device__ __forceinline__ void cg_team_solve(const PoissonArgs &a, int chunk, const UnkC *__restrict__ unk_g,
                                               const float *__restrict__ b, const float *__restrict__ x0,
                                               int *__restrict__ iters_out, const int32_t *__restrict__ hole,
-                                              const float *orig, float *img, double *__restrict__ diff_part, int group)
+                                              const float *orig, float *img, double *__restrict__ diff_part, int ch,
+                                              int *timeout)
 {
-	constexpr int NV = PRE ? 2 * C : C;  // sums of the residual phase: |r|^2 (and <r, z>)
-	const int Ctot = a.C;
-	CgTeam<SINGLE> cluster;
-	extern __shared__ float smem[];
-	__shared__ double red[kClusterBlock / 32][8];
-	__shared__ double partA[8], partB[8], tot[8];
-	__shared__ float s_coef[4];
-	__shared__ int s_active[4];
-	__shared__ double s_nr[4], s_rho[4];
-	__shared__ float *base[3][kClusterMax];  // z (r without PRE), dA, dB of every CTA
-	const int rank = cluster.rank(), ncta = cluster.size();
-	const int cb = group * C;  // this cluster's first channel
-	b += (size_t)cb * a.nh;
-	x0 += (size_t)cb * a.nh;
-	const int nh = a.nh;
+	extern __shared__ float2 s_pair[];  // two buffers of cg_slots(chunk)
+	__shared__ __align__(16) CgShared<PRE> sh;
+	constexpr int NV = PRE ? 2 : 1;
+	int rank = 0, ncta = 1;
+	if (!SINGLE) {
+		rank = (int)cooperative_groups::this_cluster().block_rank();
+		ncta = (int)cooperative_groups::this_cluster().num_blocks();
+	}
+	const int Ctot = a.C, nh = a.nh;
+	b += (size_t)ch * nh;
+	x0 += (size_t)ch * nh;
 	const int lo = rank * chunk, own = max(0, min(nh, lo + chunk) - lo);
 	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-	const size_t vlen = (size_t)C * chunk;
-	float *s_r = smem, *s_dA = smem + vlen, *s_dB = smem + 2 * vlen, *s_x = smem + 3 * vlen;
-	float *s_z = PRE ? smem + 4 * vlen : s_r;
-	UnkC *s_unk = reinterpret_cast<UnkC *>(smem + (kClusterVectors + (PRE ? 1 : 0)) * vlen);
-	if (threadIdx.x < ncta) {
-		base[0][threadIdx.x] = cluster.map(s_z, (int)threadIdx.x);
-		base[1][threadIdx.x] = cluster.map(s_dA, (int)threadIdx.x);
-		base[2][threadIdx.x] = cluster.map(s_dB, (int)threadIdx.x);
+	const int slots = cg_slots(chunk), zero_slot = 3 * chunk + 2;
+	const float oml = 1.0f - a.lambda[ch];
+	const uint32_t bar_a = cg_u32(&sh.bar[kBarStencil]), bar_b = cg_u32(&sh.bar[kBarUpdate]);
+
+	if (threadIdx.x == 0) {
+		sh.ghosts = 0;
+		sh.doubles = 0;
+		sh.failed = 0;
+		if (!SINGLE) {
+			for (int i = 0; i < 3; i++)
+				asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cg_u32(&sh.bar[i])) : "memory");
+			asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+		}
 	}
-	for (int l = threadIdx.x; l < own; l += blockDim.x) s_unk[l] = unk_g[lo + l];
+	if (threadIdx.x < 2) s_pair[threadIdx.x * slots + zero_slot] = make_float2(0.f, 0.f);
 	__syncthreads();
 
-	// block partial sums of the first nv values into dst (written by warp 0;
-	// read by the other CTAs after the next cluster barrier)
-	auto block_reduce = [&](const float *v, double *dst, int nv) {
-#pragma unroll
-		for (int c = 0; c < NV; c++) {
-			if (c >= nv) break;
-			const float s = warp_sum(v[c]);
-			if (lane == 0) red[wid][c] = (double)s;
-		}
-		__syncthreads();
-		if (wid == 0) {
-#pragma unroll
-			for (int c = 0; c < NV; c++) {
-				if (c >= nv) break;
-				const double s = warp_sum((lane < kClusterBlock / 32) ? red[lane][c] : 0.0);
-				if (lane == 0) dst[c] = s;
-			}
-		}
-	};
-	// cluster totals of the first nv block partials src, in rank order, left
-	// in every lane of warp 0 (call from warp 0 only, after a cluster barrier)
-	auto warp0_totals = [&](const double *src, double *out, int nv) {
-#pragma unroll
-		for (int c = 0; c < NV; c++) {
-			if (c >= nv) break;
-			const double v = warp_sum((lane < ncta) ? cluster.map(const_cast<double *>(src), lane)[c] : 0.0);
-			out[c] = __shfl_sync(0xffffffffu, v, 0);
-		}
-	};
-	// channel values of vector `v` (0: z, 1: dA, 2: dB) at a 16-bit code
-	auto nb = [&](int v, uint32_t code) -> const float * {
-		const int o = (int)(code >> 12), l = (int)(code & 0xFFF);
-		const float *bp = (o == rank) ? (v == 0 ? s_z : v == 1 ? s_dA : s_dB) : base[v][o];
-		return bp + (size_t)l * C;
-	};
-
+	// this thread's unknowns: the row (up and left link, own coefficient, sum of
+	// the links, lambda S), the neighbours' slots (up | down << 16, left |
+	// right << 16) and for those of other CTAs their codes (owner << 12 | index)
+	float su[U], sl[U], sc[U], sum[U], ls[U], minv[PRE ? U : 1];
+	uint32_t nud[U], nlr[U], cud[U], clr[U];
+	float r[U], x[U], d[U], q[U];
+	float acc = 0.f, accz = 0.f;
+	int ghosts = 0;
 	// r0 = b - A x0 (x0 from global: neighbours may belong to other CTAs)
-	float facc[8];
 #pragma unroll
-	for (int c = 0; c < 8; c++) facc[c] = 0.f;
-	for (int l = threadIdx.x; l < own; l += blockDim.x) {
+	for (int u = 0; u < U; u++) {
+		const int l = threadIdx.x + u * kClusterBlock;
+		if (l >= own) break;
 		const int k = lo + l;
-		const UnkC n = s_unk[l];
+		const UnkC n = unk_g[k];
 		const uint32_t codes[4] = {n.ud >> 16, n.lr >> 16, n.ud & 0xFFFF, n.lr & 0xFFFF};
 		const float coefs[4] = {n.s_up, n.s_left, (n.links & 1) ? n.S : 0.f, (n.links & 2) ? n.S : 0.f};
-		const float sum = coefs[0] + coefs[1] + coefs[2] + coefs[3];
-		int gk[4];
+		const float sm = coefs[0] + coefs[1] + coefs[2] + coefs[3];
+		int gk[4], slot[4];
+		uint32_t far[4];
 #pragma unroll
 		for (int j = 0; j < 4; j++) {
 			gk[j] = (codes[j] != kNoNb) ? (int)(codes[j] >> 12) * chunk + (int)(codes[j] & 0xFFF) : -1;
 			if (gk[j] >= 0 && !nli_in_bounds(gk[j], nh, kSiteCgNeighbour)) gk[j] = -1;
+			const bool local = gk[j] >= 0 && (int)(codes[j] >> 12) == rank;
+			far[j] = gk[j] >= 0 && !local ? codes[j] : (uint32_t)kNoNb;
+			ghosts += far[j] != kNoNb;
+			slot[j] = gk[j] < 0 ? zero_slot
+			          : local   ? (int)(codes[j] & 0xFFF)
+			          : j == 0  ? chunk + l
+			          : j == 2  ? 2 * chunk + l
+			          : j == 1  ? 3 * chunk
+			                    : 3 * chunk + 1;
 		}
+		su[u] = n.s_up;
+		sl[u] = n.s_left;
+		sc[u] = n.S;
+		sum[u] = sm;
+		ls[u] = a.lambda[ch] * n.S;
+		nud[u] = (uint32_t)slot[0] | ((uint32_t)slot[2] << 16);
+		nlr[u] = (uint32_t)slot[1] | ((uint32_t)slot[3] << 16);
+		cud[u] = far[0] | (far[2] << 16);
+		clr[u] = far[1] | (far[3] << 16);
+		const float xk = x0[k];
+		float lap = -xk * sm;
 #pragma unroll
-		for (int c = 0; c < C; c++) {
-			const float *xc = x0 + (size_t)c * nh;
-			const float xk = xc[k];
-			float lap = -xk * sum;
-#pragma unroll
-			for (int j = 0; j < 4; j++)
-				if (gk[j] >= 0) lap += coefs[j] * xc[gk[j]];
-			const float rv = b[(size_t)c * nh + k] - (a.lambda[cb + c] * n.S * xk - (1.0f - a.lambda[cb + c]) * lap);
-			s_r[(size_t)l * C + c] = rv;
-			s_dA[(size_t)l * C + c] = 0.f;
-			s_x[(size_t)l * C + c] = xk;
-			facc[c] = fmaf(rv, rv, facc[c]);
-			if (PRE) {
-				const float zv = jacobi_inv(n, a.lambda[cb + c]) * rv;
-				s_z[(size_t)l * C + c] = zv;
-				facc[C + c] = fmaf(rv, zv, facc[C + c]);
-			}
+		for (int j = 0; j < 4; j++)
+			if (gk[j] >= 0) lap += coefs[j] * x0[gk[j]];
+		const float rv = b[k] - (a.lambda[ch] * n.S * xk - (1.0f - a.lambda[ch]) * lap);
+		r[u] = rv;
+		x[u] = xk;
+		d[u] = 0.f;
+		acc = fmaf(rv, rv, acc);
+		if (PRE) {
+			minv[u] = jacobi_inv(n, a.lambda[ch]);
+			accz = fmaf(rv, fm(minv[u], rv), accz);
 		}
 	}
-	block_reduce(facc, partB, NV);
-	cluster.sync();
-	double nr0[4], nr[4], rho[4];
-	if (wid == 0) {
-		double t[8];
-		warp0_totals(partB, t, NV);
-		if (lane == 0)
-			for (int c = 0; c < NV; c++) tot[c] = t[c];
+	if (!SINGLE && ghosts) atomicAdd(&sh.ghosts, ghosts);
+	__syncthreads();
+	// bytes an update phase brings: every CTA's sums and a pair per neighbour of
+	// an own unknown that another CTA owns (which has this one as neighbour)
+	const uint32_t bytes_a = ncta * (uint32_t)sizeof(float4);
+	const uint32_t bytes_b = NV * bytes_a + sh.ghosts * (uint32_t)sizeof(float2);
+	if (!SINGLE) {
+		if (threadIdx.x == 0) {
+			cg_expect(bar_a, bytes_a);
+			cg_expect(bar_b, bytes_b);
+			cg_expect(cg_u32(&sh.bar[kBarDouble]), ncta * (uint32_t)sizeof(double));
+		}
+		// every CTA's barriers are ready before anything is sent
+		cooperative_groups::this_cluster().sync();
+	}
+
+	// the pair of every own unknown into buffer h, and into the slots of the
+	// CTAs that have it as a neighbour: it is its upper neighbour's lower
+	// neighbour, and so on
+	auto publish = [&](int h) {
+		float2 *buf = s_pair + h * slots;
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const int l = threadIdx.x + u * kClusterBlock;
+			if (l >= own) break;
+			const float2 v = make_float2(PRE ? fm(minv[u], r[u]) : r[u], d[u]);
+			buf[l] = v;
+			if (SINGLE || (cud[u] & clr[u]) == 0xffffffffu) continue;
+			auto push = [&](uint32_t code, int slot) {
+				if (code == (uint32_t)kNoNb) return;
+				const int to = (int)(code >> 12);
+				cg_send(cg_remote(cg_u32(buf + slot), to), v, cg_remote(bar_b, to));
+			};
+			push(cud[u] & 0xFFFF, 2 * chunk + (int)(cud[u] & 0xFFF));
+			push(cud[u] >> 16, chunk + (int)((cud[u] >> 16) & 0xFFF));
+			push(clr[u] & 0xFFFF, 3 * chunk + 1);
+			push(clr[u] >> 16, 3 * chunk);
+		}
+	};
+	// warp 0, after a block barrier: the CTA's sum of red sent to every CTA
+	auto send_sum = [&](const float *red, float4 *dst, uint32_t bar) {
+		const Sum2 t = sum2_16(sum2(red[lane & 15]));
+		const float4 v = make_float4(t.h, t.l, t.a, 0.f);
+		if (SINGLE) {
+			if (lane == 0) dst[0] = v;
+			__syncwarp();
+		} else if (lane < ncta) {
+			cg_send(cg_remote(cg_u32(dst + rank), lane), v, cg_remote(bar, lane));
+		}
+	};
+	auto wait = [&](uint32_t bar, uint32_t parity, uint32_t bytes) {
+		if (SINGLE) return;
+		const bool ok = __all_sync(0xffffffffu, cg_wait(bar, parity));
+		if (lane == 0) {
+			cg_expect(bar, bytes);
+			if (!ok) sh.failed = 1;
+		}
+		__syncwarp();
+	};
+	auto total = [&](const float4 *src) {
+		const float4 v = (lane & 15) < ncta ? src[lane & 15] : make_float4(0.f, 0.f, 0.f, 0.f);
+		return sum2_16(Sum2{v.x, v.y, v.z});
+	};
+
+	publish(0);
+	acc = warp_sum(acc);
+	accz = PRE ? warp_sum(accz) : 0.f;
+	if (lane == 0) {
+		sh.redB[0][0][wid] = acc;
+		if (PRE) sh.redB[0][NV - 1][wid] = accz;
 	}
 	__syncthreads();
-#pragma unroll
-	for (int c = 0; c < C; c++) {
-		nr0[c] = tot[c];
-		rho[c] = PRE ? tot[C + c] : tot[c];
+	// warp 0 holds the solve's scalars
+	Sum2 rho = sum2(0.f), stop = sum2(0.f);  // <r, z>; tol |r0|^2
+	double nr0 = 0.0;
+	int it = 0;
+	uint32_t parity = 0;  // of the phases of bar_a (and, one ahead, of bar_b)
+	if (wid == 0) {
+		for (int v = 0; v < NV; v++) send_sum(sh.redB[0][v], sh.sumB[v], bar_b);
+		wait(bar_b, 0, bytes_b);
+		rho = total(sh.sumB[NV - 1]);
+		nr0 = cg_double_total<PRE, SINGLE>(sh, sh.redB[0][0], rank, ncta);
+		const double t = (double)a.tol * nr0;
+		stop.h = (float)t;
+		stop.l = (float)(t - (double)stop.h);
+		stop.a = fabsf(stop.h);
+		if (lane == 0) sh.active = nr0 > 0 && !sh.failed;
 	}
-	bool active[4];
-	int it[4];
-	float beta[4];
-#pragma unroll
-	for (int c = 0; c < 4; c++) {
-		nr[c] = (c < C) ? nr0[c] : 0.0;
-		if (c >= C) rho[c] = 0.0;
-		active[c] = (c < C) && (nr0[c] > 0);
-		it[c] = 0;
-		beta[c] = 0.f;
-	}
-	int h = 0;  // direction buffer holding d_old: 0 -> dA, 1 -> dB
-	float q[kClusterPerThread][C];
-	for (;;) {
-		bool any = false;
-#pragma unroll
-		for (int c = 0; c < C; c++) any |= active[c];
-		if (!any) break;
-		float *dold = h ? s_dB : s_dA, *dnew = h ? s_dA : s_dB;
+	__syncthreads();
+	bool active = sh.active != 0;
+	float beta = 0.f;
+	int h = 0;  // buffer of the current pairs
+	while (active) {
 		// d = z + beta d_old (own and neighbours) ; q = A d ; <z, q>
+		const float2 *buf = s_pair + h * slots;
+		acc = 0.f;
 #pragma unroll
-		for (int c = 0; c < 8; c++) facc[c] = 0.f;
-#pragma unroll
-		for (int u = 0; u < kClusterPerThread; u++) {
-			const int l = threadIdx.x + u * kClusterBlock;
-			if (l >= own) break;
-			const UnkC n = s_unk[l];
-			const uint32_t codes[4] = {n.ud >> 16, n.lr >> 16, n.ud & 0xFFFF, n.lr & 0xFFFF};
-			const float coefs[4] = {n.s_up, n.s_left, (n.links & 1) ? n.S : 0.f, (n.links & 2) ? n.S : 0.f};
-			const float sum = coefs[0] + coefs[1] + coefs[2] + coefs[3];
-			const float *nr_[4], *nd_[4];
-			bool has[4];
-#pragma unroll
-			for (int j = 0; j < 4; j++) {
-				// a checked build tests the code's owning CTA and index
-				has[j] = codes[j] != kNoNb &&
-				         nli_in_bounds((long long)(codes[j] >> 12) * chunk + (codes[j] & 0xFFF),
-				                       (long long)ncta * chunk, kSiteCgNeighbour) &&
-				         nli_in_bounds(codes[j] & 0xFFF, chunk, kSiteCgNeighbour);
-				nr_[j] = has[j] ? nb(0, codes[j]) : nullptr;
-				nd_[j] = has[j] ? nb(1 + h, codes[j]) : nullptr;
-			}
-#pragma unroll
-			for (int c = 0; c < C; c++) {
-				if (!active[c]) continue;
-				const size_t o = (size_t)l * C + c;
-				const float rk = s_z[o];
-				const float dk = rk + beta[c] * dold[o];
-				float lap = -dk * sum;
-#pragma unroll
-				for (int j = 0; j < 4; j++)
-					if (has[j]) lap += coefs[j] * (nr_[j][c] + beta[c] * nd_[j][c]);
-				const float qv = a.lambda[cb + c] * n.S * dk - (1.0f - a.lambda[cb + c]) * lap;
-				dnew[o] = dk;
-				q[u][c] = qv;
-				facc[c] = fmaf(rk, qv, facc[c]);
-			}
+		for (int u = 0; u < U; u++) {
+			if ((int)threadIdx.x + u * kClusterBlock >= own) break;
+			const float2 vu = buf[nud[u] & 0xFFFF], vl = buf[nlr[u] & 0xFFFF];
+			const float2 vd = buf[nud[u] >> 16], vr = buf[nlr[u] >> 16];
+			const float rk = PRE ? fm(minv[u], r[u]) : r[u];
+			const float dk = fmaf(beta, d[u], rk);
+			// a neighbour outside the hole reads zeros
+			float lap = fm(-dk, sum[u]);
+			lap = fmaf(su[u], fmaf(beta, vu.y, vu.x), lap);
+			lap = fmaf(sl[u], fmaf(beta, vl.y, vl.x), lap);
+			lap = fmaf(sc[u], fmaf(beta, vd.y, vd.x), lap);
+			lap = fmaf(sc[u], fmaf(beta, vr.y, vr.x), lap);
+			const float qv = fmaf(ls[u], dk, -fm(oml, lap));
+			d[u] = dk;
+			q[u] = qv;
+			acc = fmaf(rk, qv, acc);
 		}
-		block_reduce(facc, partA, C);
-		cluster.sync();
+		acc = warp_sum(acc);
+		if (lane == 0) sh.redA[wid] = acc;
+		__syncthreads();
 		if (wid == 0) {
-			double rq[4];
-			warp0_totals(partA, rq, C);
-#pragma unroll
-			for (int c = 0; c < C; c++)
-				if (lane == c) s_coef[c] = active[c] ? (float)(rho[c] / rq[c]) : 0.f;
+			send_sum(sh.redA, sh.sumA, bar_a);
+			wait(bar_a, parity, bytes_a);
+			float alpha;
+			if (!sum2_quotient(rho, total(sh.sumA), alpha)) {
+				const double rq = cg_double_total<PRE, SINGLE>(sh, sh.redA, rank, ncta);
+				alpha = (float)(cg_double_total<PRE, SINGLE>(sh, sh.redB[h][NV - 1], rank, ncta) / rq);
+			}
+			if (lane == 0) sh.coef = alpha;
 		}
 		__syncthreads();
-		float alpha[4];
+		const float alpha = sh.coef;
+		// r -= alpha q ; z = M r ; |r|^2 (and <r, z>) ; x += alpha d
+		acc = accz = 0.f;
 #pragma unroll
-		for (int c = 0; c < C; c++) alpha[c] = s_coef[c];
-		// x += alpha d ; r -= alpha q ; z = M r ; |r|^2 (and <r, z>)   (own unknowns only)
-#pragma unroll
-		for (int c = 0; c < 8; c++) facc[c] = 0.f;
-#pragma unroll
-		for (int u = 0; u < kClusterPerThread; u++) {
-			const int l = threadIdx.x + u * kClusterBlock;
-			if (l >= own) break;
-			float minv[C];
-			if (PRE) {
-				const UnkC n = s_unk[l];
-#pragma unroll
-				for (int c = 0; c < C; c++) minv[c] = jacobi_inv(n, a.lambda[cb + c]);
-			}
-#pragma unroll
-			for (int c = 0; c < C; c++) {
-				if (!active[c]) continue;
-				const size_t o = (size_t)l * C + c;
-				s_x[o] += alpha[c] * dnew[o];
-				const float rv = s_r[o] - alpha[c] * q[u][c];
-				s_r[o] = rv;
-				facc[c] = fmaf(rv, rv, facc[c]);
-				if (PRE) {
-					const float zv = minv[c] * rv;
-					s_z[o] = zv;
-					facc[C + c] = fmaf(rv, zv, facc[C + c]);
-				}
-			}
-		}
-		// partA / partB are rewritten only after the next cluster barrier,
-		// by which time every CTA has read them
-		block_reduce(facc, partB, NV);
-		cluster.sync();
-		if (wid == 0) {
-			double nrn[8];
-			warp0_totals(partB, nrn, NV);
-#pragma unroll
-			for (int c = 0; c < C; c++)
-				if (lane == c && active[c]) {
-					const double rhon = PRE ? nrn[C + c] : nrn[c];
-					s_coef[c] = (float)(rhon / rho[c]);
-					s_rho[c] = rhon;
-					s_nr[c] = nrn[c];
-					s_active[c] = ((nrn[c] < (double)a.tol * nr0[c]) || (it[c] >= a.limit)) ? 0 : 1;
-				}
-		}
-		__syncthreads();
-		// s_coef, s_nr and s_active are rewritten by warp 0 only after the
-		// next block barrier, by which time every thread has read them
-#pragma unroll
-		for (int c = 0; c < C; c++) {
-			if (!active[c]) continue;
-			beta[c] = s_coef[c];
-			nr[c] = s_nr[c];
-			rho[c] = s_rho[c];
-			it[c]++;
-			active[c] = s_active[c] != 0;
+		for (int u = 0; u < U; u++) {
+			if ((int)threadIdx.x + u * kClusterBlock >= own) break;
+			r[u] = fmaf(-alpha, q[u], r[u]);
+			acc = fmaf(r[u], r[u], acc);
+			if (PRE) accz = fmaf(r[u], fm(minv[u], r[u]), accz);
 		}
 		h = 1 - h;
+		publish(h);
+		acc = warp_sum(acc);
+		accz = PRE ? warp_sum(accz) : 0.f;
+		if (lane == 0) {
+			sh.redB[h][0][wid] = acc;
+			if (PRE) sh.redB[h][NV - 1][wid] = accz;
+		}
+		__syncthreads();
+		if (wid == 0) {
+			for (int v = 0; v < NV; v++) send_sum(sh.redB[h][v], sh.sumB[v], bar_b);
+			wait(bar_b, parity ^ 1u, bytes_b);
+			const Sum2 nrn = total(sh.sumB[0]), rhon = PRE ? total(sh.sumB[NV - 1]) : nrn;
+			float bt;
+			const float over = (nrn.h - stop.h) + (nrn.l - stop.l);
+			bool done = over < 0.f;
+			if (!sum2_quotient(rhon, rho, bt) || !sum2_safe(nrn.h) ||
+			    !(fabsf(over) > 0x1p-39f * (nrn.a + stop.a))) {
+				const double rn = cg_double_total<PRE, SINGLE>(sh, sh.redB[h][0], rank, ncta);
+				const double zn = PRE ? cg_double_total<PRE, SINGLE>(sh, sh.redB[h][NV - 1], rank, ncta) : rn;
+				bt = (float)(zn / cg_double_total<PRE, SINGLE>(sh, sh.redB[1 - h][NV - 1], rank, ncta));
+				done = rn < (double)a.tol * nr0;
+			}
+			if (lane == 0) {
+				sh.coef = bt;
+				sh.active = !(done || it >= a.limit || sh.failed);
+			}
+			rho = rhon;
+			it++;
+		}
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			if ((int)threadIdx.x + u * kClusterBlock >= own) break;
+			x[u] = fmaf(alpha, d[u], x[u]);
+		}
+		parity ^= 1u;
+		// the sums of a phase arrive again only after the other phase, in which
+		// every warp 0 has read them; coef and active change only after the
+		// next block barrier, by which every thread has
+		__syncthreads();
+		beta = sh.coef;
+		active = sh.active != 0;
 	}
-	if (rank == 0 && threadIdx.x < C) iters_out[cb + threadIdx.x] = it[threadIdx.x];
+	if (rank == 0 && threadIdx.x == 0) iters_out[ch] = it;
+	if (threadIdx.x == 0 && sh.failed) {
+		// the missing data may still land: one more bounded wait before leaving
+		cg_wait(bar_a, parity);
+		cg_wait(bar_b, parity ^ 1u);
+		atomicExch(timeout, 1);
+	}
 	// u = orig + delta on the hole (:89-104)
 	double dacc = 0.0;
-	for (int l = threadIdx.x; l < own; l += blockDim.x) {
-		const int pix = hole[lo + l];
 #pragma unroll
-		for (int c = 0; c < C; c++) {
-			const float o = orig[(size_t)Ctot * pix + cb + c];
-			const float v = o + s_x[(size_t)l * C + c];
-			const float prev = img[(size_t)Ctot * pix + cb + c];
-			const float dd = prev - v;
-			dacc += (double)(dd * dd);
-			img[(size_t)Ctot * pix + cb + c] = v;
-		}
+	for (int u = 0; u < U; u++) {
+		const int l = threadIdx.x + u * kClusterBlock;
+		if (l >= own) break;
+		const int pix = hole[lo + l];
+		const float o = orig[(size_t)Ctot * pix + ch];
+		const float v = o + x[u];
+		const float prev = img[(size_t)Ctot * pix + ch];
+		const float dd = prev - v;
+		dacc += (double)(dd * dd);
+		img[(size_t)Ctot * pix + ch] = v;
 	}
-	dacc = block_sum<kClusterBlock>(dacc, &red[0][0]);
-	if (threadIdx.x == 0) diff_part[group * ncta + rank] = dacc;
-	cluster.sync();  // no CTA leaves while others may still read its shared memory
+	dacc = block_sum<kClusterBlock>(dacc, sh.red);
+	if (threadIdx.x == 0) diff_part[ch * ncta + rank] = dacc;
+	// no CTA leaves while one may still send to it
+	if (!SINGLE) cooperative_groups::this_cluster().sync();
 }
 
-template <int C, bool PRE>
+// Unknowns per thread the solvers are compiled for: the registers of the
+// larger counts would leave fewer loads in flight on the smaller systems.
+constexpr int cg_per_thread(int chunk)
+{
+	return chunk <= 2 * kClusterBlock ? 2 : chunk <= 5 * kClusterBlock ? 5 : kClusterPerThread;
+}
+
+template <bool PRE, int U>
 __global__ void __launch_bounds__(kClusterBlock, 1)
     k_poisson_cg_cluster(PoissonArgs a, int chunk, const UnkC *__restrict__ unk_g, const float *__restrict__ b,
                          const float *__restrict__ x0, int *__restrict__ iters_out, const int32_t *__restrict__ hole,
-                         const float *orig, float *img, double *__restrict__ diff_part)
+                         const float *orig, float *img, double *__restrict__ diff_part, int *timeout)
 {
 	const int ncta = (int)cooperative_groups::this_cluster().num_blocks();
-	cg_team_solve<C, PRE, false>(a, chunk, unk_g, b, x0, iters_out, hole, orig, img, diff_part,
-	                             (int)blockIdx.x / ncta);
+	cg_team_solve<PRE, false, U>(a, chunk, unk_g, b, x0, iters_out, hole, orig, img, diff_part,
+	                             (int)blockIdx.x / ncta, timeout);
 }
 
 // One CTA per channel (systems of at most kClusterMaxChunk unknowns).
-template <int C, bool PRE>
+template <bool PRE, int U>
 __global__ void __launch_bounds__(kClusterBlock, 1)
     k_poisson_cg_cta(PoissonArgs a, int chunk, const UnkC *__restrict__ unk_g, const float *__restrict__ b,
                      const float *__restrict__ x0, int *__restrict__ iters_out, const int32_t *__restrict__ hole,
-                     const float *orig, float *img, double *__restrict__ diff_part)
+                     const float *orig, float *img, double *__restrict__ diff_part, int *timeout)
 {
-	cg_team_solve<C, PRE, true>(a, chunk, unk_g, b, x0, iters_out, hole, orig, img, diff_part, (int)blockIdx.x);
+	cg_team_solve<PRE, true, U>(a, chunk, unk_g, b, x0, iters_out, hole, orig, img, diff_part, (int)blockIdx.x,
+	                            timeout);
 }
 
 __global__ void k_hole_index(const int32_t *__restrict__ hole, int nh, int32_t *__restrict__ index)
@@ -1157,40 +1335,26 @@ static double read_total(nli_ctx *ctx, double *partials, int n, int *cg_iters_de
 	return *reinterpret_cast<double *>(h);
 }
 
-static void (*cluster_kernel(int CC, bool pre))(PoissonArgs, int, const UnkC *, const float *, const float *, int *,
-                                                const int32_t *, const float *, float *, double *)
+typedef void (*CgKernel)(PoissonArgs, int, const UnkC *, const float *, const float *, int *, const int32_t *,
+                         const float *, float *, double *, int *);
+
+template <bool PRE>
+static CgKernel cg_kernel(bool single, int per)
 {
-	if (pre)
-		return (CC == 1)   ? k_poisson_cg_cluster<1, true>
-		       : (CC == 2) ? k_poisson_cg_cluster<2, true>
-		       : (CC == 3) ? k_poisson_cg_cluster<3, true>
-		                   : k_poisson_cg_cluster<4, true>;
-	return (CC == 1)   ? k_poisson_cg_cluster<1, false>
-	       : (CC == 2) ? k_poisson_cg_cluster<2, false>
-	       : (CC == 3) ? k_poisson_cg_cluster<3, false>
-	                   : k_poisson_cg_cluster<4, false>;
+	if (per == 2) return single ? k_poisson_cg_cta<PRE, 2> : k_poisson_cg_cluster<PRE, 2>;
+	if (per == 5) return single ? k_poisson_cg_cta<PRE, 5> : k_poisson_cg_cluster<PRE, 5>;
+	return single ? k_poisson_cg_cta<PRE, 8> : k_poisson_cg_cluster<PRE, 8>;
 }
 
-static void (*cta_kernel(int CC, bool pre))(PoissonArgs, int, const UnkC *, const float *, const float *, int *,
-                                            const int32_t *, const float *, float *, double *)
+static CgKernel cg_kernel(bool pre, bool single, int per)
 {
-	if (pre)
-		return (CC == 1)   ? k_poisson_cg_cta<1, true>
-		       : (CC == 2) ? k_poisson_cg_cta<2, true>
-		       : (CC == 3) ? k_poisson_cg_cta<3, true>
-		                   : k_poisson_cg_cta<4, true>;
-	return (CC == 1)   ? k_poisson_cg_cta<1, false>
-	       : (CC == 2) ? k_poisson_cg_cta<2, false>
-	       : (CC == 3) ? k_poisson_cg_cta<3, false>
-	                   : k_poisson_cg_cta<4, false>;
+	return pre ? cg_kernel<true>(single, per) : cg_kernel<false>(single, per);
 }
 
-// Vectors of `chunk` floats per channel a cluster CTA keeps in shared
-// memory: r, two direction buffers, x (and z when preconditioned).
-static int cluster_vectors(bool pre) { return kClusterVectors + (pre ? 1 : 0); }
+constexpr int kCgPerThread[] = {2, 5, 8};  // cg_per_thread's values
 
-// shared-memory cluster kernel: kClusterVectors vectors x chunk floats per CTA, one cluster per channel
 constexpr size_t kSmemBudget = 216 * 1024;
+static_assert(2 * sizeof(float2) * (3 * kClusterMaxChunk + 3) <= kSmemBudget, "every chunk fits a CTA");
 
 // Solver layout of a system of nh unknowns per channel: *ncta CTAs of
 // *chunk unknowns each (one CTA with block barriers when *ncta is 1, a
@@ -1201,21 +1365,21 @@ static void cg_layout(nli_ctx *ctx, int nh, int *ncta, int *chunk)
 		// largest cluster the device runs with the biggest shared-memory footprint
 		int maxc = 0;
 		bool ok = true;
-		for (int CC = 1; CC <= 4; CC++)
-			for (int pre = 0; pre < 2; pre++) {
-				ok &= cudaFuncSetAttribute(cluster_kernel(CC, pre), cudaFuncAttributeNonPortableClusterSizeAllowed,
-				                           1) == 0;
-				ok &= cudaFuncSetAttribute(cluster_kernel(CC, pre), cudaFuncAttributeMaxDynamicSharedMemorySize,
-				                           (int)kSmemBudget) == 0;
-				ok &= cudaFuncSetAttribute(cta_kernel(CC, pre), cudaFuncAttributeMaxDynamicSharedMemorySize,
-				                           (int)kSmemBudget) == 0;
+		for (int pre = 0; pre < 2; pre++)
+			for (int per : kCgPerThread) {
+				const CgKernel cluster = cg_kernel(pre, false, per), cta = cg_kernel(pre, true, per);
+				ok &= cudaFuncSetAttribute(cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == 0;
+				ok &= cudaFuncSetAttribute(cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget) == 0;
+				ok &= cudaFuncSetAttribute(cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget) == 0;
 			}
 		if (ok) {
 			cudaLaunchConfig_t qc = {};
 			qc.gridDim = dim3(kClusterMax);
 			qc.blockDim = dim3(kClusterBlock);
 			qc.dynamicSmemBytes = kSmemBudget;
-			if (cudaOccupancyMaxPotentialClusterSize(&maxc, cluster_kernel(4, true), &qc) != cudaSuccess) maxc = 0;
+			if (cudaOccupancyMaxPotentialClusterSize(&maxc, cg_kernel(true, false, kClusterPerThread), &qc) !=
+			    cudaSuccess)
+				maxc = 0;
 		}
 		cudaGetLastError();
 		ctx->cg_cluster_max = std::min(maxc, kClusterMax);
@@ -1225,10 +1389,8 @@ static void cg_layout(nli_ctx *ctx, int nh, int *ncta, int *chunk)
 		const int per = std::max(1, ctx->tune_cg_unknowns_per_cta);
 		*ncta = std::max(1, std::min(std::min(ctx->cg_cluster_max, ctx->tune_cg_cluster_cap), (nh + per - 1) / per));
 		*chunk = (nh + *ncta - 1) / *ncta;
-		if ((size_t)cluster_vectors(ctx->tune_cg_precond) * *chunk * sizeof(float) + *chunk * sizeof(UnkC) >
-		        kSmemBudget ||
-		    *chunk > kClusterMaxChunk)
-			*ncta = *chunk = 0;
+		// (a 16-bit code names a neighbour, and the last one means none)
+		if (*chunk > kClusterMaxChunk || nh > kNoNb) *ncta = *chunk = 0;
 		// small systems: one CTA, block barriers only (NLI_TUNE_CG_SINGLE_MAX)
 		if (nh <= std::min(ctx->tune_cg_single_max, kClusterMaxChunk)) {
 			*ncta = 1;
@@ -1363,7 +1525,8 @@ static int poisson_solve(nli_ctx *ctx, PoissonSystem &P, const int32_t *hole, co
 	int *iters = ctx->buf<int>("poi.iters", 4);
 	if (P.ncta > 0) {
 		const bool pre = ctx->tune_cg_precond != 0;
-		const size_t smem = (size_t)cluster_vectors(pre) * P.chunk * sizeof(float) + P.chunk * sizeof(UnkC);
+		const size_t smem = cg_smem_bytes(P.chunk);
+		const CgKernel kern = cg_kernel(pre, P.ncta == 1, cg_per_thread(P.chunk));
 		UnkC *unkc = ctx->buf<UnkC>("poi.unkc", nh);
 		k_poisson_compact<<<(nh + 255) / 256, 256, 0, s>>>(P.unk, nh, P.chunk, unkc);
 		NLI_CHECK_LAUNCH();
@@ -1371,8 +1534,8 @@ static int poisson_solve(nli_ctx *ctx, PoissonSystem &P, const int32_t *hole, co
 		if (P.ncta == 1) {
 			// one CTA per channel: no cluster
 			ProfScope ps(ctx, "poisson_cg");
-			cta_kernel(1, pre)<<<C, kClusterBlock, smem, s>>>(P.pa, P.chunk, unkc, P.b, P.x, iters, hole, orig, img,
-			                                                  diff_part);
+			kern<<<C, kClusterBlock, smem, s>>>(P.pa, P.chunk, unkc, P.b, P.x, iters, hole, orig, img, diff_part,
+			                                    &ctx->status->timeout);
 			NLI_CHECK_LAUNCH();
 			return C;
 		}
@@ -1389,8 +1552,8 @@ static int poisson_solve(nli_ctx *ctx, PoissonSystem &P, const int32_t *hole, co
 		cfg.attrs = attr;
 		cfg.numAttrs = 1;
 		ProfScope ps(ctx, "poisson_cg");
-		NLI_CUDA(cudaLaunchKernelEx(&cfg, cluster_kernel(1, pre), P.pa, P.chunk, (const UnkC *)unkc, (const float *)P.b,
-		                            (const float *)P.x, iters, hole, orig, img, diff_part));
+		NLI_CUDA(cudaLaunchKernelEx(&cfg, kern, P.pa, P.chunk, (const UnkC *)unkc, (const float *)P.b,
+		                            (const float *)P.x, iters, hole, orig, img, diff_part, &ctx->status->timeout));
 		nli_count_launch_internal();
 		return C * P.ncta;
 	}
@@ -1688,10 +1851,11 @@ struct CgTask {
 struct CgArgs {
 	int n, C, ncta;
 	const int *active;
+	int *timeout;
 	CgTask t[kBatchMax];
 };
 
-template <bool PRE, bool SINGLE>
+template <bool PRE, bool SINGLE, int U>
 __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_batch(const __grid_constant__ CgArgs B)
 {
 	const int ncta = SINGLE ? 1 : B.ncta;
@@ -1700,13 +1864,21 @@ __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_batch(const __g
 	const CgTask &T = B.t[t];
 	// a stopped image: every CTA of its clusters leaves before any barrier
 	if (B.active && !B.active[T.img_index]) return;
-	cg_team_solve<1, PRE, SINGLE>(T.a, T.chunk, T.unk, T.b, T.x0, T.iters, T.hole, T.orig, T.img, T.diff, group);
+	cg_team_solve<PRE, SINGLE, U>(T.a, T.chunk, T.unk, T.b, T.x0, T.iters, T.hole, T.orig, T.img, T.diff, group,
+	                              B.timeout);
 }
 
-static void (*cg_batch_kernel(bool pre, bool single))(CgArgs)
+template <bool PRE>
+static void (*cg_batch_kernel(bool single, int per))(CgArgs)
 {
-	if (pre) return single ? k_poisson_cg_batch<true, true> : k_poisson_cg_batch<true, false>;
-	return single ? k_poisson_cg_batch<false, true> : k_poisson_cg_batch<false, false>;
+	if (per == 2) return single ? k_poisson_cg_batch<PRE, true, 2> : k_poisson_cg_batch<PRE, false, 2>;
+	if (per == 5) return single ? k_poisson_cg_batch<PRE, true, 5> : k_poisson_cg_batch<PRE, false, 5>;
+	return single ? k_poisson_cg_batch<PRE, true, 8> : k_poisson_cg_batch<PRE, false, 8>;
+}
+
+static void (*cg_batch_kernel(bool pre, bool single, int per))(CgArgs)
+{
+	return pre ? cg_batch_kernel<true>(single, per) : cg_batch_kernel<false>(single, per);
 }
 
 static std::string lk_name(int i, const char *what) { return "lk." + std::to_string(i) + "." + what; }
@@ -1859,13 +2031,14 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 		const uint32_t bit = 1u << (ctx->device & 31);
 		if (!(raised.load(std::memory_order_acquire) & bit)) {
 			for (int pr = 0; pr < 2; pr++)
-				for (int sg = 0; sg < 2; sg++) {
-					NLI_CUDA(cudaFuncSetAttribute(cg_batch_kernel(pr, sg), cudaFuncAttributeMaxDynamicSharedMemorySize,
-					                              (int)kSmemBudget));
-					if (!sg)
-						NLI_CUDA(cudaFuncSetAttribute(cg_batch_kernel(pr, sg),
-						                              cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-				}
+				for (int sg = 0; sg < 2; sg++)
+					for (int per : kCgPerThread) {
+						const auto kern = cg_batch_kernel(pr, sg, per);
+						NLI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+						                              (int)kSmemBudget));
+						if (!sg)
+							NLI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+					}
 			raised.fetch_or(bit, std::memory_order_release);
 		}
 	}
@@ -1875,6 +2048,7 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 		G.C = C;
 		G.ncta = ncta;
 		G.active = active;
+		G.timeout = &ctx->status->timeout;
 		int maxchunk = 0;
 		for (int t = 0; t < P.n; t++) {
 			const BTask &T = P.t[t];
@@ -1894,10 +2068,11 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 			maxchunk = std::max(maxchunk, T.chunk);
 		}
 		if (G.n == 0) continue;
-		const size_t smem = (size_t)cluster_vectors(pre) * maxchunk * sizeof(float) + maxchunk * sizeof(UnkC);
+		const size_t smem = cg_smem_bytes(maxchunk);
+		const auto kern = cg_batch_kernel(pre, ncta == 1, cg_per_thread(maxchunk));
 		ProfScope ps(ctx, "poisson_cg");
 		if (ncta == 1) {
-			cg_batch_kernel(pre, true)<<<G.n * C, kClusterBlock, smem, s>>>(G);
+			kern<<<G.n * C, kClusterBlock, smem, s>>>(G);
 			NLI_CHECK_LAUNCH();
 			continue;
 		}
@@ -1913,7 +2088,7 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 		attr[0].val.clusterDim.z = 1;
 		cfg.attrs = attr;
 		cfg.numAttrs = 1;
-		NLI_CUDA(cudaLaunchKernelEx(&cfg, cg_batch_kernel(pre, false), G));
+		NLI_CUDA(cudaLaunchKernelEx(&cfg, kern, G));
 		nli_count_launch_internal();
 	}
 	// systems too large for a cluster: the cooperative grid CG, one at a time
