@@ -542,6 +542,7 @@ __device__ __forceinline__ float jacobi_inv_grid(const Unknown &n, float lam)
 	return (dg > 0.f) ? 1.0f / dg : 1.0f;
 }
 
+// The solver of systems larger than the SMs hold (see k_poisson_cg_wide).
 // Conjugate gradient of conjugte_gradient (:387-477) for all channels at
 // once: r = b - A x0, d = r; per iteration q = A d, alpha = |r|^2 / <r,q>,
 // x += alpha d, r -= alpha q, beta = |r_new|^2 / |r|^2, d = r + beta d; a
@@ -1297,6 +1298,382 @@ __global__ void __launch_bounds__(kClusterBlock, 1)
 	                            timeout);
 }
 
+// ------------------------------------------------ CG over the whole grid
+// Systems too large for a cluster: the cluster CG's scheme with its CTAs on
+// every SM and the exchanges through L2.  A group of `ctas` CTAs solves one
+// channel, up to C groups side by side (a cooperative launch: all are
+// resident); each CTA owns a contiguous range of at most 4096 unknowns whose
+// rows and vectors stay in its registers and shared memory.
+//
+// What crosses: the (r, d) pair of an unknown with a neighbour in another
+// range, and each CTA's sums.  A value travels in a 64-bit word with the
+// number of its exchange in the upper half, stored and polled with relaxed
+// accesses: data and flag arrive as one, so nothing is fenced, no barrier is
+// taken, and a CTA waits for exactly what it reads: warp 0 for the sums (it
+// holds the solve's scalars), the others meanwhile for the pairs that the
+// next stencil needs, several loads in flight.  The words are cleared
+// before the launch.  Pairs alternate between two buffers; sums need one per
+// phase, because a CTA sends its next of a phase only after it has had every
+// CTA's of the other, which they send after reading the last.
+//
+// The per-thread and per-CTA sums are pairs of floats (exact to 2^-43 of their
+// terms' magnitudes, products included), in place of the double sums of
+// k_poisson_cg.
+//
+// 1024 x 685 (175 000 unknowns, 3 x 50 CTAs, 117 iterations a channel, ncu): 1255
+// us, 10.7 us an iteration, of which the two exchanges take about 8: between
+// 50 CTAs of both dies one takes 3700 to 4200 cycles on its own, between 8
+// neighbouring ones 800 to 1500.  k_poisson_cg, with three grid barriers and
+// its vectors in L2, took 4520 us.
+struct GridCgArgs {
+	PoissonArgs a;
+	int chunk, ctas, ch0;
+	const Unknown *unk;
+	const float *b, *x0;
+	ulonglong2 *pairs;  // [2][groups of the launch][nh]
+	ulonglong2 *sums;   // [groups of the launch][1 + NV][ctas]
+	DevStatus *st;
+	int *iters;
+	const int32_t *hole;
+	const float *orig;
+	float *img;
+	double *diff;
+	const int *active;
+};
+
+// Running sum of products as a pair.
+struct Dot2 {
+	float h = 0.f, l = 0.f;
+	__device__ __forceinline__ void add(float a, float b)
+	{
+		const float p = fm(a, b), e = fmaf(a, b, -p);
+		const float s = h + p, t = s - h;
+		l += ((h - (s - t)) + (p - t)) + e;
+		h = s;
+	}
+};
+
+__device__ __forceinline__ void grid_put(ulonglong2 *p, float x, float y, uint32_t tag)
+{
+	const unsigned long long t = (unsigned long long)tag << 32;
+	asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(t | __float_as_uint(x)),
+	             "l"(t | __float_as_uint(y))
+	             : "memory");
+}
+
+// Polls the words p[i], i < n <= N, until all carry `tag`, the loads of a round
+// in flight together; false when the bounded wait ran out (here or, told by
+// the status word, elsewhere).
+template <int N>
+__device__ __forceinline__ bool grid_get(const ulonglong2 *const (&p)[N], int n, uint32_t tag, float2 (&v)[N],
+                                         DevStatus *st, unsigned limit)
+{
+	for (unsigned polls = 0;; polls++) {
+		unsigned long long x[N], y[N];
+#pragma unroll
+		for (int i = 0; i < N; i++)
+			if (i < n)
+				asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x[i]), "=l"(y[i]) : "l"(p[i]) : "memory");
+		bool all = true;
+#pragma unroll
+		for (int i = 0; i < N; i++)
+			if (i < n) {
+				all &= (uint32_t)(x[i] >> 32) == tag && (uint32_t)(y[i] >> 32) == tag;
+				v[i] = make_float2(__uint_as_float((uint32_t)x[i]), __uint_as_float((uint32_t)y[i]));
+			}
+		if (all) return true;
+		if (polls >= limit || ((polls & 255u) == 255u && *(volatile int *)&st->timeout)) {
+			atomicExch(&st->timeout, 1);
+			return false;
+		}
+	}
+}
+
+template <bool PRE, int U>
+__global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __grid_constant__ GridCgArgs A)
+{
+	// a batch image that has stopped iterating: every block leaves at once
+	if (A.active && *A.active == 0) return;
+	constexpr int NV = PRE ? 2 : 1;
+	extern __shared__ float2 s_pair[];  // two buffers of cg_slots(chunk)
+	__shared__ float2 s_red[NV][16];
+	__shared__ double s_dbl[kClusterBlock / 32];
+	__shared__ float s_coef;
+	__shared__ int s_active, s_failed;
+	__shared__ uint32_t s_far[32];  // of warp 0
+	const int ctas = A.ctas, chunk = A.chunk;
+	const int group = (int)blockIdx.x / ctas, rank = (int)blockIdx.x - group * ctas;
+	const int ch = A.ch0 + group, C = A.a.C, nh = A.a.nh;
+	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+	const int lo = rank * chunk, own = max(0, min(nh, lo + chunk) - lo);
+	const int slots = cg_slots(chunk), zero_slot = 3 * chunk + 2;
+	const float lambda = A.a.lambda[ch], oml = 1.0f - lambda;
+	const float *b = A.b + (size_t)ch * nh, *x0 = A.x0 + (size_t)ch * nh;
+	const int groups = (int)gridDim.x / ctas;
+	uint32_t *s_step = reinterpret_cast<uint32_t *>(s_pair + 2 * slots);  // [chunk], see below
+	ulonglong2 *pairs = A.pairs + (size_t)group * nh;
+	const size_t pair_stride = (size_t)groups * nh;  // between the two buffers
+	ulonglong2 *sums = A.sums + (size_t)group * (1 + NV) * ctas;
+	const unsigned set = *(volatile unsigned *)&A.st->wait_limit;
+	const unsigned limit = set ? set : 1u << 22;  // some seconds
+
+	if (threadIdx.x == 0) s_failed = 0;
+	if (threadIdx.x < 2) s_pair[threadIdx.x * slots + zero_slot] = make_float2(0.f, 0.f);
+
+	// this thread's unknowns: the row, the neighbours' slots, and which
+	// neighbours lie in other ranges (far); the distance to the upper and
+	// lower neighbour (up | down << 16) is in s_step
+	float su[U], sl[U], sc[U], sum[U], ls[U], minv[PRE ? U : 1];
+	uint32_t nud[U], nlr[U];
+	uint32_t far = 0;  // 4 bits per unknown: up, left, down, right
+	float r[U], x[U], d[U], q[U];
+	Dot2 acc, accz;
+#pragma unroll
+	for (int u = 0; u < U; u++) {
+		const int l = threadIdx.x + u * kClusterBlock;
+		if (l >= own) break;
+		const int k = lo + l;
+		const Unknown n = A.unk[k];
+		const int m[4] = {n.n_up, n.n_left, n.n_down, n.n_right};
+		const float coefs[4] = {n.s_up, n.s_left, n.s_down, n.s_right};
+		const float xk = x0[k];
+		sum[u] = n.s_up + n.s_left + n.s_down + n.s_right;
+		float lap = fm(-xk, sum[u]);
+		int slot[4];
+#pragma unroll
+		for (int j = 0; j < 4; j++) {
+			const bool there = m[j] >= 0 && nli_in_bounds(m[j], nh, kSiteCgNeighbour);
+			const bool local = there && m[j] >= lo && m[j] < lo + own;
+			if (there && !local) far |= 1u << (4 * u + j);
+			if (there) lap = fmaf(coefs[j], x0[m[j]], lap);
+			slot[j] = !there ? zero_slot : local ? m[j] - lo : j == 0 ? chunk + l : j == 2 ? 2 * chunk + l : 3 * chunk + (j == 3);
+		}
+		su[u] = n.s_up;
+		sl[u] = n.s_left;
+		sc[u] = n.S;
+		ls[u] = fm(lambda, n.S);
+		nud[u] = (uint32_t)slot[0] | ((uint32_t)slot[2] << 16);
+		nlr[u] = (uint32_t)slot[1] | ((uint32_t)slot[3] << 16);
+		s_step[l] = ((uint32_t)(k - n.n_up) & 0xFFFFu) | ((uint32_t)(n.n_down - k) << 16);
+		const float rv = b[k] - fmaf(ls[u], xk, -fm(oml, lap));
+		r[u] = rv;
+		x[u] = xk;
+		d[u] = 0.f;
+		acc.add(rv, rv);
+		if (PRE) {
+			minv[u] = jacobi_inv_grid(n, lambda);
+			accz.add(rv, fm(minv[u], rv));
+		}
+	}
+	// the pair of every own unknown into buffer h, and with the exchange's number
+	// for the CTAs that have it as a neighbour
+	auto publish = [&](int h, uint32_t tag) {
+		float2 *buf = s_pair + h * slots;
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const int l = threadIdx.x + u * kClusterBlock;
+			if (l >= own) break;
+			const float2 v = make_float2(PRE ? fm(minv[u], r[u]) : r[u], d[u]);
+			buf[l] = v;
+			if (far >> (4 * u) & 15u) grid_put(pairs + h * pair_stride + lo + l, v.x, v.y, tag);
+		}
+	};
+	// the pairs of the neighbours in other ranges (f) of thread t's unknowns into
+	// their slots, four loads in flight
+	auto fetch_for = [&](int t, uint32_t f, int h, uint32_t tag) {
+		float2 *buf = s_pair + h * slots;
+		const ulonglong2 *from = pairs + h * pair_stride + lo;
+		while (f) {
+			const ulonglong2 *p[4];
+			int slot[4], n = 0;
+#pragma unroll
+			for (int i = 0; i < 4; i++) {
+				p[i] = nullptr;
+				slot[i] = 0;
+				if (f) {
+					const int bit = __ffs(f) - 1, j = bit & 3, l = t + (bit >> 2) * kClusterBlock;
+					f &= f - 1;
+					const uint32_t st = s_step[l];
+					p[i] = from + l + (j == 0 ? -(int)(st & 0xFFFFu) : j == 1 ? -1 : j == 2 ? (int)(st >> 16) : 1);
+					slot[i] = j == 0 ? chunk + l : j == 2 ? 2 * chunk + l : 3 * chunk + (j == 3);
+					n++;
+				}
+			}
+			float2 v[4];
+			if (!grid_get(p, n, tag, v, A.st, limit)) {
+				s_failed = 1;
+				return;
+			}
+#pragma unroll
+			for (int i = 0; i < 4; i++)
+				if (i < n) buf[slot[i]] = v[i];
+		}
+	};
+	// every warp but the first for itself, the second for the first too
+	auto fetch = [&](int h, uint32_t tag) {
+		fetch_for((int)threadIdx.x, far, h, tag);
+		if (wid == 1) fetch_for(lane, s_far[lane], h, tag);
+	};
+	if (wid == 0) s_far[lane] = far;
+	// a warp's sum into s_red
+	auto warp_pair = [&](const Dot2 &v, float2 *red) {
+		Sum2 t = {v.h, v.l, 0.f};
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) t = sum2_add(t, sum2_shfl(t, o));
+		if (lane == 0) red[wid] = make_float2(t.h, t.l);
+	};
+	// warp 0, after a block barrier: the CTA's sum to the group, and the group's
+	auto send = [&](int v, ulonglong2 *row, uint32_t tag) {
+		const float2 w = s_red[v][lane & 15];
+		const Sum2 t = sum2_16(Sum2{w.x, w.y, 0.f});
+		if (lane == 0) grid_put(row + rank, t.h, t.l, tag);
+	};
+	auto total = [&](const ulonglong2 *row, uint32_t tag) {
+		Sum2 t = {0.f, 0.f, 0.f};
+		bool ok = true;
+		constexpr int kRounds = 5;  // up to 160 CTAs
+		const ulonglong2 *p[kRounds];
+		float2 v[kRounds];
+		int n = 0;
+#pragma unroll
+		for (int i = 0; i < kRounds; i++) {
+			p[i] = row + lane + 32 * i;
+			v[i] = make_float2(0.f, 0.f);
+			n += lane + 32 * i < ctas;
+		}
+		if (n > 0) ok = grid_get(p, n, tag, v, A.st, limit);
+#pragma unroll
+		for (int i = 0; i < kRounds; i++)
+			if (i < n) t = sum2_add(t, Sum2{v[i].x, v[i].y, 0.f});
+		__syncwarp();
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) t = sum2_add(t, sum2_shfl(t, o));
+		if (!ok) s_failed = 1;
+		__syncwarp();
+		return t;
+	};
+	auto quotient = [&](Sum2 n, Sum2 m) -> float {
+		if (!(sum2_safe(n.h) && sum2_safe(m.h)))
+			return (float)(((double)n.h + (double)n.l) / ((double)m.h + (double)m.l));
+		const float y = __fdividef(1.0f, m.h), q0 = n.h * y;
+		return q0 + fmaf(-q0, m.l, fmaf(-q0, m.h, n.h) + n.l) * y;
+	};
+
+	publish(0, 1u);
+	warp_pair(acc, s_red[0]);
+	if (PRE) warp_pair(accz, s_red[NV - 1]);
+	__syncthreads();
+	// warp 0 holds the solve's scalars
+	Sum2 rho = {0.f, 0.f, 0.f}, stop = rho;  // <r, z>; tol |r0|^2
+	int it = 0;
+	uint32_t tag = 1u;  // of the current pairs
+	if (wid != 0) {
+		fetch(0, tag);
+	} else {
+		for (int v = 0; v < NV; v++) send(v, sums + (1 + v) * ctas, tag);
+		const Sum2 nr0 = total(sums + ctas, tag);
+		rho = PRE ? total(sums + NV * ctas, tag) : nr0;
+		const double t = (double)A.a.tol * ((double)nr0.h + (double)nr0.l);
+		stop.h = (float)t;
+		stop.l = (float)(t - (double)stop.h);
+		if (lane == 0) s_active = nr0.h > 0.f && !s_failed;
+	}
+	__syncthreads();
+	bool active = s_active != 0;
+	float beta = 0.f;
+	int h = 0;  // buffer of the current pairs
+	while (active) {
+		// d = z + beta d_old (own and neighbours) ; q = A d ; <z, q>
+		const float2 *buf = s_pair + h * slots;
+		acc = Dot2();
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			if ((int)threadIdx.x + u * kClusterBlock >= own) break;
+			const float2 vu = buf[nud[u] & 0xFFFF], vl = buf[nlr[u] & 0xFFFF];
+			const float2 vd = buf[nud[u] >> 16], vr = buf[nlr[u] >> 16];
+			const float rk = PRE ? fm(minv[u], r[u]) : r[u];
+			const float dk = fmaf(beta, d[u], rk);
+			// a neighbour outside the hole reads zeros
+			float lap = fm(-dk, sum[u]);
+			lap = fmaf(su[u], fmaf(beta, vu.y, vu.x), lap);
+			lap = fmaf(sl[u], fmaf(beta, vl.y, vl.x), lap);
+			lap = fmaf(sc[u], fmaf(beta, vd.y, vd.x), lap);
+			lap = fmaf(sc[u], fmaf(beta, vr.y, vr.x), lap);
+			q[u] = fmaf(ls[u], dk, -fm(oml, lap));
+			d[u] = dk;
+			acc.add(rk, q[u]);
+		}
+		warp_pair(acc, s_red[0]);
+		__syncthreads();
+		if (wid == 0) {
+			send(0, sums, tag);
+			const float alpha = quotient(rho, total(sums, tag));
+			if (lane == 0) s_coef = alpha;
+		}
+		__syncthreads();
+		const float alpha = s_coef;
+		// r -= alpha q ; z = M r ; |r|^2 (and <r, z>) ; x += alpha d
+		acc = Dot2();
+		accz = Dot2();
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			if ((int)threadIdx.x + u * kClusterBlock >= own) break;
+			r[u] = fmaf(-alpha, q[u], r[u]);
+			acc.add(r[u], r[u]);
+			if (PRE) accz.add(r[u], fm(minv[u], r[u]));
+		}
+		h = 1 - h;
+		tag++;
+		publish(h, tag);
+		warp_pair(acc, s_red[0]);
+		if (PRE) warp_pair(accz, s_red[NV - 1]);
+		__syncthreads();
+		if (wid != 0) {
+			fetch(h, tag);
+		} else {
+			for (int v = 0; v < NV; v++) send(v, sums + (1 + v) * ctas, tag);
+			const Sum2 nrn = total(sums + ctas, tag);
+			const Sum2 rhon = PRE ? total(sums + NV * ctas, tag) : nrn;
+			const float bt = quotient(rhon, rho);
+			const bool done = (nrn.h - stop.h) + (nrn.l - stop.l) < 0.f;
+			if (lane == 0) {
+				s_coef = bt;
+				s_active = !(done || it >= A.a.limit || s_failed);
+			}
+			rho = rhon;
+			it++;
+		}
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			if ((int)threadIdx.x + u * kClusterBlock >= own) break;
+			x[u] = fmaf(alpha, d[u], x[u]);
+		}
+		// s_coef and s_active change only after the next block barrier, by
+		// which every thread has read them
+		__syncthreads();
+		beta = s_coef;
+		active = s_active != 0;
+	}
+	if (rank == 0 && threadIdx.x == 0) A.iters[ch] = it;
+	if (s_failed) return;  // reported by the status word
+	// u = orig + delta on the hole (:89-104)
+	double dacc = 0.0;
+#pragma unroll
+	for (int u = 0; u < U; u++) {
+		const int l = threadIdx.x + u * kClusterBlock;
+		if (l >= own) break;
+		const int pix = A.hole[lo + l];
+		const float o = A.orig[(size_t)C * pix + ch];
+		const float v = o + x[u];
+		const float prev = A.img[(size_t)C * pix + ch];
+		const float dd = prev - v;
+		dacc += (double)(dd * dd);
+		A.img[(size_t)C * pix + ch] = v;
+	}
+	dacc = block_sum<kClusterBlock>(dacc, s_dbl);
+	if (threadIdx.x == 0) A.diff[ch * ctas + rank] = dacc;
+}
+
 __global__ void k_hole_index(const int32_t *__restrict__ hole, int nh, int32_t *__restrict__ index)
 {
 	const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1460,18 +1837,111 @@ static PoissonSystem poisson_system(nli_ctx *ctx, const UpdArgs &u, const nli_up
 	return P;
 }
 
-// Blocks of the cooperative grid CG for nh unknowns: co-resident, at most
-// one per SM.
-static int grid_cg_blocks(nli_ctx *ctx, int nh)
+// Layout of a system that is too large for a cluster: `groups` channels at a
+// time on `ctas` CTAs each (k_poisson_cg_wide; as many channels at once as the
+// SMs can hold, since an iteration costs two exchanges whatever its size), or
+// groups = 0 for k_poisson_cg, which keeps its vectors in memory: more unknowns
+// than the SMs hold, or rows too wide for a neighbour's distance.
+struct GridLayout {
+	int groups, ctas, chunk;
+	int parts;  // partial sums of (du)^2
+};
+
+typedef void (*WideKernel)(GridCgArgs);
+
+// two buffers of pairs and a word per unknown
+static size_t wide_smem_bytes(int chunk) { return cg_smem_bytes(chunk) + sizeof(uint32_t) * (size_t)chunk; }
+static_assert(2 * sizeof(float2) * (3 * kClusterMaxChunk + 3) + 4 * kClusterMaxChunk <= kSmemBudget, "every chunk fits");
+
+static WideKernel wide_kernel(bool pre, int chunk)
 {
-	int dev_blocks_per_sm = 0;
+	if (chunk <= 5 * kClusterBlock) return pre ? k_poisson_cg_wide<true, 5> : k_poisson_cg_wide<false, 5>;
+	return pre ? k_poisson_cg_wide<true, kClusterPerThread> : k_poisson_cg_wide<false, kClusterPerThread>;
+}
+
+static GridLayout grid_layout(nli_ctx *ctx, int nh, int C, int W)
+{
+	GridLayout g = {0, 0, 0, 0};
 	const bool pre = ctx->tune_cg_precond != 0;
+	if (W <= 0xFFFF)
+		for (int groups = C; groups >= 1 && g.groups == 0; groups--) {
+			const int ctas = std::min({ctx->num_sms / groups, (nh + kClusterBlock - 1) / kClusterBlock, 160});
+			const int chunk = ctas > 0 ? (nh + ctas - 1) / ctas : nh;
+			if (chunk <= kClusterMaxChunk) g = {groups, ctas, chunk, C * ctas};
+		}
+	if (g.groups > 0) {
+		static std::atomic<uint32_t> raised{0};  // one bit per device
+		const uint32_t bit = 1u << (ctx->device & 31);
+		if (!(raised.load(std::memory_order_acquire) & bit)) {
+			for (int pr = 0; pr < 2; pr++)
+				for (int c : {1, kClusterMaxChunk})
+					NLI_CUDA(cudaFuncSetAttribute(wide_kernel(pr, c), cudaFuncAttributeMaxDynamicSharedMemorySize,
+					                              (int)kSmemBudget));
+			raised.fetch_or(bit, std::memory_order_release);
+		}
+		return g;
+	}
+	int per_sm = 0;
 	const void *kern = pre ? (const void *)k_poisson_cg<true> : (const void *)k_poisson_cg<false>;
-	NLI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dev_blocks_per_sm, kern, kCgBlock, 0));
-	const int max_blocks = dev_blocks_per_sm * ctx->num_sms;
+	NLI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCgBlock, 0));
+	const int max_blocks = per_sm * ctx->num_sms;
 	NLI_REQUIRE(max_blocks > 0, NLI_E_CUDA, "conjugate gradient kernel cannot be made resident");
-	int grid = (nh + kCgBlock - 1) / kCgBlock;
-	return std::min(std::max(grid, 1), std::min(max_blocks, ctx->num_sms));
+	const int grid = (nh + kCgBlock - 1) / kCgBlock;
+	g.ctas = g.parts = std::min(std::max(grid, 1), std::min(max_blocks, ctx->num_sms));
+	return g;
+}
+
+// A cooperative launch through the launch attribute, which stream capture
+// takes.
+static void launch_cooperative(nli_ctx *ctx, const void *kern, int grid, int block, size_t smem, void **args)
+{
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(grid);
+	cfg.blockDim = dim3(block);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = ctx->stream;
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeCooperative;
+	attr[0].val.cooperative = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = 1;
+	NLI_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
+	nli_count_launch_internal();
+}
+
+// k_poisson_cg_wide for system P.  active (may be null): a device flag; 0
+// makes every block leave at once.
+static void launch_wide_cg(nli_ctx *ctx, const PoissonSystem &P, const GridLayout &g, int *iters, const int32_t *hole,
+                           const float *orig, float *img, double *diff_part, const int *active)
+{
+	const bool pre = ctx->tune_cg_precond != 0;
+	const int nh = P.pa.nh, C = P.pa.C, rows = pre ? 3 : 2;  // sums per group and CTA
+	const size_t npairs = 2 * (size_t)g.groups * nh, nsums = (size_t)g.groups * rows * g.ctas;
+	ulonglong2 *words = ctx->buf<ulonglong2>("poi.words", npairs + nsums);
+	GridCgArgs A;
+	A.a = P.pa;
+	A.chunk = g.chunk;
+	A.ctas = g.ctas;
+	A.unk = P.unk;
+	A.b = P.b;
+	A.x0 = P.x;
+	A.pairs = words;
+	A.sums = words + npairs;
+	A.st = ctx->status;
+	A.iters = iters;
+	A.hole = hole;
+	A.orig = orig;
+	A.img = img;
+	A.diff = diff_part;
+	A.active = active;
+	ProfScope ps(ctx, "poisson_cg");
+	for (int c = 0; c < C; c += g.groups) {
+		A.ch0 = c;
+		void *args[] = {&A};
+		NLI_CUDA(cudaMemsetAsync(words, 0, sizeof(ulonglong2) * (npairs + nsums), ctx->stream));
+		launch_cooperative(ctx, (const void *)wide_kernel(pre, g.chunk), std::min(g.groups, C - c) * g.ctas,
+		                   kClusterBlock, wide_smem_bytes(g.chunk), args);
+	}
 }
 
 struct GridCgBufs {
@@ -1499,20 +1969,8 @@ static void launch_grid_cg(nli_ctx *ctx, const PoissonSystem &P, int grid, const
 	double *part = g.part;
 	void *args[] = {&pa,   &unk, &b,     &x,    (void *)&r, &d,         &q,         &z,
 	                &part, &st,  &iters, (void *)&hole, &orig, &img, &diff_part, (void *)&active};
-	// cooperative through the launch attribute, which stream capture takes
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3(grid);
-	cfg.blockDim = dim3(kCgBlock);
-	cfg.dynamicSmemBytes = 0;
-	cfg.stream = s;
-	cudaLaunchAttribute attr[1];
-	attr[0].id = cudaLaunchAttributeCooperative;
-	attr[0].val.cooperative = 1;
-	cfg.attrs = attr;
-	cfg.numAttrs = 1;
 	ProfScope ps(ctx, "poisson_cg");
-	NLI_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
-	nli_count_launch_internal();
+	launch_cooperative(ctx, kern, grid, kCgBlock, 0, args);
 }
 
 // Solves the system from x0 (the CG of :387-477) and writes u = orig + x on
@@ -1557,7 +2015,13 @@ static int poisson_solve(nli_ctx *ctx, PoissonSystem &P, const int32_t *hole, co
 		nli_count_launch_internal();
 		return C * P.ncta;
 	}
-	const int grid = grid_cg_blocks(ctx, nh);
+	const GridLayout gl = grid_layout(ctx, nh, C, P.pa.W);
+	if (gl.groups > 0) {
+		double *diff_part = ctx->buf<double>("poi.diff", gl.parts + 1);
+		launch_wide_cg(ctx, P, gl, iters, hole, orig, img, diff_part, nullptr);
+		return gl.parts;
+	}
+	const int grid = gl.ctas;
 	double *part = ctx->buf<double>("poi.part", (size_t)grid * 16);
 	double *diff_part = ctx->buf<double>("poi.diff", grid + 1);
 	GridCgBufs g;
@@ -1964,7 +2428,7 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 			T.unkc = ctx->buf<UnkC>(lk_name(it.flag, "unkc"), nh);
 			T.nparts = C * T.ncta;
 		} else {
-			T.nparts = grid_cg_blocks(ctx, it.nh);
+			T.nparts = grid_layout(ctx, it.nh, C, it.W).parts;
 		}
 		T.diff = ctx->buf<double>(lk_name(it.flag, "diff"), (size_t)T.nparts + 1);
 	}
@@ -2103,6 +2567,12 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 		S.unk = T.unk;
 		S.b = T.b;
 		S.x = T.x;
+		const GridLayout gl = grid_layout(ctx, T.nh, C, T.W);
+		if (gl.groups > 0) {
+			launch_wide_cg(ctx, S, gl, T.iters, T.hole, T.orig, T.img, T.diff,
+			               active ? active + T.img_index : nullptr);
+			continue;
+		}
 		GridCgBufs g;
 		g.r = ctx->buf<float>(lk_name(i, "r"), nh * C);
 		g.d = ctx->buf<float>(lk_name(i, "d"), nh * C);
