@@ -11,6 +11,7 @@
 #include <cooperative_groups.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "nli_device.cuh"
 
@@ -258,12 +259,66 @@ struct CoefOut {
 	float *GY;  // W*H*C
 };
 
-__device__ __forceinline__ void gather_coef(const UpdArgs &u, int W, int H, int C, int qx, int qy,
-                                            const uint8_t *__restrict__ ext, const int2 *__restrict__ nnf,
-                                            const float *__restrict__ conf, const float *__restrict__ img,
-                                            const float2 *__restrict__ grad, CoefOut out)
+// The image is read as padded float4 pixels (launch_pad4): a pixel and its
+// forward differences are three of them, differences across the last column
+// and row being 0 (gradient.cpp:37-63).
+struct Pix3 {
+	float4 v, gx, gy;
+};
+
+__device__ __forceinline__ Pix3 load_pix3(const float4 *__restrict__ pad, int W, int H, int x, int y)
 {
-	float S = 0.f, U[4] = {0, 0, 0, 0}, GX[4] = {0, 0, 0, 0}, GY[4] = {0, 0, 0, 0};
+	const float4 *p = pad + (size_t)y * (W + 1) + x;
+	const float4 v = __ldg(p), r = __ldg(p + 1), d = __ldg(p + W + 1);
+	const bool mx = x != W - 1, my = y != H - 1;
+	Pix3 t;
+	t.v = v;
+	t.gx = make_float4(mx ? fs(r.x, v.x) : 0.f, mx ? fs(r.y, v.y) : 0.f, mx ? fs(r.z, v.z) : 0.f, mx ? fs(r.w, v.w) : 0.f);
+	t.gy = make_float4(my ? fs(d.x, v.x) : 0.f, my ? fs(d.y, v.y) : 0.f, my ? fs(d.z, v.z) : 0.f, my ? fs(d.w, v.w) : 0.f);
+	return t;
+}
+
+// a + w v over the first C components
+template <int C>
+__device__ __forceinline__ void add_wc(float4 &a, float w, const float4 &v)
+{
+	a.x = fmaf(w, v.x, a.x);
+	if (C > 1) a.y = fmaf(w, v.y, a.y);
+	if (C > 2) a.z = fmaf(w, v.z, a.z);
+	if (C > 3) a.w = fmaf(w, v.w, a.w);
+}
+
+template <int C>
+__device__ __forceinline__ void store_c(float *p, const float4 &v)
+{
+	p[0] = v.x;
+	if (C > 1) p[1] = v.y;
+	if (C > 2) p[2] = v.z;
+	if (C > 3) p[3] = v.w;
+}
+
+// The sums of one coefficient pixel.
+struct CoefSum {
+	float S;
+	float4 U, GX, GY;
+};
+
+template <int C>
+__device__ __forceinline__ void store_coef(const CoefOut &out, int q, const CoefSum &a)
+{
+	out.S[q] = a.S;
+	store_c<C>(out.U + (size_t)C * q, a.U);
+	store_c<C>(out.GX + (size_t)C * q, a.GX);
+	store_c<C>(out.GY + (size_t)C * q, a.GY);
+}
+
+template <int C>
+__device__ __forceinline__ void gather_coef(const UpdArgs &u, int W, int H, int qx, int qy,
+                                            const uint8_t *__restrict__ ext, const int2 *__restrict__ nnf,
+                                            const float *__restrict__ conf, const float4 *__restrict__ pad, CoefOut out)
+{
+	const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+	CoefSum a = {0.f, zero, zero, zero};
 	const int cy0 = max(qy - u.hy, 0), cy1 = min(qy + u.hy, H - 1);
 	const int cx0 = max(qx - u.hx, 0), cx1 = min(qx + u.hx, W - 1);
 	for (int cy = cy0; cy <= cy1; cy++)
@@ -275,144 +330,162 @@ __device__ __forceinline__ void gather_coef(const UpdArgs &u, int W, int H, int 
 			if (nx < 0 || ny < 0 || nx >= W || ny >= H) continue;
 			float w = u.weights[(qy - cy + u.hy) * u.px + (qx - cx + u.hx)];
 			if (conf) w = conf[c] * w;
-			S += w;
-			const float *iv = img + (size_t)C * (ny * W + nx);
-			const float2 *gv = grad + (size_t)C * (ny * W + nx);
-			for (int k = 0; k < C; k++) {
-				U[k] = fmaf(w, iv[k], U[k]);
-				const float2 g = gv[k];
-				GX[k] = fmaf(w, g.x, GX[k]);
-				GY[k] = fmaf(w, g.y, GY[k]);
-			}
+			const Pix3 t = load_pix3(pad, W, H, nx, ny);
+			a.S += w;
+			add_wc<C>(a.U, w, t.v);
+			add_wc<C>(a.GX, w, t.gx);
+			add_wc<C>(a.GY, w, t.gy);
 		}
-	const int q = qy * W + qx;
-	out.S[q] = S;
-	for (int k = 0; k < C; k++) {
-		out.U[(size_t)C * q + k] = U[k];
-		out.GX[(size_t)C * q + k] = GX[k];
-		out.GY[(size_t)C * q + k] = GY[k];
-	}
+	store_coef<C>(out, qy * W + qx, a);
 }
 
 // Hole pixel k and the neighbours it owns (see k_poisson_coef).
-__device__ __forceinline__ void coef_hole_pixel(const UpdArgs &u, int W, int H, int C, int pix,
+template <int C>
+__device__ __forceinline__ void coef_hole_pixel(const UpdArgs &u, int W, int H, int k, const int32_t *__restrict__ hole,
                                                 const uint8_t *__restrict__ dom, const uint8_t *__restrict__ ext,
                                                 const int2 *__restrict__ nnf, const float *__restrict__ conf,
-                                                const float *__restrict__ img, const float2 *__restrict__ grad,
-                                                CoefOut out)
+                                                const float4 *__restrict__ pad, CoefOut out, int32_t *__restrict__ index)
 {
+	const int pix = hole[k];
 	const int x = pix % W, y = pix / W;
-	gather_coef(u, W, H, C, x, y, ext, nnf, conf, img, grad, out);
+	index[pix] = k;
+	gather_coef<C>(u, W, H, x, y, ext, nnf, conf, pad, out);
 	// left neighbour: owned by this hole pixel when it is not a hole pixel
-	if (x > 0 && !dom[pix - 1]) gather_coef(u, W, H, C, x - 1, y, ext, nnf, conf, img, grad, out);
+	if (x > 0 && !dom[pix - 1]) gather_coef<C>(u, W, H, x - 1, y, ext, nnf, conf, pad, out);
 	// upper neighbour: owned here when it is neither a hole pixel nor the left
 	// neighbour of a hole pixel (then its right neighbour owns it)
 	if (y > 0 && !dom[pix - W] && !(x + 1 < W && dom[pix - W + 1]))
-		gather_coef(u, W, H, C, x, y - 1, ext, nnf, conf, img, grad, out);
+		gather_coef<C>(u, W, H, x, y - 1, ext, nnf, conf, pad, out);
 }
 
+template <int C>
 __global__ void __launch_bounds__(128) k_poisson_coef(UpdArgs u, const int32_t *__restrict__ hole, int nh,
                                                       const uint8_t *__restrict__ dom,
                                                       const uint8_t *__restrict__ ext, const int2 *__restrict__ nnf,
-                                                      const float *__restrict__ conf, const float *__restrict__ img,
-                                                      const float2 *__restrict__ grad, CoefOut out)
+                                                      const float *__restrict__ conf, const float4 *__restrict__ pad,
+                                                      CoefOut out, int32_t *__restrict__ index)
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= nh) return;
-	coef_hole_pixel(u, u.W, u.H, u.C, hole[i], dom, ext, nnf, conf, img, grad, out);
+	coef_hole_pixel<C>(u, u.W, u.H, i, hole, dom, ext, nnf, conf, pad, out, index);
 }
 
-// Item `item` (thread group of 8 lanes, `sub` = lane within the group).
-__device__ __forceinline__ void coef8_item(const UpdArgs &u, int W, int H, int C, int item, int sub,
+// Item `item` of 3 nh (thread group of 8 lanes, `sub` = lane within the
+// group): the coefficients of hole pixel `item` for the first nh, then of the
+// left and upper neighbours of the hole pixels where these are owned.  Also
+// writes the hole pixels' unknown index.
+template <int C>
+__device__ __forceinline__ void coef8_item(const UpdArgs &u, int W, int H, int item, int sub,
                                            const int32_t *__restrict__ hole, int nh, const uint8_t *__restrict__ dom,
                                            const uint8_t *__restrict__ ext, const int2 *__restrict__ nnf,
-                                           const float *__restrict__ conf, const float *__restrict__ img,
-                                           const float2 *__restrict__ grad, CoefOut out)
+                                           const float *__restrict__ conf, const float4 *__restrict__ pad, CoefOut out,
+                                           int32_t *__restrict__ index)
 {
-	bool owned = false;
-	int qx = 0, qy = 0;
-	if (item < 3 * nh) {
-		const int k = item / 3, which = item - 3 * k;
-		const int pix = hole[k];
-		if (!nli_in_bounds(pix, (long long)W * H, kSiteHole)) return;  // the item's 8 lanes leave together
-		const int x = pix % W, y = pix / W;
-		if (which == 0) {
-			owned = true;
-			qx = x;
-			qy = y;
-		} else if (which == 1) {
-			owned = x > 0 && !dom[pix - 1];
-			qx = x - 1;
-			qy = y;
-		} else {
-			owned = y > 0 && !dom[pix - W] && !(x + 1 < W && dom[pix - W + 1]);
-			qx = x;
-			qy = y - 1;
-		}
+	if (item >= 3 * nh) return;
+	const int k = item < nh ? item : (item - nh) >> 1;
+	const int pix = hole[k];
+	if (!nli_in_bounds(pix, (long long)W * H, kSiteHole)) return;  // the item's 8 lanes leave together
+	int qx = pix % W, qy = pix / W;
+	bool owned = true;
+	if (item < nh) {
+		if (sub == 0) index[pix] = k;
+	} else if (((item - nh) & 1) == 0) {
+		owned = qx > 0 && !dom[pix - 1];
+		qx--;
+	} else {
+		owned = qy > 0 && !dom[pix - W] && !(qx + 1 < W && dom[pix - W + 1]);
+		qy--;
 	}
 	// all 8 lanes of an item agree on `owned`; whole groups leave together
 	if (!owned) return;
 	const unsigned gmask = 0xffu << (threadIdx.x & 24);
-	float S = 0.f, U[4] = {0, 0, 0, 0}, GX[4] = {0, 0, 0, 0}, GY[4] = {0, 0, 0, 0};
+	const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+	CoefSum a = {0.f, zero, zero, zero};
 	const int taps = u.px * u.py;
-	for (int t = sub; t < taps; t += 8) {
-		const int ty = t / u.px, tx = t - ty * u.px;
-		// centre c = q - (tap offset), tap offset = (tx - hx, ty - hy)
-		const int cx = qx - (tx - u.hx), cy = qy - (ty - u.hy);
-		if (cx < 0 || cy < 0 || cx >= W || cy >= H) continue;
-		const int c = cy * W + cx;
-		if (!ext[c]) continue;
-		const int2 nb = nnf[c];
-		const int nx = nb.x + qx - cx, ny = nb.y + qy - cy;
-		if (nx < 0 || ny < 0 || nx >= W || ny >= H) continue;
-		if (!nli_in_bounds((long long)ny * W + nx, (long long)W * H, kSiteCoefSource)) continue;
-		float w = u.weights[t];
-		if (conf) w = conf[c] * w;
-		S += w;
-		const float *iv = img + (size_t)C * (ny * W + nx);
-		const float2 *gv = grad + (size_t)C * (ny * W + nx);
-		for (int k = 0; k < C; k++) {
-			U[k] = fmaf(w, iv[k], U[k]);
-			const float2 g = gv[k];
-			GX[k] = fmaf(w, g.x, GX[k]);
-			GY[k] = fmaf(w, g.y, GY[k]);
+	// a lane's taps in groups whose loads are in flight together; a tap
+	// without a centre reads the pixel itself and adds nothing
+	constexpr int kGroup = 4;
+	for (int t0 = sub; t0 < taps; t0 += 8 * kGroup) {
+		int2 nb[kGroup];
+		float w[kGroup];
+		bool ok[kGroup];
+		int dx[kGroup], dy[kGroup];
+#pragma unroll
+		for (int i = 0; i < kGroup; i++) {
+			const int t = t0 + 8 * i;
+			const int ty = t / u.px, tx = t - ty * u.px;
+			// centre c = q - (tap offset), tap offset = (tx - hx, ty - hy)
+			dx[i] = tx - u.hx;
+			dy[i] = ty - u.hy;
+			const int cx = qx - dx[i], cy = qy - dy[i];
+			ok[i] = t < taps && cx >= 0 && cy >= 0 && cx < W && cy < H;
+			const int c = ok[i] ? cy * W + cx : pix;
+			ok[i] = ok[i] && ext[c];
+			nb[i] = nnf[c];
+			w[i] = t < taps ? u.weights[t] : 0.f;
+			if (conf) w[i] = conf[c] * w[i];
+		}
+		Pix3 v[kGroup];
+#pragma unroll
+		for (int i = 0; i < kGroup; i++) {
+			const int nx = nb[i].x + dx[i], ny = nb[i].y + dy[i];
+			ok[i] = ok[i] && nx >= 0 && ny >= 0 && nx < W && ny < H &&
+			        nli_in_bounds((long long)ny * W + nx, (long long)W * H, kSiteCoefSource);
+			v[i] = load_pix3(pad, W, H, ok[i] ? nx : qx, ok[i] ? ny : qy);
+		}
+#pragma unroll
+		for (int i = 0; i < kGroup; i++) {
+			if (!ok[i]) continue;
+			a.S += w[i];
+			add_wc<C>(a.U, w[i], v[i].v);
+			add_wc<C>(a.GX, w[i], v[i].gx);
+			add_wc<C>(a.GY, w[i], v[i].gy);
 		}
 	}
+	auto fold = [gmask](float4 &v, int o) {
+		v.x += __shfl_xor_sync(gmask, v.x, o);
+		if (C > 1) v.y += __shfl_xor_sync(gmask, v.y, o);
+		if (C > 2) v.z += __shfl_xor_sync(gmask, v.z, o);
+		if (C > 3) v.w += __shfl_xor_sync(gmask, v.w, o);
+	};
 #pragma unroll
 	for (int o = 4; o > 0; o >>= 1) {
-		S += __shfl_xor_sync(gmask, S, o);
-#pragma unroll
-		for (int k = 0; k < 4; k++) {
-			if (k >= C) break;
-			U[k] += __shfl_xor_sync(gmask, U[k], o);
-			GX[k] += __shfl_xor_sync(gmask, GX[k], o);
-			GY[k] += __shfl_xor_sync(gmask, GY[k], o);
-		}
+		a.S += __shfl_xor_sync(gmask, a.S, o);
+		fold(a.U, o);
+		fold(a.GX, o);
+		fold(a.GY, o);
 	}
-	if (sub == 0) {
-		const int q = qy * W + qx;
-		out.S[q] = S;
-		for (int k = 0; k < C; k++) {
-			out.U[(size_t)C * q + k] = U[k];
-			out.GX[(size_t)C * q + k] = GX[k];
-			out.GY[(size_t)C * q + k] = GY[k];
-		}
-	}
+	if (sub == 0) store_coef<C>(out, qy * W + qx, a);
 }
 
-// The same gather with 8 lanes per coefficient pixel: item (k, which) is
-// hole pixel k itself (which 0), its left neighbour (1) or its upper
-// neighbour (2) when that pixel is owned as in k_poisson_coef; lane j of
-// the item's 8 takes window taps j, j + 8, ...; the 8 partial sums are
-// added with shuffles.  Same terms as gather_coef, summed in a tree.
+// The same gather with 8 lanes per coefficient pixel: lane j of an item's 8
+// takes window taps j, j + 8, ...; the 8 partial sums are added with
+// shuffles.  Same terms as gather_coef, summed in a tree.  Bound by L1 and the
+// latency of the gathers.  The hole pixels come first, so that whole warps of
+// neighbour items that are not owned (nearly all) leave at once: interleaved
+// with them, two thirds of every warp's lanes were idle, and with ten scalar
+// loads per tap (pixel and gradient image) instead of three float4 a 512 x 512
+// hole of 39 000 pixels took 92.5 us; this takes 38.8 (1024 x 685, 175 000
+// pixels: 366 and 139 us).
+template <int C>
 __global__ void __launch_bounds__(256) k_poisson_coef8(UpdArgs u, const int32_t *__restrict__ hole, int nh,
                                                        const uint8_t *__restrict__ dom,
                                                        const uint8_t *__restrict__ ext, const int2 *__restrict__ nnf,
-                                                       const float *__restrict__ conf, const float *__restrict__ img,
-                                                       const float2 *__restrict__ grad, CoefOut out)
+                                                       const float *__restrict__ conf, const float4 *__restrict__ pad,
+                                                       CoefOut out, int32_t *__restrict__ index)
 {
-	coef8_item(u, u.W, u.H, u.C, (blockIdx.x * blockDim.x + threadIdx.x) >> 3, threadIdx.x & 7, hole, nh, dom, ext,
-	           nnf, conf, img, grad, out);
+	coef8_item<C>(u, u.W, u.H, (blockIdx.x * blockDim.x + threadIdx.x) >> 3, threadIdx.x & 7, hole, nh, dom, ext, nnf,
+	              conf, pad, out, index);
+}
+
+// Calls f with the channel count as a compile-time constant.
+template <class F>
+static void with_channels(int C, F &&f)
+{
+	if (C == 1) f(std::integral_constant<int, 1>());
+	if (C == 2) f(std::integral_constant<int, 2>());
+	if (C == 3) f(std::integral_constant<int, 3>());
+	if (C == 4) f(std::integral_constant<int, 4>());
 }
 
 // Per unknown (hole pixel) data of the symmetric system
@@ -424,10 +497,6 @@ struct Unknown {
 	float S;         // unscaled a1 / a2 at the centre
 	float s_up, s_left, s_down, s_right;  // unscaled link coefficients (0 if no link)
 	int n_up, n_left, n_down, n_right;    // unknown index of the neighbour, -1 if not a hole pixel
-	// the same neighbours as (owning CTA << 20) | index within its range,
-	// for the cluster kernel (-1 if not a hole pixel)
-	int c_up, c_left, c_down, c_right;
-	int links;  // bit 0: down link inside the image, bit 1: right link inside the image
 };
 
 struct PoissonArgs {
@@ -437,14 +506,28 @@ struct PoissonArgs {
 	int limit;
 };
 
+// The cluster CG's record: neighbours as 16-bit codes (owning CTA << 12 | index
+// within its range, kNoNb for none).
+constexpr int kNoNb = 0xFFFF;
+
+struct UnkC {
+	float S, s_up, s_left;
+	uint32_t ud;     // up code << 16 | down code
+	uint32_t lr;     // left code << 16 | right code
+	uint32_t links;  // bit 0: down link inside the image, bit 1: right link inside the image
+};
+
 // Right-hand side b and initial perturbation delta0 = image - orig
-// (patch_non_local_poisson.cpp:62-82), and the per-unknown system data.
+// (patch_non_local_poisson.cpp:62-82), and the per-unknown system data: the
+// cluster CG's record for ranges of `chunk` unknowns, or (chunk 0) the grid
+// CG's.  hole_index holds the unknown index of the hole pixels only.
 __device__ __forceinline__ void poisson_setup_unknown(const PoissonArgs &a, int chunk, int k,
                                                       const int32_t *__restrict__ hole,
+                                                      const uint8_t *__restrict__ dom,
                                                       const int32_t *__restrict__ hole_index, CoefOut co,
                                                       const float *__restrict__ img, const float *__restrict__ orig,
-                                                      Unknown *__restrict__ unk, float *__restrict__ b,
-                                                      float *__restrict__ x0)
+                                                      Unknown *__restrict__ unk, UnkC *__restrict__ unkc,
+                                                      float *__restrict__ b, float *__restrict__ x0)
 {
 	const int W = a.W, H = a.H, C = a.C;
 	const int pix = hole[k];
@@ -455,17 +538,26 @@ __device__ __forceinline__ void poisson_setup_unknown(const PoissonArgs &a, int 
 	n.s_left = (x != 0) ? co.S[pix - 1] : 0.f;
 	n.s_down = (y != H - 1) ? n.S : 0.f;
 	n.s_right = (x != W - 1) ? n.S : 0.f;
-	n.n_up = (y != 0) ? hole_index[pix - W] : -1;
-	n.n_left = (x != 0) ? hole_index[pix - 1] : -1;
-	n.n_down = (y != H - 1) ? hole_index[pix + W] : -1;
-	n.n_right = (x != W - 1) ? hole_index[pix + 1] : -1;
-	auto code = [chunk](int m) { return (m >= 0 && chunk > 0) ? ((m / chunk) << 20) | (m % chunk) : -1; };
-	n.c_up = code(n.n_up);
-	n.c_left = code(n.n_left);
-	n.c_down = code(n.n_down);
-	n.c_right = code(n.n_right);
-	n.links = ((y != H - 1) ? 1 : 0) | ((x != W - 1) ? 2 : 0);
-	unk[k] = n;
+	auto at = [&](bool inside, int p) { return inside && dom[p] ? hole_index[p] : -1; };
+	n.n_up = at(y != 0, pix - W);
+	n.n_left = at(x != 0, pix - 1);
+	n.n_down = at(y != H - 1, pix + W);
+	n.n_right = at(x != W - 1, pix + 1);
+	if (chunk > 0) {
+		auto code = [chunk](int m) -> uint32_t {
+			return (m >= 0) ? (uint32_t)(((m / chunk) << 12) | (m % chunk)) : (uint32_t)kNoNb;
+		};
+		UnkC c;
+		c.S = n.S;
+		c.s_up = n.s_up;
+		c.s_left = n.s_left;
+		c.ud = (code(n.n_up) << 16) | code(n.n_down);
+		c.lr = (code(n.n_left) << 16) | code(n.n_right);
+		c.links = ((y != H - 1) ? 1u : 0u) | ((x != W - 1) ? 2u : 0u);
+		unkc[k] = c;
+	} else {
+		unk[k] = n;
+	}
 	for (int c = 0; c < C; c++) {
 		const float lam = a.lambda[c], oml = 1.0f - lam;
 		const float a1 = lam * n.S;
@@ -494,13 +586,14 @@ __device__ __forceinline__ void poisson_setup_unknown(const PoissonArgs &a, int 
 }
 
 __global__ void k_poisson_setup(PoissonArgs a, int chunk, const int32_t *__restrict__ hole,
-                                const int32_t *__restrict__ hole_index, CoefOut co, const float *__restrict__ img,
-                                const float *__restrict__ orig, Unknown *__restrict__ unk, float *__restrict__ b,
+                                const uint8_t *__restrict__ dom, const int32_t *__restrict__ hole_index, CoefOut co,
+                                const float *__restrict__ img, const float *__restrict__ orig,
+                                Unknown *__restrict__ unk, UnkC *__restrict__ unkc, float *__restrict__ b,
                                 float *__restrict__ x0)
 {
 	const int k = blockIdx.x * blockDim.x + threadIdx.x;
 	if (k >= a.nh) return;
-	poisson_setup_unknown(a, chunk, k, hole, hole_index, co, img, orig, unk, b, x0);
+	poisson_setup_unknown(a, chunk, k, hole, dom, hole_index, co, img, orig, unk, unkc, b, x0);
 }
 
 __device__ __forceinline__ float apply_A(const Unknown &n, float lam, const float *__restrict__ v, float vk)
@@ -760,38 +853,6 @@ constexpr int kClusterBlock = 512;
 constexpr int kClusterMax = 16;
 constexpr int kClusterMaxChunk = 4096;
 constexpr int kClusterPerThread = kClusterMaxChunk / kClusterBlock;  // unknowns per thread
-constexpr int kNoNb = 0xFFFF;
-
-struct UnkC {
-	float S, s_up, s_left;
-	uint32_t ud;     // up code << 16 | down code
-	uint32_t lr;     // left code << 16 | right code
-	uint32_t links;  // bit 0: down link inside the image, bit 1: right link inside the image
-};
-
-__device__ __forceinline__ void poisson_compact_unknown(const Unknown *__restrict__ unk, int k, int chunk,
-                                                        UnkC *__restrict__ out)
-{
-	const Unknown n = unk[k];
-	auto code = [chunk](int m) -> uint32_t {
-		return (m >= 0) ? (uint32_t)(((m / chunk) << 12) | (m % chunk)) : (uint32_t)kNoNb;
-	};
-	UnkC c;
-	c.S = n.S;
-	c.s_up = n.s_up;
-	c.s_left = n.s_left;
-	c.ud = (code(n.n_up) << 16) | code(n.n_down);
-	c.lr = (code(n.n_left) << 16) | code(n.n_right);
-	c.links = (uint32_t)n.links;
-	out[k] = c;
-}
-
-__global__ void k_poisson_compact(const Unknown *__restrict__ unk, int nh, int chunk, UnkC *__restrict__ out)
-{
-	const int k = blockIdx.x * blockDim.x + threadIdx.x;
-	if (k >= nh) return;
-	poisson_compact_unknown(unk, k, chunk, out);
-}
 
 // 1 / the diagonal of an unknown's row, lam S + (1 - lam) (sum of its four
 // link coefficients) (1 where that is not positive): the Jacobi
@@ -1674,17 +1735,6 @@ __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __gr
 	if (threadIdx.x == 0) A.diff[ch * ctas + rank] = dacc;
 }
 
-__global__ void k_hole_index(const int32_t *__restrict__ hole, int nh, int32_t *__restrict__ index)
-{
-	const int k = blockIdx.x * blockDim.x + threadIdx.x;
-	if (k < nh) index[hole[k]] = k;
-}
-
-__global__ void k_fill_int(int32_t *p, int n, int v)
-{
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
-}
-
 NLI_CHECK_READER(check_word_update)
 
 static double read_total(nli_ctx *ctx, double *partials, int n, int *cg_iters_dev, int C, int nh = 0)
@@ -1782,38 +1832,42 @@ static void cg_layout(nli_ctx *ctx, int nh, int *ncta, int *chunk)
 struct PoissonSystem {
 	PoissonArgs pa;
 	CoefOut co;
-	Unknown *unk;
+	const float4 *pad;  // the image as padded pixels
+	Unknown *unk = nullptr;  // grid layouts
+	UnkC *unkc = nullptr;    // cluster layouts
 	float *b, *x;
 	int chunk = 0, ncta = 0;
 };
 
 static PoissonSystem poisson_system(nli_ctx *ctx, const UpdArgs &u, const nli_update_params &up, const float *image,
                                     const float *orig, const uint8_t *dom, const uint8_t *ext, const int2 *nnf,
-                                    const float *conf, const int32_t *hole, const int32_t *hole_index, int nh)
+                                    const float *conf, const int32_t *hole, int nh)
 {
 	cudaStream_t s = ctx->stream;
 	const int W = u.W, H = u.H, C = u.C;
 	const size_t n = (size_t)W * H;
 	PoissonSystem P;
-	float *grad = ctx->buf<float>("poi.grad", n * 2 * C);
-	launch_gradient(s, image, W, H, C, grad);
+	float4 *pad = ctx->buf<float4>("poi.pad", (size_t)(W + 1) * (H + 1));
+	launch_pad4(s, image, W, H, C, pad);
+	P.pad = pad;
+	int32_t *index = ctx->buf<int32_t>("upd.hole_index", n);
 	P.co.S = ctx->buf<float>("poi.S", n);
 	P.co.U = ctx->buf<float>("poi.U", n * C);
 	P.co.GX = ctx->buf<float>("poi.GX", n * C);
 	P.co.GY = ctx->buf<float>("poi.GY", n * C);
-	{
+	with_channels(C, [&](auto c) {
+		constexpr int CC = decltype(c)::value;
 		ProfScope ps(ctx, "poisson_coef");
 		if (u.px % 2 == 1 && u.py % 2 == 1) {
 			const long long threads = 3LL * nh * 8;
-			k_poisson_coef8<<<(int)((threads + 255) / 256), 256, 0, s>>>(
-			    u, hole, nh, dom, ext, nnf, conf, image, reinterpret_cast<const float2 *>(grad), P.co);
+			k_poisson_coef8<CC><<<(int)((threads + 255) / 256), 256, 0, s>>>(u, hole, nh, dom, ext, nnf, conf, pad, P.co,
+			                                                                 index);
 		} else {
 			// even patch sides: the window of gather_coef is one wider than the patch
-			k_poisson_coef<<<(nh + 127) / 128, 128, 0, s>>>(u, hole, nh, dom, ext, nnf, conf, image,
-			                                                 reinterpret_cast<const float2 *>(grad), P.co);
+			k_poisson_coef<CC><<<(nh + 127) / 128, 128, 0, s>>>(u, hole, nh, dom, ext, nnf, conf, pad, P.co, index);
 		}
 		NLI_CHECK_LAUNCH();
-	}
+	});
 	PoissonArgs &pa = P.pa;
 	pa.W = W;
 	pa.H = H;
@@ -1823,15 +1877,18 @@ static PoissonSystem poisson_system(nli_ctx *ctx, const UpdArgs &u, const nli_up
 	if (up.method == NLI_UPDATE_DEPTH) pa.lambda[3] = up.lambda_d;
 	pa.tol = up.cg_tol;
 	pa.limit = up.cg_iters;
-	P.unk = ctx->buf<Unknown>("poi.unk", nh);
 	P.b = ctx->buf<float>("poi.b", (size_t)nh * C);
 	P.x = ctx->buf<float>("poi.x", (size_t)nh * C);
 
 	cg_layout(ctx, nh, &P.ncta, &P.chunk);
+	if (P.ncta > 0)
+		P.unkc = ctx->buf<UnkC>("poi.unkc", nh);
+	else
+		P.unk = ctx->buf<Unknown>("poi.unk", nh);
 	{
 		ProfScope ps(ctx, "poisson_setup");
-		k_poisson_setup<<<(nh + 255) / 256, 256, 0, s>>>(pa, P.chunk, hole, hole_index, P.co, image, orig, P.unk,
-		                                                  P.b, P.x);
+		k_poisson_setup<<<(nh + 255) / 256, 256, 0, s>>>(pa, P.chunk, hole, dom, index, P.co, image, orig, P.unk,
+		                                                  P.unkc, P.b, P.x);
 		NLI_CHECK_LAUNCH();
 	}
 	return P;
@@ -1985,14 +2042,11 @@ static int poisson_solve(nli_ctx *ctx, PoissonSystem &P, const int32_t *hole, co
 		const bool pre = ctx->tune_cg_precond != 0;
 		const size_t smem = cg_smem_bytes(P.chunk);
 		const CgKernel kern = cg_kernel(pre, P.ncta == 1, cg_per_thread(P.chunk));
-		UnkC *unkc = ctx->buf<UnkC>("poi.unkc", nh);
-		k_poisson_compact<<<(nh + 255) / 256, 256, 0, s>>>(P.unk, nh, P.chunk, unkc);
-		NLI_CHECK_LAUNCH();
 		double *diff_part = ctx->buf<double>("poi.diff", (size_t)C * P.ncta + 1);
 		if (P.ncta == 1) {
 			// one CTA per channel: no cluster
 			ProfScope ps(ctx, "poisson_cg");
-			kern<<<C, kClusterBlock, smem, s>>>(P.pa, P.chunk, unkc, P.b, P.x, iters, hole, orig, img, diff_part,
+			kern<<<C, kClusterBlock, smem, s>>>(P.pa, P.chunk, P.unkc, P.b, P.x, iters, hole, orig, img, diff_part,
 			                                    &ctx->status->timeout);
 			NLI_CHECK_LAUNCH();
 			return C;
@@ -2010,7 +2064,7 @@ static int poisson_solve(nli_ctx *ctx, PoissonSystem &P, const int32_t *hole, co
 		cfg.attrs = attr;
 		cfg.numAttrs = 1;
 		ProfScope ps(ctx, "poisson_cg");
-		NLI_CUDA(cudaLaunchKernelEx(&cfg, kern, P.pa, P.chunk, (const UnkC *)unkc, (const float *)P.b,
+		NLI_CUDA(cudaLaunchKernelEx(&cfg, kern, P.pa, P.chunk, (const UnkC *)P.unkc, (const float *)P.b,
 		                            (const float *)P.x, iters, hole, orig, img, diff_part, &ctx->status->timeout));
 		nli_count_launch_internal();
 		return C * P.ncta;
@@ -2036,9 +2090,9 @@ static int poisson_solve(nli_ctx *ctx, PoissonSystem &P, const int32_t *hole, co
 
 static void poisson_run(nli_ctx *ctx, const UpdArgs &u, const nli_update_params &up, float *image, const float *orig,
                         const uint8_t *dom, const uint8_t *ext, const int2 *nnf, const float *conf,
-                        const int32_t *hole, const int32_t *hole_index, int nh, int *n_partials)
+                        const int32_t *hole, int nh, int *n_partials)
 {
-	PoissonSystem P = poisson_system(ctx, u, up, image, orig, dom, ext, nnf, conf, hole, hole_index, nh);
+	PoissonSystem P = poisson_system(ctx, u, up, image, orig, dom, ext, nnf, conf, hole, nh);
 	*n_partials = poisson_solve(ctx, P, hole, orig, image);
 }
 
@@ -2052,7 +2106,6 @@ double update_run(nli_ctx *ctx, const nli_update_params &up, float *image, const
 	fill_upd_args(u, up, W, H, C);
 	cudaStream_t s = ctx->stream;
 	const int2 *nnf = reinterpret_cast<const int2 *>(nnf_i);
-	const int32_t *hole_index = nullptr;
 	if (!hole) {
 		int32_t *l = ctx->buf<int32_t>("upd.hole", (size_t)W * H);
 		nh = compact_mask(ctx, dom, W, H, l, "upd");
@@ -2060,14 +2113,8 @@ double update_run(nli_ctx *ctx, const nli_update_params &up, float *image, const
 	}
 	if (nh <= 0) return 0.0;
 	if (up.method == NLI_UPDATE_POISSON || up.method == NLI_UPDATE_DEPTH) {
-		int32_t *idx = ctx->buf<int32_t>("upd.hole_index", (size_t)W * H);
-		k_fill_int<<<(W * H + 255) / 256, 256, 0, s>>>(idx, W * H, -1);
-		NLI_CHECK_LAUNCH();
-		k_hole_index<<<(nh + 255) / 256, 256, 0, s>>>(hole, nh, idx);
-		NLI_CHECK_LAUNCH();
-		hole_index = idx;
 		int np = 0;
-		poisson_run(ctx, u, up, image, orig, dom, ext, nnf, conf, hole, hole_index, nh, &np);
+		poisson_run(ctx, u, up, image, orig, dom, ext, nnf, conf, hole, nh, &np);
 		double *diff_part = ctx->buf<double>("poi.diff", np + 1);
 		if (!read_back) {
 			launch_sum_partials(s, diff_part, np, diff_part + np);
@@ -2126,7 +2173,7 @@ struct BTask {
 	float *newval;      // NL-means / NL-medians: new values of the hole
 	double *partials;   // NL-means / NL-medians: per-block sums
 	int32_t *hidx;      // NL-Poisson: unknown index per pixel
-	float *grad;
+	float4 *pad;        // NL-Poisson: the image as padded pixels
 	CoefOut co;
 	Unknown *unk;
 	UnkC *unkc;
@@ -2231,50 +2278,33 @@ __global__ void __launch_bounds__(1024) k_total_batch(const __grid_constant__ BA
 	if (threadIdx.x == 0) *T.total = v;
 }
 
-// Unknown index per pixel: -1, then k at hole pixel k.
-__global__ void k_hidx_fill_batch(const __grid_constant__ BArgs B)
+__global__ void k_upd_pad_batch(const __grid_constant__ BArgs B, int C)
 {
 	const int t = blockIdx.y;
 	if (!btask_on(B, t)) return;
 	const BTask &T = B.t[t];
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < T.W * T.H; i += gridDim.x * blockDim.x) T.hidx[i] = -1;
+	pad4_span(T.img, T.W, T.H, C, T.pad, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
-__global__ void k_hidx_set_batch(const __grid_constant__ BArgs B)
-{
-	const int t = blockIdx.y;
-	if (!btask_on(B, t)) return;
-	const BTask &T = B.t[t];
-	for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < T.nh; k += gridDim.x * blockDim.x) T.hidx[T.hole[k]] = k;
-}
-
-__global__ void k_gradient_batch(const __grid_constant__ BArgs B, int C)
-{
-	const int t = blockIdx.y;
-	if (!btask_on(B, t)) return;
-	const BTask &T = B.t[t];
-	gradient_span(T.img, T.W, T.H, C, T.grad, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-}
-
-__global__ void __launch_bounds__(256) k_coef8_batch(UpdArgs u, const __grid_constant__ BArgs B, int C)
+template <int C>
+__global__ void __launch_bounds__(256) k_coef8_batch(UpdArgs u, const __grid_constant__ BArgs B)
 {
 	const int t = task_of_block(B, blockIdx.x);
 	if (!btask_on(B, t)) return;
 	const BTask &T = B.t[t];
 	const int item = (((int)blockIdx.x - B.blk[t]) * 256 + (int)threadIdx.x) >> 3;
-	coef8_item(u, T.W, T.H, C, item, threadIdx.x & 7, T.hole, T.nh, T.dom, T.ext, T.nnf, T.conf, T.img,
-	           reinterpret_cast<const float2 *>(T.grad), T.co);
+	coef8_item<C>(u, T.W, T.H, item, threadIdx.x & 7, T.hole, T.nh, T.dom, T.ext, T.nnf, T.conf, T.pad, T.co, T.hidx);
 }
 
-__global__ void __launch_bounds__(128) k_coef_batch(UpdArgs u, const __grid_constant__ BArgs B, int C)
+template <int C>
+__global__ void __launch_bounds__(128) k_coef_batch(UpdArgs u, const __grid_constant__ BArgs B)
 {
 	const int t = task_of_block(B, blockIdx.x);
 	if (!btask_on(B, t)) return;
 	const BTask &T = B.t[t];
 	const int i = ((int)blockIdx.x - B.blk[t]) * 128 + (int)threadIdx.x;
 	if (i >= T.nh) return;
-	coef_hole_pixel(u, T.W, T.H, C, T.hole[i], T.dom, T.ext, T.nnf, T.conf, T.img,
-	                reinterpret_cast<const float2 *>(T.grad), T.co);
+	coef_hole_pixel<C>(u, T.W, T.H, i, T.hole, T.dom, T.ext, T.nnf, T.conf, T.pad, T.co, T.hidx);
 }
 
 __global__ void k_setup_batch(const __grid_constant__ BArgs B)
@@ -2284,17 +2314,7 @@ __global__ void k_setup_batch(const __grid_constant__ BArgs B)
 	const BTask &T = B.t[t];
 	const int k = ((int)blockIdx.x - B.blk[t]) * 256 + (int)threadIdx.x;
 	if (k >= T.nh) return;
-	poisson_setup_unknown(T.pa, T.chunk, k, T.hole, T.hidx, T.co, T.img, T.orig, T.unk, T.b, T.x);
-}
-
-__global__ void k_compact_batch(const __grid_constant__ BArgs B)
-{
-	const int t = blockIdx.y;
-	if (!btask_on(B, t)) return;
-	const BTask &T = B.t[t];
-	if (T.ncta == 0) return;
-	for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < T.nh; k += gridDim.x * blockDim.x)
-		poisson_compact_unknown(T.unk, k, T.chunk, T.unkc);
+	poisson_setup_unknown(T.pa, T.chunk, k, T.hole, T.dom, T.hidx, T.co, T.img, T.orig, T.unk, T.unkc, T.b, T.x);
 }
 
 // CG systems of one layout class (the same CTAs per system): system g of
@@ -2371,7 +2391,7 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 	std::memset(&D, 0, sizeof(D));
 	std::memset(&P, 0, sizeof(P));
 	M.active = D.active = P.active = active;
-	long long maxnh = 0, maxpix = 0;
+	long long maxnh = 0, maxpad = 0;
 	for (int i = 0; i < n; i++) {
 		const UpdBatchItem &it = items[i];
 		const nli_update_params &up = ups[i];
@@ -2393,7 +2413,6 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 		T.total = it.total;
 		T.iters = it.cg_iters;
 		maxnh = std::max<long long>(maxnh, it.nh);
-		maxpix = std::max<long long>(maxpix, (long long)it.W * it.H);
 		const size_t np = (size_t)it.W * it.H;
 		const size_t nh = (size_t)std::max(it.nh, 1);
 		if (&B != &P) {
@@ -2413,12 +2432,12 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 		pa.tol = up.cg_tol;
 		pa.limit = up.cg_iters;
 		T.hidx = ctx->buf<int32_t>(lk_name(it.flag, "hidx"), np);
-		T.grad = ctx->buf<float>(lk_name(it.flag, "grad"), np * 2 * C);
+		T.pad = ctx->buf<float4>(lk_name(it.flag, "pad"), (size_t)(it.W + 1) * (it.H + 1));
+		maxpad = std::max(maxpad, (long long)(it.W + 1) * (it.H + 1));
 		T.co.S = ctx->buf<float>(lk_name(it.flag, "S"), np);
 		T.co.U = ctx->buf<float>(lk_name(it.flag, "U"), np * C);
 		T.co.GX = ctx->buf<float>(lk_name(it.flag, "GX"), np * C);
 		T.co.GY = ctx->buf<float>(lk_name(it.flag, "GY"), np * C);
-		T.unk = ctx->buf<Unknown>(lk_name(it.flag, "unk"), nh);
 		T.b = ctx->buf<float>(lk_name(it.flag, "b"), nh * C);
 		T.x = ctx->buf<float>(lk_name(it.flag, "x"), nh * C);
 		cg_layout(ctx, it.nh, &T.ncta, &T.chunk);
@@ -2428,6 +2447,7 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 			T.unkc = ctx->buf<UnkC>(lk_name(it.flag, "unkc"), nh);
 			T.nparts = C * T.ncta;
 		} else {
+			T.unk = ctx->buf<Unknown>(lk_name(it.flag, "unk"), nh);
 			T.nparts = grid_layout(ctx, it.nh, C, it.W).parts;
 		}
 		T.diff = ctx->buf<double>(lk_name(it.flag, "diff"), (size_t)T.nparts + 1);
@@ -2461,23 +2481,20 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 	}
 	if (P.n == 0) return;
 	// ---- NL-Poisson / NL-depth: system set-up for every image
-	k_hidx_fill_batch<<<per_image_grid(maxpix, P.n), blk, 0, s>>>(P);
+	k_upd_pad_batch<<<per_image_grid(maxpad, P.n), blk, 0, s>>>(P, C);
 	NLI_CHECK_LAUNCH();
-	k_hidx_set_batch<<<per_image_grid(maxnh, P.n), blk, 0, s>>>(P);
-	NLI_CHECK_LAUNCH();
-	k_gradient_batch<<<per_image_grid(maxpix * C, P.n), blk, 0, s>>>(P, C);
-	NLI_CHECK_LAUNCH();
-	{
+	with_channels(C, [&](auto c) {
+		constexpr int CC = decltype(c)::value;
 		ProfScope ps(ctx, "poisson_coef");
 		if (u.px % 2 == 1 && u.py % 2 == 1) {
 			for (int t = 0; t < P.n; t++) P.blk[t + 1] = P.blk[t] + div_up(3LL * P.t[t].nh * 8, 256);
-			if (P.blk[P.n] > 0) k_coef8_batch<<<P.blk[P.n], 256, 0, s>>>(u, P, C);
+			if (P.blk[P.n] > 0) k_coef8_batch<CC><<<P.blk[P.n], 256, 0, s>>>(u, P);
 		} else {
 			for (int t = 0; t < P.n; t++) P.blk[t + 1] = P.blk[t] + div_up(P.t[t].nh, 128);
-			if (P.blk[P.n] > 0) k_coef_batch<<<P.blk[P.n], 128, 0, s>>>(u, P, C);
+			if (P.blk[P.n] > 0) k_coef_batch<CC><<<P.blk[P.n], 128, 0, s>>>(u, P);
 		}
 		if (P.blk[P.n] > 0) NLI_CHECK_LAUNCH();
-	}
+	});
 	{
 		ProfScope ps(ctx, "poisson_setup");
 		for (int t = 0; t < P.n; t++) P.blk[t + 1] = P.blk[t] + div_up(P.t[t].nh, 256);
@@ -2486,8 +2503,6 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 			NLI_CHECK_LAUNCH();
 		}
 	}
-	k_compact_batch<<<per_image_grid(maxnh, P.n), blk, 0, s>>>(P);
-	NLI_CHECK_LAUNCH();
 	// ---- the solves, one launch per CTA layout
 	const bool pre = ctx->tune_cg_precond != 0;
 	{
@@ -2899,14 +2914,9 @@ void update_backward_run(nli_ctx *ctx, const nli_update_params &up, const float 
 		NLI_CHECK_LAUNCH();
 		*grad_sigma = sum_on_host(ctx, part, grid, 1, 0);
 	} else if (nh > 0) {
-		int32_t *idx = ctx->buf<int32_t>("upd.hole_index", n);
-		k_fill_int<<<(int)((n + 255) / 256), 256, 0, s>>>(idx, (int)n, -1);
-		NLI_CHECK_LAUNCH();
-		k_hole_index<<<(nh + 255) / 256, 256, 0, s>>>(hole, nh, idx);
-		NLI_CHECK_LAUNCH();
 		// system of the forward step with orig = image; its right-hand side
 		// is replaced by g on the hole, and z = A^-1 g is written as an image
-		PoissonSystem P = poisson_system(ctx, u, up, image, image, dom, ext, nnf, conf, hole, idx, nh);
+		PoissonSystem P = poisson_system(ctx, u, up, image, image, dom, ext, nnf, conf, hole, nh);
 		k_hole_to_planar<<<(nh * C + 255) / 256, 256, 0, s>>>(grad_out, hole, nh, C, P.b);
 		NLI_CHECK_LAUNCH();
 		NLI_CUDA(cudaMemsetAsync(P.x, 0, sizeof(float) * nh * C, s));
@@ -2928,9 +2938,11 @@ void update_backward_run(nli_ctx *ctx, const nli_update_params &up, const float 
 		                                        up.method == NLI_UPDATE_DEPTH ? 1 : 0);
 		NLI_CHECK_LAUNCH();
 		const int grid2 = (int)((n + 127) / 128);
+		float *grad = ctx->buf<float>("adj.grad", n * 2 * C);
+		launch_gradient(s, image, W, H, C, grad);
 		double *sig_part = ctx->buf<double>("adj.sig", grid2);
 		k_poisson_adj_scatter<<<grid2, 128, 0, s>>>(u, a, ad, ext, nnf, conf, image,
-		                                            reinterpret_cast<const float2 *>(ctx->buf<float>("poi.grad", n * 2 * C)),
+		                                            reinterpret_cast<const float2 *>(grad),
 		                                            gacc, sig_part);
 		NLI_CHECK_LAUNCH();
 		*grad_lambda = sum_on_host(ctx, lam_part, grid, 2, 0);
