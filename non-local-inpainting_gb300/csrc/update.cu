@@ -2663,16 +2663,12 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 // weights w_k = e_k / sum_j e_j, e_k = exp(-r_k^2 / (2 sigma^2))
 // (gaussian_weights.cpp:19-79): dw_k/dsigma = w_k (rho_k - m), rho_k =
 // r_k^2 / sigma^3, m = sum_j w_j rho_j.
+// Both factors per tap, formed once on the host: rho_k (NL-means), and
+// rho_k - m as a pair of floats (NL-Poisson).
 struct AdjArgs {
-	double sigma3;  // sigma^3
-	double m;       // sum_j w_j rho_j of the weight table
+	double rho[kMaxTaps];
+	float2 rho_m[kMaxTaps];
 };
-
-__device__ __forceinline__ double tap_rho(const UpdArgs &u, const AdjArgs &a, int k)
-{
-	const int kx = k % u.px - u.hx, ky = k / u.px - u.hy;
-	return (double)(kx * kx + ky * ky) / a.sigma3;
-}
 
 // Identity part: out = u outside the domain (and on domain pixels without
 // any valid candidate, handled by the means kernel).
@@ -2732,7 +2728,7 @@ __global__ void __launch_bounds__(256) k_means_backward(UpdArgs u, AdjArgs a, co
 					const int k = (jj - y_a) * u.px + (ii - x_a);
 					float w = u.weights[k];
 					if (conf && dom[jj * W + ii]) w = fm(w, conf[jj * W + ii]);
-					const double wd = (double)w * inv, rho = tap_rho(u, a, k);
+					const double wd = (double)w * inv, rho = a.rho[k];
 					const size_t s = (size_t)C * (q.y * W + q.x);
 					for (int c = 0; c < C; c++) {
 						atomicAdd(gacc + s + c, (double)gp[c] * wd);
@@ -2759,7 +2755,6 @@ struct AdjCoef {
 	float *dU;   // W*H*C
 	float *dGX;  // W*H*C
 	float *dGY;  // W*H*C
-	uint8_t *active;
 };
 
 __global__ void k_poisson_adj_coef(PoissonArgs pa, CoefOut co, AdjCoef ad, const uint8_t *__restrict__ dom,
@@ -2779,7 +2774,6 @@ __global__ void k_poisson_adj_coef(PoissonArgs pa, CoefOut co, AdjCoef ad, const
 		const bool hl = (x != 0) && dom[q - 1];
 		const bool hu = (y != 0) && dom[q - W];
 		const bool act = hq || hr || hd;
-		ad.active[q] = act ? 1 : 0;
 		float dS = 0.f;
 		for (int c = 0; c < C; c++) {
 			const float lam = pa.lambda[c], oml = 1.0f - lam;
@@ -2843,33 +2837,101 @@ __global__ void k_poisson_adj_coef(PoissonArgs pa, CoefOut co, AdjCoef ad, const
 	}
 }
 
+// A sum of products kept as a pair of floats.
+__device__ __forceinline__ void pair_add(float2 &s, float2 v)
+{
+	const float t = s.x + v.x, b = t - s.x;
+	s.y += ((s.x - (t - b)) + (v.x - b)) + v.y;
+	s.x = t;
+}
+
+__device__ __forceinline__ float2 pair_mul(float2 a, float2 b)
+{
+	const float p = fm(a.x, b.x);
+	return make_float2(p, fmaf(a.x, b.x, -p) + fmaf(a.x, b.y, fm(a.y, b.x)));
+}
+
 // Scatter of the coefficient adjoints through the gathers of
-// k_poisson_coef: for every active q and every extended-domain centre c of
-// its window with n = nnf(c) + q - c in the image,
+// k_poisson_coef: for every coefficient pixel q and every extended-domain
+// centre c of its window with n = nnf(c) + q - c in the image,
 //   du(n) += w dU(q), gx / gy of n (forward differences of u) take w dGX(q),
 //   w dGY(q), and dsigma += dw/dsigma (dS(q) + sum_c dU u(n) + dGX gx(n) +
 //   dGY gy(n)).
-__global__ void __launch_bounds__(128) k_poisson_adj_scatter(UpdArgs u, AdjArgs a, AdjCoef ad,
+// Where the field is coherent, consecutive taps of a window name the same n:
+// their weights (and weights times rho - m) are first added up, as pairs of
+// floats (exact to 2^-43), and n is read and its up to nine double atomics
+// issued once per run of taps.  One thread per coefficient pixel, the hole
+// pixels first (as k_poisson_coef8's items).  With a thread per image pixel, every
+// tap on its own and rho_k by a double division a 512 x 512 step took 1248 us
+// (29 million atomics); this takes 536 us.
+template <int C>
+__global__ void __launch_bounds__(128) k_poisson_adj_scatter(UpdArgs u, const __grid_constant__ AdjArgs a, AdjCoef ad,
+                                                             const int32_t *__restrict__ hole, int nh,
+                                                             const uint8_t *__restrict__ dom,
                                                              const uint8_t *__restrict__ ext,
                                                              const int2 *__restrict__ nnf,
                                                              const float *__restrict__ conf,
-                                                             const float *__restrict__ img,
-                                                             const float2 *__restrict__ grad,
+                                                             const float4 *__restrict__ pad,
                                                              double *__restrict__ gacc, double *__restrict__ partials)
 {
 	__shared__ double red[4];
-	const int W = u.W, H = u.H, C = u.C;
-	const int q = blockIdx.x * blockDim.x + threadIdx.x;
+	const int W = u.W, H = u.H;
+	const int item = blockIdx.x * blockDim.x + threadIdx.x;
 	double dsig = 0.0;
-	if (q < W * H && ad.active[q]) {
-		const int qx = q % W, qy = q / W;
-		float dU[4], dGX[4], dGY[4];
+	int qx = 0, qy = 0;
+	bool owned = item < 3 * nh;
+	if (owned) {
+		const int pix = hole[item < nh ? item : (item - nh) >> 1];
+		qx = pix % W, qy = pix / W;
+		if (item >= nh) {
+			if (((item - nh) & 1) == 0) {
+				owned = qx > 0 && !dom[pix - 1];
+				qx--;
+			} else {
+				owned = qy > 0 && !dom[pix - W] && !(qx + 1 < W && dom[pix - W + 1]);
+				qy--;
+			}
+		}
+	}
+	if (owned) {
+		const int q = qy * W + qx;
+		float dU[C], dGX[C], dGY[C];
+#pragma unroll
 		for (int c = 0; c < C; c++) {
 			dU[c] = ad.dU[(size_t)C * q + c];
 			dGX[c] = ad.dGX[(size_t)C * q + c];
 			dGY[c] = ad.dGY[(size_t)C * q + c];
 		}
-		const double dS = ad.dS[q];
+		const float dS = ad.dS[q];
+		int run = -1;                   // the run's source pixel
+		float2 wsum = make_float2(0.f, 0.f), dsum = wsum;  // of w and of dw/dsigma
+		auto flush = [&]() {
+			const int nx = run % W, ny = run / W;
+			const Pix3 t3 = load_pix3(pad, W, H, nx, ny);
+			const float v[4] = {t3.v.x, t3.v.y, t3.v.z, t3.v.w}, gx[4] = {t3.gx.x, t3.gx.y, t3.gx.z, t3.gx.w};
+			const float gy[4] = {t3.gy.x, t3.gy.y, t3.gy.z, t3.gy.w};
+			const double w = (double)wsum.x + (double)wsum.y;
+			double t = (double)dS;
+#pragma unroll
+			for (int c = 0; c < C; c++) {
+				const size_t o = (size_t)C * run + c;
+				t += (double)dU[c] * v[c] + (double)dGX[c] * gx[c] + (double)dGY[c] * gy[c];
+				double own = w * dU[c];
+				if (nx != W - 1) {
+					const double g = w * dGX[c];
+					atomicAdd(gacc + o + C, g);
+					own -= g;
+				}
+				if (ny != H - 1) {
+					const double g = w * dGY[c];
+					atomicAdd(gacc + o + (size_t)C * W, g);
+					own -= g;
+				}
+				atomicAdd(gacc + o, own);
+			}
+			dsig += ((double)dsum.x + (double)dsum.y) * t;
+			wsum = dsum = make_float2(0.f, 0.f);
+		};
 		const int cy0 = max(qy - u.hy, 0), cy1 = min(qy + u.hy, H - 1);
 		const int cx0 = max(qx - u.hx, 0), cx1 = min(qx + u.hx, W - 1);
 		for (int cy = cy0; cy <= cy1; cy++)
@@ -2880,28 +2942,18 @@ __global__ void __launch_bounds__(128) k_poisson_adj_scatter(UpdArgs u, AdjArgs 
 				const int nx = nb.x + qx - cx, ny = nb.y + qy - cy;
 				if (nx < 0 || ny < 0 || nx >= W || ny >= H) continue;
 				const int k = (qy - cy + u.hy) * u.px + (qx - cx + u.hx);
-				const double cf = conf ? (double)conf[c0] : 1.0;
-				const double w = cf * (double)u.weights[k];
-				const double dw = w * (tap_rho(u, a, k) - a.m);
 				const int n = ny * W + nx;
-				double t = dS;
-				for (int c = 0; c < C; c++) {
-					const size_t o = (size_t)C * n + c;
-					const float2 gv = grad[o];
-					t += (double)dU[c] * img[o] + (double)dGX[c] * gv.x + (double)dGY[c] * gv.y;
-					double own = w * dU[c];
-					if (nx != W - 1) {
-						atomicAdd(gacc + o + C, w * dGX[c]);
-						own -= w * dGX[c];
-					}
-					if (ny != H - 1) {
-						atomicAdd(gacc + o + (size_t)C * W, w * dGY[c]);
-						own -= w * dGY[c];
-					}
-					atomicAdd(gacc + o, own);
+				if (n != run) {
+					if (run >= 0) flush();
+					run = n;
 				}
-				dsig += dw * t;
+				const float cf = conf ? conf[c0] : 1.0f, wk = u.weights[k];
+				const float p = fm(cf, wk);
+				const float2 w = make_float2(p, fmaf(cf, wk, -p));
+				pair_add(wsum, w);
+				pair_add(dsum, pair_mul(w, a.rho_m[k]));
 			}
+		if (run >= 0) flush();
 	}
 	dsig = block_sum<128>(dsig, red);
 	if (threadIdx.x == 0) partials[blockIdx.x] = dsig;
@@ -2943,11 +2995,18 @@ void update_backward_run(nli_ctx *ctx, const nli_update_params &up, const float 
 	UpdArgs u;
 	fill_upd_args(u, up, W, H, C);
 	AdjArgs a;
-	a.sigma3 = (double)up.sigma * up.sigma * up.sigma;
-	a.m = 0.0;
-	for (int k = 0; k < u.px * u.py; k++) {
+	std::memset(&a, 0, sizeof(a));
+	const double sigma3 = (double)up.sigma * up.sigma * up.sigma;
+	double m = 0.0;
+	for (int k = 0; k < kMaxTaps; k++) {
 		const int kx = k % u.px - u.hx, ky = k / u.px - u.hy;
-		a.m += (double)u.weights[k] * (double)(kx * kx + ky * ky) / a.sigma3;
+		a.rho[k] = (double)(kx * kx + ky * ky) / sigma3;
+		if (k < u.px * u.py) m += (double)u.weights[k] * a.rho[k];
+	}
+	for (int k = 0; k < kMaxTaps; k++) {
+		const double d = a.rho[k] - m;
+		a.rho_m[k].x = (float)d;
+		a.rho_m[k].y = (float)(d - (double)a.rho_m[k].x);
 	}
 	cudaStream_t s = ctx->stream;
 	const size_t n = (size_t)W * H;
@@ -2984,20 +3043,18 @@ void update_backward_run(nli_ctx *ctx, const nli_update_params &up, const float 
 		ad.dU = ctx->buf<float>("adj.dU", n * C);
 		ad.dGX = ctx->buf<float>("adj.dGX", n * C);
 		ad.dGY = ctx->buf<float>("adj.dGY", n * C);
-		ad.active = ctx->buf<uint8_t>("adj.active", n);
 		const int grid = (int)((n + 255) / 256);
 		double *lam_part = ctx->buf<double>("adj.lam", 2 * (size_t)grid);
 		k_poisson_adj_coef<<<grid, 256, 0, s>>>(P.pa, P.co, ad, dom, out, zimg, gacc, lam_part,
 		                                        up.method == NLI_UPDATE_DEPTH ? 1 : 0);
 		NLI_CHECK_LAUNCH();
-		const int grid2 = (int)((n + 127) / 128);
-		float *grad = ctx->buf<float>("adj.grad", n * 2 * C);
-		launch_gradient(s, image, W, H, C, grad);
+		const int grid2 = (3 * nh + 127) / 128;
 		double *sig_part = ctx->buf<double>("adj.sig", grid2);
-		k_poisson_adj_scatter<<<grid2, 128, 0, s>>>(u, a, ad, ext, nnf, conf, image,
-		                                            reinterpret_cast<const float2 *>(grad),
-		                                            gacc, sig_part);
-		NLI_CHECK_LAUNCH();
+		with_channels(C, [&](auto c) {
+			k_poisson_adj_scatter<decltype(c)::value><<<grid2, 128, 0, s>>>(u, a, ad, hole, nh, dom, ext, nnf, conf, P.pad,
+			                                                                 gacc, sig_part);
+			NLI_CHECK_LAUNCH();
+		});
 		*grad_lambda = sum_on_host(ctx, lam_part, grid, 2, 0);
 		*grad_lambda_d = sum_on_host(ctx, lam_part, grid, 2, 1);
 		*grad_sigma = sum_on_host(ctx, sig_part, grid2, 1, 0);
