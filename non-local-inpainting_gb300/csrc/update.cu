@@ -2695,13 +2695,15 @@ struct AdjArgs {
 	float2 rho_m[kMaxTaps];
 };
 
+// dL/du is accumulated by channel (element (p, c) at c * W * H + p): the threads
+// of a warp then add to neighbouring words where their pixels are neighbours.
 // Identity part: out = u outside the domain (and on domain pixels without
 // any valid candidate, handled by the means kernel).
 __global__ void k_adj_init(const float *__restrict__ g, const uint8_t *__restrict__ dom, int n, int C,
                            double *__restrict__ gacc)
 {
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n * C; i += gridDim.x * blockDim.x)
-		gacc[i] = dom[i / C] ? 0.0 : (double)g[i];
+		gacc[(size_t)(i % C) * n + i / C] = dom[i / C] ? 0.0 : (double)g[i];
 }
 
 // NL-means: out_c(p) = N_c / D, N_c = sum_i w_i u_c(s_i), D = sum_i w_i, with
@@ -2756,12 +2758,12 @@ __global__ void __launch_bounds__(256) k_means_backward(UpdArgs u, AdjArgs a, co
 					const double wd = (double)w * inv, rho = a.rho[k];
 					const size_t s = (size_t)C * (q.y * W + q.x);
 					for (int c = 0; c < C; c++) {
-						atomicAdd(gacc + s + c, (double)gp[c] * wd);
+						atomicAdd(gacc + (size_t)c * W * H + (q.y * W + q.x), (double)gp[c] * wd);
 						dsig += (double)gp[c] * wd * rho * ((double)img[s + c] - (double)out[c]);
 					}
 				}
 		} else {
-			for (int c = 0; c < C; c++) atomicAdd(gacc + (size_t)C * pix + c, (double)gp[c]);
+			for (int c = 0; c < C; c++) atomicAdd(gacc + (size_t)c * W * H + pix, (double)gp[c]);
 		}
 	}
 	dsig = block_sum<256>(dsig, red);
@@ -2849,7 +2851,7 @@ __global__ void k_poisson_adj_coef(PoissonArgs pa, CoefOut co, AdjCoef ad, const
 				if (hu) v += (double)oml * z[o - (size_t)C * W] * co.S[q - W];   // q is the lower neighbour
 				if (hr) v += (double)oml * z[o + C] * co.S[q];                   // q is the left neighbour
 				if (hl) v += (double)oml * z[o - C] * co.S[q - 1];               // q is the right neighbour
-				if (v != 0.0) atomicAdd(gacc + o, v);
+				if (v != 0.0) atomicAdd(gacc + (size_t)c * W * H + q, v);
 			}
 		}
 		if (act) ad.dS[q] = dS;
@@ -2884,11 +2886,13 @@ __device__ __forceinline__ float2 pair_mul(float2 a, float2 b)
 //   dGY gy(n)).
 // Where the field is coherent, consecutive taps of a window name the same n:
 // their weights (and weights times rho - m) are first added up, as pairs of
-// floats (exact to 2^-43), and n is read and its up to nine double atomics
+// floats (exact to 2^-43; FP64 is a sixty-fourth of the FP32 rate here, and what
+// is left of it still bounds the kernel where the field is rough), and n is read and its up to nine double atomics
 // issued once per run of taps.  One thread per coefficient pixel, the hole
 // pixels first (as k_poisson_coef8's items).  With a thread per image pixel, every
 // tap on its own and rho_k by a double division a 512 x 512 step took 1248 us
-// (29 million atomics); this takes 536 us.
+// (29 million atomics), with the runs but their sums in double 534 us; this
+// takes 294 us.
 template <int C>
 __global__ void __launch_bounds__(128) k_poisson_adj_scatter(UpdArgs u, const __grid_constant__ AdjArgs a, AdjCoef ad,
                                                              const int32_t *__restrict__ hole, int nh,
@@ -2930,31 +2934,35 @@ __global__ void __launch_bounds__(128) k_poisson_adj_scatter(UpdArgs u, const __
 		const float dS = ad.dS[q];
 		int run = -1;                   // the run's source pixel
 		float2 wsum = make_float2(0.f, 0.f), dsum = wsum;  // of w and of dw/dsigma
+		float2 sig = wsum;                                 // the pixel's share of dL/dsigma
 		auto flush = [&]() {
 			const int nx = run % W, ny = run / W;
 			const Pix3 t3 = load_pix3(pad, W, H, nx, ny);
 			const float v[4] = {t3.v.x, t3.v.y, t3.v.z, t3.v.w}, gx[4] = {t3.gx.x, t3.gx.y, t3.gx.z, t3.gx.w};
 			const float gy[4] = {t3.gy.x, t3.gy.y, t3.gy.z, t3.gy.w};
 			const double w = (double)wsum.x + (double)wsum.y;
-			double t = (double)dS;
+			Dot2 t;
+			t.h = dS;
 #pragma unroll
 			for (int c = 0; c < C; c++) {
-				const size_t o = (size_t)C * run + c;
-				t += (double)dU[c] * v[c] + (double)dGX[c] * gx[c] + (double)dGY[c] * gy[c];
+				double *at = gacc + (size_t)c * W * H + run;
+				t.add(dU[c], v[c]);
+				t.add(dGX[c], gx[c]);
+				t.add(dGY[c], gy[c]);
 				double own = w * dU[c];
 				if (nx != W - 1) {
 					const double g = w * dGX[c];
-					atomicAdd(gacc + o + C, g);
+					atomicAdd(at + 1, g);
 					own -= g;
 				}
 				if (ny != H - 1) {
 					const double g = w * dGY[c];
-					atomicAdd(gacc + o + (size_t)C * W, g);
+					atomicAdd(at + W, g);
 					own -= g;
 				}
-				atomicAdd(gacc + o, own);
+				atomicAdd(at, own);
 			}
-			dsig += ((double)dsum.x + (double)dsum.y) * t;
+			pair_add(sig, pair_mul(dsum, make_float2(t.h, t.l)));
 			wsum = dsum = make_float2(0.f, 0.f);
 		};
 		const int cy0 = max(qy - u.hy, 0), cy1 = min(qy + u.hy, H - 1);
@@ -2979,6 +2987,7 @@ __global__ void __launch_bounds__(128) k_poisson_adj_scatter(UpdArgs u, const __
 				pair_add(dsum, pair_mul(w, a.rho_m[k]));
 			}
 		if (run >= 0) flush();
+		dsig = (double)sig.x + (double)sig.y;
 	}
 	dsig = block_sum<128>(dsig, red);
 	if (threadIdx.x == 0) partials[blockIdx.x] = dsig;
@@ -2993,10 +3002,10 @@ __global__ void k_hole_to_planar(const float *__restrict__ g, const int32_t *__r
 	b[i] = g[(size_t)C * hole[k] + c];
 }
 
-__global__ void k_to_float(const double *__restrict__ a, size_t n, float *__restrict__ out)
+__global__ void k_to_float(const double *__restrict__ a, int n, int C, float *__restrict__ out)
 {
-	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-		out[i] = (float)a[i];
+	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n * C; i += gridDim.x * blockDim.x)
+		out[i] = (float)a[(size_t)(i % C) * n + i / C];
 }
 
 static double sum_on_host(nli_ctx *ctx, const double *partials, int n, int stride, int offset)
@@ -3084,7 +3093,7 @@ void update_backward_run(nli_ctx *ctx, const nli_update_params &up, const float 
 		*grad_lambda_d = sum_on_host(ctx, lam_part, grid, 2, 1);
 		*grad_sigma = sum_on_host(ctx, sig_part, grid2, 1, 0);
 	}
-	k_to_float<<<(int)std::min<size_t>((n * C + 255) / 256, 8192), 256, 0, s>>>(gacc, n * C, grad_image);
+	k_to_float<<<(int)std::min<size_t>((n * C + 255) / 256, 8192), 256, 0, s>>>(gacc, (int)n, C, grad_image);
 	NLI_CHECK_LAUNCH();
 	NLI_CUDA(cudaStreamSynchronize(s));
 }
