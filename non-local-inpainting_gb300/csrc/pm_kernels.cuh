@@ -39,7 +39,9 @@
 // (u_s(x+1) - u_t(x+1)) - (u_s(x) - u_t(x)), which equals (gx_s - gx_t) up to
 // float rounding.  Results are accepted in the list's order with a strict
 // "<", so the field equals evaluating each point's candidates one after the
-// other, whatever the grouping.
+// other, whatever the grouping.  Where a call has too few points to fill
+// the SMs it is the other way round: two or four warps share a point
+// (k_pm_sweep_team).
 //
 // Why groups: in a run whose field has converged about two of a point's
 // eighteen proposals survive the bound, so one point filled two of the three
@@ -611,18 +613,16 @@ struct PmCount {
 	unsigned evals, partial, improved, pad;
 };
 
-// Evaluates the list's n entries (candidate x | y << 15 | group << 30), K at a
-// time, and accepts each in order when strictly better than the match of
-// the point it belongs to.  A lane holds its own point's state: group index
-// g, target position txy (x | y << 16), match (as the list's, without the
-// group) and distance bd; lane g * lanes speaks for group g.  count->partial
-// takes the candidates that had reached their point's distance of before
-// the call at the early test (independent of how points are grouped).
+// One round: this lane's part (column c of sub-warp sw) of candidate `cand`
+// (x | y << 15) against the target at t (x | y << 16).  Lanes with c == 0 return
+// their sub-warp's distance, or infinity when every active candidate of the
+// warp had reached its `bound` by the early test.  count->partial takes the
+// active candidates that had reached `start` by then.
 // P > 0: square P x P patch known at compile time (rows unrolled); P == 0:
 // sizes from the arguments.
 template <int KIND, int C, int P>
-__device__ __forceinline__ void eval_list(const PmArgs &p, const float *s_w, const unsigned *list, int n, int g,
-                                          unsigned txy, unsigned &match, float &bd, PmCount *count)
+__device__ __forceinline__ float eval_round(const PmArgs &p, const float *s_w, unsigned cand, unsigned t, int sw, int c,
+                                            bool active, float bound, float start, PmCount *count)
 {
 	constexpr bool G = Kind<KIND>::grad;
 	const int L = P ? P + G : p.L;
@@ -630,11 +630,96 @@ __device__ __forceinline__ void eval_list(const PmArgs &p, const float *s_w, con
 	const int rows = P ? P + G : p.rows;
 	const int px = P ? P : p.rx + p.ex;
 	const int py = P ? P : p.ry + p.ey;
-	const int lane = threadIdx.x & 31;
-	const int sw = lane / L, c = lane - sw * L;
 	const bool tapcol = c < px;
 	const float *W = s_w + c;
 	const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+	// this lane's pixel of the next row to load (sides below 32768: 31 bits)
+	int so = ((int)((cand >> 15) & 0x7fffu) - p.ry) * p.sWp + ((int)(cand & 0x7fffu) - p.rx) + c;
+	int to = ((int)(t >> 16) - p.ry) * p.tWp + ((int)(t & 0xffffu) - p.rx) + c;
+	const int s_n = p.sWp * (p.sH + 1);
+	auto load_s = [&](float4 &v) {
+		// the lanes left over hold no column of a window
+		if (sw < K && nli_in_bounds(so, s_n, kSitePmSource)) v = __ldg(p.src + so);
+		so += p.sWp;
+	};
+	auto load_t = [&](float4 &v) {
+		if (sw < K) v = __ldg(p.tgt + to);
+		to += p.tWp;
+	};
+	// source rows in flight (fewer for 4 channels: registers); the target's
+	// window is the warp's own and in L1 after the first candidate
+	constexpr int PF = C == 4 ? 1 : 2;
+	float4 v[PF], u = zero;
+#pragma unroll
+	for (int r = 0; r < PF; r++) {
+		v[r] = zero;
+		if (r < rows) load_s(v[r]);
+	}
+	load_t(u);
+	float4 dp = zero;
+	float wp = 0.f;
+	Acc A = {0.f, 0.f, 0.f, 0.f};
+	bool stop = false;
+	auto row = [&](int r, float4 &vr) {
+		const float4 d = subc<C>(vr, u);
+		const bool tap = tapcol && r < py;
+		const float w = tap ? W[r * px] : 0.f;
+		if (r + PF < rows) load_s(vr);
+		if (r + 1 < rows) load_t(u);
+		row_terms<KIND, C>(d, dp, w, wp, tap, G && tapcol && r > 0, A);
+		dp = d;
+		wp = w;
+	};
+	auto check = [&]() {
+		const float part = subwarp_sum(combine<KIND>(A, p), c, L);
+		const unsigned reached = __ballot_sync(kFull, active && c == 0 && part >= start);
+		if (reached && (threadIdx.x & 31) == 0) count->partial += __popc(reached);
+		return __all_sync(kFull, !active || c != 0 || part >= bound);
+	};
+	if constexpr (P > 0) {
+#pragma unroll
+		for (int r = 0; r < P + G; r++) {
+			row(r, v[r % PF]);
+			if (r == check_row<P, G>() && check()) {
+				stop = true;
+				break;
+			}
+		}
+	} else {
+#pragma unroll 1
+		for (int r0 = 0; r0 < rows && !stop; r0 += PF) {
+#pragma unroll
+			for (int i = 0; i < PF; i++) {
+				const int r = r0 + i;
+				if (r >= rows) break;
+				row(r, v[i]);
+				if (r == rows / 2 && check()) {
+					stop = true;
+					break;
+				}
+			}
+		}
+	}
+	if (stop) return __int_as_float(0x7f800000);
+	return subwarp_sum(combine<KIND>(A, p), c, L);
+}
+
+// Evaluates the list's n entries (candidate x | y << 15 | group << 30), K at a
+// time, and accepts each in order when strictly better than the match of
+// the point it belongs to.  A lane holds its own point's state: group index
+// g, target position txy (x | y << 16), match (as the list's, without the
+// group) and distance bd; lane g * lanes speaks for group g.  A candidate
+// counts as partial against its point's distance of before the call, which
+// does not depend on how points are grouped.
+template <int KIND, int C, int P>
+__device__ __forceinline__ void eval_list(const PmArgs &p, const float *s_w, const unsigned *list, int n, int g,
+                                          unsigned txy, unsigned &match, float &bd, PmCount *count)
+{
+	constexpr bool G = Kind<KIND>::grad;
+	const int L = P ? P + G : p.L;
+	const int K = P ? 32 / (P + G) : p.K;
+	const int lane = threadIdx.x & 31;
+	const int sw = lane / L, c = lane - sw * L;
 	const float bd0 = bd;
 #pragma unroll 1
 	for (int b = 0; b < n; b += K) {
@@ -643,79 +728,9 @@ __device__ __forceinline__ void eval_list(const PmArgs &p, const float *s_w, con
 		// idle lanes repeat the round's first entry; nothing reads their sums
 		const unsigned e = list[active ? idx : b];
 		const int speaker = (int)(e >> 30) * p.group.lanes;
-		const int cx = (int)(e & 0x7fffu), cy = (int)((e >> 15) & 0x7fffu);
 		const unsigned t = __shfl_sync(kFull, txy, speaker);
-		const float bound = __shfl_sync(kFull, bd, speaker);
-		// this lane's pixel of the next row to load (sides below 32768: 31 bits)
-		int so = (cy - p.ry) * p.sWp + (cx - p.rx) + c;
-		int to = ((int)(t >> 16) - p.ry) * p.tWp + ((int)(t & 0xffffu) - p.rx) + c;
-		const int s_n = p.sWp * (p.sH + 1);
-		auto load_s = [&](float4 &v) {
-			// the lanes left over hold no column of a window
-			if (sw < K && nli_in_bounds(so, s_n, kSitePmSource)) v = __ldg(p.src + so);
-			so += p.sWp;
-		};
-		auto load_t = [&](float4 &v) {
-			if (sw < K) v = __ldg(p.tgt + to);
-			to += p.tWp;
-		};
-		// source rows in flight (fewer for 4 channels: registers); the target's
-		// window is the warp's own and in L1 after the first candidate
-		constexpr int PF = C == 4 ? 1 : 2;
-		float4 v[PF], u = zero;
-#pragma unroll
-		for (int r = 0; r < PF; r++) {
-			v[r] = zero;
-			if (r < rows) load_s(v[r]);
-		}
-		load_t(u);
-		float4 dp = zero;
-		float wp = 0.f;
-		Acc A = {0.f, 0.f, 0.f, 0.f};
-		bool stop = false;
-		auto row = [&](int r, float4 &vr) {
-			const float4 d = subc<C>(vr, u);
-			const bool tap = tapcol && r < py;
-			const float w = tap ? W[r * px] : 0.f;
-			if (r + PF < rows) load_s(vr);
-			if (r + 1 < rows) load_t(u);
-			row_terms<KIND, C>(d, dp, w, wp, tap, G && tapcol && r > 0, A);
-			dp = d;
-			wp = w;
-		};
-		auto check = [&]() {
-			const float part = subwarp_sum(combine<KIND>(A, p), c, L);
-			const float start = __shfl_sync(kFull, bd0, speaker);
-			const unsigned reached = __ballot_sync(kFull, active && c == 0 && part >= start);
-			if (reached && lane == 0) count->partial += __popc(reached);
-			return __all_sync(kFull, !active || c != 0 || part >= bound);
-		};
-		if constexpr (P > 0) {
-#pragma unroll
-			for (int r = 0; r < P + G; r++) {
-				row(r, v[r % PF]);
-				if (r == check_row<P, G>() && check()) {
-					stop = true;
-					break;
-				}
-			}
-		} else {
-#pragma unroll 1
-			for (int r0 = 0; r0 < rows && !stop; r0 += PF) {
-#pragma unroll
-				for (int i = 0; i < PF; i++) {
-					const int r = r0 + i;
-					if (r >= rows) break;
-					row(r, v[i]);
-					if (r == rows / 2 && check()) {
-						stop = true;
-						break;
-					}
-				}
-			}
-		}
-		if (stop) continue;
-		const float sum = subwarp_sum(combine<KIND>(A, p), c, L);
+		const float bound = __shfl_sync(kFull, bd, speaker), start = __shfl_sync(kFull, bd0, speaker);
+		const float sum = eval_round<KIND, C, P>(p, s_w, e, t, sw, c, active, bound, start, count);
 		const int in_round = min(K, n - b);
 #pragma unroll 1
 		for (int s = 0; s < in_round; s++) {
@@ -1186,7 +1201,8 @@ __device__ __forceinline__ void pm_count_clear(unsigned *list)
 // The warp's list of proposals (one per lane at most, packed x | y << 15 with
 // the group above): those that are valid, differ from their point's match and
 // from every lower lane's for the same point.  Returns their number.
-__device__ __forceinline__ int list_proposals(bool valid, unsigned packed, unsigned match, int g, unsigned *list)
+__device__ __forceinline__ int list_proposals(bool valid, unsigned packed, unsigned match, int g, unsigned *list,
+                                              bool counts = true)
 {
 	const int lane = threadIdx.x & 31;
 	const unsigned below = (1u << lane) - 1u;
@@ -1199,7 +1215,7 @@ __device__ __forceinline__ int list_proposals(bool valid, unsigned packed, unsig
 	const unsigned kmask = __ballot_sync(kFull, keep);
 	__syncwarp();
 	if (keep) list[__popc(kmask & below)] = entry;
-	if (lane == 0) pm_count(list)->evals += __popc(kmask);
+	if (lane == 0 && counts) pm_count(list)->evals += __popc(kmask);
 	__syncwarp();
 	return __popc(kmask);
 }
@@ -1278,15 +1294,176 @@ __device__ __forceinline__ void pm_sweep_group(const PmArgs &p, const float *s_w
 	}
 }
 
+// ------------------------------------------------- warps sharing a point
+// Small calls: a block of NW warps takes one point at a time.  Such a sweep lasts
+// as long as one point's chain of instructions (about 2900 in a first call,
+// half of them in rounds), whatever the memory does, so the chain is cut:
+// warp 0 proposes by propagation while the others already draw around the match
+// as it is (the draws are made again where propagation improves it), a window's
+// draws are tried by several lanes at once, and each warp evaluates its share of a
+// step's candidates.  They are then accepted in the list's order, so the field
+// is the one a single warp finds.  A sweep of 750 points (64 x 48, 9 x 9 patch)
+// takes 14.3 us instead of 18.5, the call 252 us instead of 297; the coarse
+// sweeps of a run at 256 x 256 (255 points) 13 us instead of 18.
+// Blocks of NW warps per SM that the team kernels' registers are held to (80 a
+// thread; at 64 they spill and a sweep of 2 warps a point is 5 % slower, at 128
+// too few points run at once: 20 us instead of 14 for 750 points).
+constexpr int team_blocks(int NW) { return 24 / NW; }
+
+// Warps that share a point in a call of nt points; 1: points are grouped by
+// warp.  A team is worth it while all its blocks run at once.  On 152 SMs,
+// with limits of (6, 12), (8, 16), (10, 16) and (6, 24) points per SM for 4
+// and 2 warps: a whole run at 256 x 256 takes 40.0, 40.5, 41.0 and 41.0 ms
+// (43.2 without teams), one on 152 x 97 RGB-D 17.05, 17.2, 17.2 and 17.8 (17.05).
+inline int pm_team(long long nt, int num_sms)
+{
+	return nt <= (long long)team_blocks(4) * num_sms ? 4 : nt <= (long long)team_blocks(2) * num_sms ? 2 : 1;
+}
+
+constexpr unsigned kNoProposal = 0xfffffffeu;
+
+struct PmTeam {
+	unsigned prop[8];    // propagation's proposals
+	unsigned draw[32];   // random search's, by window
+	int shot[32];        // which draw each was
+	float dist[32];      // the step's distances
+};
+
+// Draws of windows first, first + stride, ... by one warp, lanes / window
+// each: the first draw of a window's stream that lands in the source, tested by
+// the bound, into team->draw and team->shot.
+template <int KIND, int C>
+__device__ __forceinline__ void team_draws(const PmArgs &p, const uint2 key, int pix, int x, int y, unsigned match,
+                                           float bd, int windows, int sweep, int first, int stride, PmTeam *team)
+{
+	const int lane = threadIdx.x & 31;
+	const int bx = match == kNoMatch ? -1 : (int)(match & 0x7fffu), by = match == kNoMatch ? -1 : (int)(match >> 15);
+	const int mine = (windows - first + stride - 1) / stride;  // this warp's windows
+	if (mine <= 0) return;
+	const int per = 32 / mine;
+	const int j = lane / per, sub = lane - j * per, k = first + stride * j;
+	const bool has = j < mine;
+	const unsigned group = has ? ((per == 32 ? kFull : (1u << per) - 1u) << (j * per)) : 0u;
+	const int w = p.max_window >> k;
+	const int x_min = max(bx - w, 0), y_min = max(by - w, 0);
+	const uint32_t nx = (uint32_t)(min(bx + w + 1, p.sW) - x_min), ny = (uint32_t)(min(by + w + 1, p.sH) - y_min);
+	bool found = !has;
+	int cx = 0, cy = 0, shot = -1;
+#pragma unroll 1
+	for (int t0 = 0; t0 < p.shots; t0 += per) {
+		const int t = t0 + sub;
+		int qx = 0, qy = 0;
+		bool ok = false;
+		if (!found && t < p.shots) {
+			const uint4 u = Rng::block_of(key, (uint32_t)pix, (uint32_t)sweep, (uint32_t)k, (uint32_t)t >> 1);
+			qx = x_min + (int)__umulhi((t & 1) ? u.z : u.x, nx);
+			qy = y_min + (int)__umulhi((t & 1) ? u.w : u.y, ny);
+			ok = src_ok(p, qx, qy);
+		}
+		const unsigned hit = __ballot_sync(kFull, ok) & group;
+		const int from = hit ? __ffs(hit) - 1 : lane;
+		qx = __shfl_sync(kFull, qx, from);
+		qy = __shfl_sync(kFull, qy, from);
+		if (hit && !found) {
+			cx = qx;
+			cy = qy;
+			shot = t0 + from - j * per;
+			found = true;
+		}
+		if (__all_sync(kFull, found)) break;
+	}
+	const bool keep = has && shot >= 0 && !(p.smom && bound_rejects<KIND, C>(p, x, y, cx, cy, bd));
+	if (has && sub == 0) {
+		team->draw[k] = keep ? (unsigned)cx | ((unsigned)cy << 15) : kNoProposal;
+		team->shot[k] = shot;
+	}
+}
+
+// A step's proposals (in every warp's lanes alike) evaluated by the block's warps
+// together and accepted in order.  `first`: the warp that counts.
+template <int KIND, int C, int P, int NW>
+__device__ __forceinline__ void team_step(const PmArgs &p, const float *s_w, unsigned *list, PmTeam *team, bool valid,
+                                          unsigned packed, unsigned txy, unsigned &match, float &bd)
+{
+	constexpr bool G = Kind<KIND>::grad;
+	const int L = P ? P + G : p.L;
+	const int K = P ? 32 / (P + G) : p.K;
+	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+	const int sw = lane / L, c = lane - sw * L;
+	const int n = list_proposals(valid, packed, match, 0, list, wid == 0);
+	if (n == 0) return;
+	for (int b = wid * K; b < n; b += NW * K) {
+		const int idx = b + sw;
+		const bool active = sw < K && idx < n;
+		const float d = eval_round<KIND, C, P>(p, s_w, list[active ? idx : b], txy, sw, c, active, bd, bd, pm_count(list));
+		if (active && c == 0) team->dist[idx] = d;
+	}
+	__syncthreads();
+	for (int i = 0; i < n; i++) {
+		const float d = team->dist[i];
+		if (d < bd) {
+			bd = d;
+			match = list[i];
+		}
+	}
+	__syncthreads();
+}
+
+// One point of a sweep by the whole block.
+template <int KIND, int C, int P, int NW>
+__device__ __forceinline__ void pm_sweep_team(const PmArgs &p, const float *s_w, unsigned *list, PmTeam *team,
+                                              const uint2 key, int windows, int pix, int sweep, int jump, const PmIo &io,
+                                              int &max_shot)
+{
+	if (!nli_in_bounds(pix, (long long)p.tW * p.tH, kSitePmTarget)) return;
+	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+	const int x = pix % p.tW, y = pix / p.tW;
+	const unsigned txy = (unsigned)x | ((unsigned)y << 16);
+	unsigned match = kNoMatch;
+	float bd = FLT_MAX;
+	const bool inside = tgt_patch_inside(p, x, y);
+	if (inside) {
+		const int2 q = io.nnf_in[pix];
+		bd = io.dist_in[pix];
+		if (q.x >= 0) match = (unsigned)q.x | ((unsigned)q.y << 15);
+		const unsigned before = match;
+		if (wid == 0) {
+			int cx = 0, cy = 0;
+			const bool valid = lane < (jump > 1 ? 8 : 4) && propagated<KIND, C>(p, x, y, lane, sweep, jump, io, bd, cx, cy);
+			if (lane < 8) team->prop[lane] = valid ? (unsigned)cx | ((unsigned)cy << 15) : kNoProposal;
+		} else {
+			team_draws<KIND, C>(p, key, pix, x, y, match, bd, windows, sweep, wid - 1, NW - 1, team);
+		}
+		__syncthreads();
+		unsigned packed = lane < 8 ? team->prop[lane] : kNoProposal;
+		team_step<KIND, C, P, NW>(p, s_w, list, team, packed != kNoProposal, packed, txy, match, bd);
+		if (match != before) {
+			if (wid == 0 && lane == 0) pm_count(list)->improved++;
+			team_draws<KIND, C>(p, key, pix, x, y, match, bd, windows, sweep, wid, NW, team);
+			__syncthreads();
+		}
+		packed = lane < windows ? team->draw[lane] : kNoProposal;
+		if (wid == 0 && lane < windows) max_shot = max(max_shot, team->shot[lane]);
+		team_step<KIND, C, P, NW>(p, s_w, list, team, packed != kNoProposal, packed, txy, match, bd);
+	}
+	if (threadIdx.x == 0) {
+		io.nnf_out[pix] = match == kNoMatch ? make_int2(-1, -1) : make_int2(match & 0x7fffu, match >> 15);
+		io.dist_out[pix] = bd;
+		// a match changes only together with a strictly smaller distance
+		const unsigned hist = sweep ? io.hist_in[pix] : 0u;
+		io.hist_out[pix] = (uint8_t)((hist << 1) | (inside && bd < io.dist_in[pix] ? 1u : 0u));
+	}
+}
+
 // Adds a warp's candidate counts to `counter` (and to `image`'s, if given).
 __device__ __forceinline__ void pm_count_add(unsigned *list, unsigned long long *counter, unsigned long long *image)
 {
 	const PmCount *c = pm_count(list);
-	if ((threadIdx.x & 31) == 0 && c->evals) {
-		atomicAdd(counter, (unsigned long long)c->evals);
+	if ((threadIdx.x & 31) == 0 && (c->evals || c->partial)) {
+		if (c->evals) atomicAdd(counter, (unsigned long long)c->evals);
 		if (c->partial) atomicAdd(counter + 1, (unsigned long long)c->partial);
 		if (image) {
-			atomicAdd(image, (unsigned long long)c->evals);
+			if (c->evals) atomicAdd(image, (unsigned long long)c->evals);
 			if (c->partial) atomicAdd(image + 1, (unsigned long long)c->partial);
 		}
 	}
@@ -1400,6 +1577,33 @@ void sweep_energy(cudaStream_t s, const PmArgs &p, const float *dist, const PmMe
 // The padded source as a tensor map of candidate windows (patchmatch.cu).
 bool encode_source_map(const PmArgs &p, CUtensorMap *map);
 
+template <int KIND, int C, int P, int NW>
+__global__ void __launch_bounds__(32 * NW, team_blocks(NW))
+    k_pm_sweep_team(DistArgs a, PmArgs p, int sweep, int jump, PmIo io, unsigned long long *counter,
+                    unsigned long long *metric_prop, int *metric_shots)
+{
+	__shared__ PmTeam team;
+	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+	const PmSmem m = pm_smem<kPmGrouped>(a, p);
+	unsigned *list = reinterpret_cast<unsigned *>(m.list);
+	load_weights(a, m.w);
+	pm_count_clear(list);
+	const uint2 key = pm_key(p);
+	const int windows = 32 - __clz(p.max_window);
+	int max_shot = -1;
+	for (int i = blockIdx.x; i < p.nt; i += gridDim.x) {
+		pm_sweep_team<KIND, C, P, NW>(p, m.w, list, &team, key, windows, p.tlist[i], sweep, jump, io, max_shot);
+		__syncthreads();  // `team` is the next point's
+	}
+	pm_count_add(list, counter, nullptr);
+	if (metric_prop && lane == 0 && pm_count(list)->improved)
+		atomicAdd(metric_prop, (unsigned long long)pm_count(list)->improved);
+	if (metric_shots && wid == 0) {
+		max_shot = __reduce_max_sync(kFull, max_shot);
+		if (lane == 0 && max_shot >= 0) atomicMax(metric_shots, max_shot);
+	}
+}
+
 // The kernels' dynamic shared-memory limit is raised once per device, to the
 // largest opt-in size (each launch passes the size it uses): a function
 // attribute set on every call costs a driver call per PatchMatch call on
@@ -1453,10 +1657,24 @@ static void launch_grouped(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int
 		                                                                              counter);
 		NLI_CHECK_LAUNCH();
 	}
+	const int team = pm_team(p.nt, ctx->num_sms);
 	for (int it = 0; it < iterations; it++) {
 		ProfScope ps(ctx, "pm_sweep");
-		k_pm_sweep_grouped<KIND, C, P><<<shape.grid, shape.block, smem, ctx->stream>>>(
-		    a, p, it, jump_for(it, p.tW, p.tH), b.io(it), counter, mt.prop ? mt.prop + it : nullptr, mt.shots);
+		const int jump = jump_for(it, p.tW, p.tH);
+		unsigned long long *prop = mt.prop ? mt.prop + it : nullptr;
+		auto by_team = [&](auto nw) {
+			constexpr int NW = decltype(nw)::value;
+			const int grid = std::min(p.nt, team_blocks(NW) * ctx->num_sms);
+			k_pm_sweep_team<KIND, C, P, NW><<<grid, 32 * NW, pm_smem_bytes(a.px * a.py, NW), ctx->stream>>>(
+			    a, p, it, jump, b.io(it), counter, prop, mt.shots);
+		};
+		if (team == 4)
+			by_team(std::integral_constant<int, 4>());
+		else if (team == 2)
+			by_team(std::integral_constant<int, 2>());
+		else
+			k_pm_sweep_grouped<KIND, C, P><<<shape.grid, shape.block, smem, ctx->stream>>>(a, p, it, jump, b.io(it),
+			                                                                               counter, prop, mt.shots);
 		NLI_CHECK_LAUNCH();
 		if (mt.energy) sweep_energy(ctx->stream, p, b.io(it).dist_out, mt, it);
 	}
