@@ -25,6 +25,8 @@ void launch_gradient(cudaStream_t s, const float *img, int W, int H, int C, floa
 // repeating the last ones so that forward differences there are exactly 0.
 __global__ void k_pad4(const float *__restrict__ img, int W, int H, int C, float4 *__restrict__ out)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	pad4_span(img, W, H, C, out, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
@@ -32,7 +34,7 @@ void launch_pad4(cudaStream_t s, const float *img, int W, int H, int C, float4 *
 {
 	const int n = (W + 1) * (H + 1);
 	const int block = 256, grid = (n + block - 1) / block;
-	k_pad4<<<grid, block, 0, s>>>(img, W, H, C, out);
+	launch_early(s, grid, block, 0, k_pad4, img, W, H, C, out);
 	NLI_CHECK_LAUNCH();
 }
 
@@ -49,6 +51,8 @@ constexpr int kPrefixTiles = 2048;
 
 __global__ void k_count(const uint8_t *__restrict__ mask, int n, int *__restrict__ counts)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	__shared__ int s[32];
 	const int base = blockIdx.x * kTile;
 	int c = 0;
@@ -116,6 +120,8 @@ __global__ void __launch_bounds__(kTile)
     k_write(const uint8_t *__restrict__ mask, int n, const int *__restrict__ counts, int32_t *__restrict__ list,
             int *__restrict__ total)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	__shared__ int sums[33], before;
 	const int p = blockIdx.x * kTile + threadIdx.x;
 	const int f = (p < n && mask[p]) ? 1 : 0;
@@ -138,14 +144,14 @@ int compact_mask(nli_ctx *ctx, const uint8_t *mask, int W, int H, int32_t *list,
 	const int tiles = (n + kTile - 1) / kTile;
 	int *counts = ctx->buf<int>(std::string("compact.counts.") + tag, tiles);
 	int *total = (int *)ctx->host_pinned;
-	k_count<<<tiles, 256, 0, ctx->stream>>>(mask, n, counts);
+	launch_early(ctx->stream, tiles, 256, 0, k_count, mask, n, counts);
 	NLI_CHECK_LAUNCH();
 	if (tiles > kPrefixTiles) {
 		k_scan<<<1, 1024, 0, ctx->stream>>>(counts, tiles);
 		NLI_CHECK_LAUNCH();
-		k_write<true><<<tiles, kTile, 0, ctx->stream>>>(mask, n, counts, list, total);
+		launch_early(ctx->stream, tiles, kTile, 0, k_write<true>, mask, n, counts, list, total);
 	} else {
-		k_write<false><<<tiles, kTile, 0, ctx->stream>>>(mask, n, counts, list, total);
+		launch_early(ctx->stream, tiles, kTile, 0, k_write<false>, mask, n, counts, list, total);
 	}
 	NLI_CHECK_LAUNCH();
 	NLI_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -155,6 +161,8 @@ int compact_mask(nli_ctx *ctx, const uint8_t *mask, int W, int H, int32_t *list,
 // Sum of n doubles in a fixed order (one block), for repeatable totals.
 __global__ void k_sum_partials(const double *__restrict__ partials, int n, double *__restrict__ out)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	__shared__ double s[32];
 	double v = 0.0;
 	for (int i = threadIdx.x; i < n; i += blockDim.x) v += partials[i];
@@ -164,7 +172,7 @@ __global__ void k_sum_partials(const double *__restrict__ partials, int n, doubl
 
 void launch_sum_partials(cudaStream_t s, const double *partials, int n, double *out)
 {
-	k_sum_partials<<<1, 1024, 0, s>>>(partials, n, out);
+	launch_early(s, 1, 1024, 0, k_sum_partials, partials, n, out);
 	NLI_CHECK_LAUNCH();
 }
 

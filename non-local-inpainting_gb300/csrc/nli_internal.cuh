@@ -259,6 +259,43 @@ void launch_gradient(cudaStream_t s, const float *img, int W, int H, int C, floa
 // Padded float4 pixel image read by the PatchMatch distance (gradient.cu).
 void launch_pad4(cudaStream_t s, const float *img, int W, int H, int C, float4 *out);
 
+// Launches in a chain where each needs the results of the one before: `kernel` is
+// launched while the launch before it on the stream still runs (programmatic
+// stream serialization), and waits in previous_launch_done().  Every thread of such
+// a kernel calls that before it touches memory that earlier launches write; a
+// launch's completion then implies that of all before it.  Both calls do nothing
+// in a kernel that was launched plainly.  A call of a few short kernels gains
+// 5 to 15 us: PatchMatch on 64 x 48 goes from 220 to 206 us, NL-medians on
+// 382 x 388 from 165 to 152, a Poisson update of 512 x 512 from 301 to 291.
+// in_graph: also while the stream is captured.  There the short kernels are
+// faster with plain edges (a captured run at 256 x 256: 39.3 ms, with all edges
+// programmatic 40.0), the sweeps are not (40.2 with none).
+__device__ __forceinline__ void next_launch_may_start()
+{
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void previous_launch_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <bool in_graph = false, class... K, class... A>
+static inline void launch_early(cudaStream_t s, int grid, int block, size_t smem, void (*kernel)(K...), const A &...args)
+{
+	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+	if (!in_graph && cudaStreamIsCapturing(s, &st) != cudaSuccess) (void)cudaGetLastError();
+	cudaLaunchAttribute at{};
+	at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t c{};
+	c.gridDim = dim3((unsigned)grid);
+	c.blockDim = dim3((unsigned)block);
+	c.dynamicSmemBytes = smem;
+	c.stream = s;
+	c.attrs = &at;
+	c.numAttrs = st == cudaStreamCaptureStatusNone ? 1 : 0;
+	const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...);
+	if (e != cudaSuccess) (void)cudaGetLastError();  // reported here, not again at the next launch
+	NLI_CUDA(e);
+}
+
 // compact.cu: raster-order list of the pixels with mask != 0; returns count
 int compact_mask(nli_ctx *ctx, const uint8_t *mask, int W, int H, int32_t *list, const char *tag);
 

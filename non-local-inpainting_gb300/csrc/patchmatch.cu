@@ -120,6 +120,8 @@ __global__ void __launch_bounds__(kMomW * kMomH)
     k_pm_moments(const __grid_constant__ PmFactors f, const float4 *__restrict__ pad, int W, int H,
                  float4 *__restrict__ mom, unsigned *vmax, int slopes)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	moments_tile(f, pad, W, H, mom, vmax, slopes, blockIdx.x);
 }
 
@@ -165,6 +167,8 @@ __global__ void k_pm_deviations(DistArgs a, const float4 *__restrict__ pad, int 
 // Also advances the context's PatchMatch call index when `calls` is set.
 __global__ void k_fill_nnf(int2 *__restrict__ nnf, float *__restrict__ dist, int n, unsigned long long *calls)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	if (calls && blockIdx.x == 0 && threadIdx.x == 0) *calls += 1ull;
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
 		nnf[i] = make_int2(-1, -1);
@@ -176,6 +180,8 @@ __global__ void k_copy_targets(const int32_t *__restrict__ tlist, int nt, const 
                                const float *__restrict__ dist_src, int2 *__restrict__ nnf_dst,
                                float *__restrict__ dist_dst)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= nt) return;
 	const int pix = tlist[i];
@@ -186,6 +192,8 @@ __global__ void k_copy_targets(const int32_t *__restrict__ tlist, int nt, const 
 __global__ void k_energy(const int32_t *__restrict__ tlist, int nt, const float *__restrict__ dist,
                          double *__restrict__ partials)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	__shared__ double s[32];
 	double v = 0.0;
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
@@ -237,7 +245,7 @@ bool encode_source_map(const PmArgs &p, CUtensorMap *map)
 
 void sweep_energy(cudaStream_t s, const PmArgs &p, const float *dist, const PmMetrics &m, int sweep)
 {
-	k_energy<<<m.partial_blocks, 256, 0, s>>>(p.tlist, p.nt, dist, m.partials);
+	launch_early(s, m.partial_blocks, 256, 0, k_energy, p.tlist, p.nt, dist, m.partials);
 	NLI_CHECK_LAUNCH();
 	launch_sum_partials(s, m.partials, m.partial_blocks, m.energy + sweep);
 }
@@ -424,6 +432,14 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 	cudaStream_t s = ctx->stream;
 	const int nT = tW * tH;
 
+	// cleared before the first kernel: a memset between two would keep the second
+	// from being launched early
+	unsigned *vmax = ctx->tune_pm_bound ? ctx->buf<unsigned>("pm.vmax", 1) : nullptr;
+	if (vmax) NLI_CUDA(cudaMemsetAsync(vmax, 0, sizeof(unsigned), s));
+	// [0]: candidates evaluated, [1]: of these, stopped after the first 32 taps
+	unsigned long long *counter = ctx->buf<unsigned long long>("pm.counter", 2);
+	if (energy) NLI_CUDA(cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned long long), s));
+
 	// padded float4 pixels of source and target
 	float4 *s4 = ctx->buf<float4>("pm.src4", (size_t)(sW + 1) * (sH + 1));
 	launch_pad4(s, src, sW, sH, C, s4);
@@ -441,19 +457,16 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 
 	// tables of the lower bound (NLI_TUNE_PM_BOUND)
 	float4 *smom = nullptr, *tmom = nullptr;
-	unsigned *vmax = nullptr;
 	// the deviation tables serve the L2 kinds (NLI_TUNE_PM_BOUND 2)
 	const int dev = (ctx->tune_pm_bound == 2 && dp.kind != NLI_DIST_L1_NORM) ? 1 : 0;
 	const int slopes = ctx->tune_pm_bound ? bound_slopes(dp, n_target, ctx->num_sms) : 0;
 	if (ctx->tune_pm_bound) {
 		PmFactors f;
 		patch_factors(f, a);
-		vmax = ctx->buf<unsigned>("pm.vmax", 1);
-		NLI_CUDA(cudaMemsetAsync(vmax, 0, sizeof(unsigned), s));
 		auto tables = [&](const char *name, const float4 *pad, int W, int H) {
 			const size_t n = (size_t)(W + 1) * (H + 1);
 			float4 *mom = ctx->buf<float4>(name, n * (dev ? 6 : slopes ? 3 : 1));
-			k_pm_moments<<<moment_tiles(W, H), kMomW * kMomH, 0, s>>>(f, pad, W, H, mom, vmax, slopes);
+			launch_early(s, moment_tiles(W, H), kMomW * kMomH, 0, k_pm_moments, f, pad, W, H, mom, vmax, slopes);
 			NLI_CHECK_LAUNCH();
 			if (dev) {
 				k_pm_deviations<<<(int)((n + 255) / 256), 256, 0, s>>>(a, pad, W, H, mom);
@@ -476,11 +489,10 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 	float *dist_y = ctx->buf<float>("pm.dist_y", nT);
 	const PmFields b = {nnf_x,  nnf_y, dist_x, dist_y, ctx->buf<uint8_t>("pm.hist_x", nT),
 	                    ctx->buf<uint8_t>("pm.hist_y", nT)};
-	// [0]: candidates evaluated, [1]: of these, stopped after the first 32 taps
-	unsigned long long *counter = ctx->buf<unsigned long long>("pm.counter", 2);
 	// the call index advances only for calls with target points, as the
 	// random streams are drawn only then
-	k_fill_nnf<<<(nT + 255) / 256, 256, 0, s>>>(nnf_x, out_dist, nT, n_target > 0 ? &ctx->status->pm_calls : nullptr);
+	launch_early(s, (nT + 255) / 256, 256, 0, k_fill_nnf, nnf_x, out_dist, nT,
+	             n_target > 0 ? &ctx->status->pm_calls : nullptr);
 	NLI_CHECK_LAUNCH();
 	if (n_target > 0) {
 		PmArgs p;
@@ -523,7 +535,6 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 			p.queue = ctx->buf<unsigned>("pm.queue", slots);
 			NLI_CUDA(cudaMemsetAsync(p.queue, 0, sizeof(unsigned) * slots, s));
 		}
-		if (energy) NLI_CUDA(cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned long long), s));
 		PmMetrics mt;
 		const int iters = std::max(pm.iterations, 0);
 		if (metrics && iters > 0) {
@@ -542,14 +553,14 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 		const bool in_y = (pm.iterations % 2) == 1;
 		const int grid = (n_target + 255) / 256;
 		if (in_y || out_dist) {
-			k_copy_targets<<<grid, 256, 0, s>>>(tlist, n_target, in_y ? nnf_y : nnf_x, in_y ? dist_y : dist_x,
+			launch_early(s, grid, 256, 0, k_copy_targets, tlist, n_target, in_y ? nnf_y : nnf_x, in_y ? dist_y : dist_x,
 			                                    in_y ? nnf_x : nullptr, out_dist);
 			NLI_CHECK_LAUNCH();
 		}
 		if (energy) {
 			const int eg = min(grid, 1024);
 			double *partials = ctx->buf<double>("pm.energy", eg + 1);
-			k_energy<<<eg, 256, 0, s>>>(tlist, n_target, in_y ? dist_y : dist_x, partials);
+			launch_early(s, eg, 256, 0, k_energy, tlist, n_target, in_y ? dist_y : dist_x, partials);
 			NLI_CHECK_LAUNCH();
 			launch_sum_partials(s, partials, eg, partials + eg);
 			unsigned long long *hc = reinterpret_cast<unsigned long long *>(ctx->host_pinned);

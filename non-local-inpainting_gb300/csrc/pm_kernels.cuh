@@ -1295,32 +1295,12 @@ __device__ __forceinline__ void pm_sweep_group(const PmArgs &p, const float *s_w
 }
 
 // ------------------------------------------------ sweeps back to back
-// A sweep needs all of the one before, but not its launch: each sweep is launched
-// while the previous one runs, loads its weights and waits for that one's
-// results.  This
-// takes about 2 us off a sweep: a call on 64 x 48 goes from 252 to 232 us, on
-// 512 x 512 from 1378 to 1368, a run at 256 x 256 from 40.2 to 39.3 ms.  The batch
+// A sweep needs all of the one before, but not its launch: it is launched early
+// (launch_early), loads its weights and waits for that one's results.  This
+// takes about 2 us off a sweep: a call on 64 x 48 goes from 252 to 231 us, on
+// 512 x 512 from 1378 to 1360, a run at 256 x 256 from 40.2 to 39.3 ms.  The batch
 // kernels stay with plain launches: their loop's sweeps got slower this way (a
 // batch of 8 images of 64 to 160 pixels 95 -> 109 ms).
-__device__ __forceinline__ void next_launch_may_start() { cudaTriggerProgrammaticLaunchCompletion(); }
-__device__ __forceinline__ void previous_launch_done() { cudaGridDependencySynchronize(); }
-
-// Launches `kernel` as above, after the launch before it on the stream.
-template <class... K, class... A>
-static void launch_early(cudaStream_t s, int grid, int block, size_t smem, void (*kernel)(K...), const A &...args)
-{
-	cudaLaunchAttribute at{};
-	at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	at.val.programmaticStreamSerializationAllowed = 1;
-	cudaLaunchConfig_t c{};
-	c.gridDim = dim3((unsigned)grid);
-	c.blockDim = dim3((unsigned)block);
-	c.dynamicSmemBytes = smem;
-	c.stream = s;
-	c.attrs = &at;
-	c.numAttrs = 1;
-	NLI_CUDA(cudaLaunchKernelEx(&c, kernel, static_cast<K>(args)...));
-}
 
 // ------------------------------------------------- warps sharing a point
 // Small calls: a block of NW warps takes one point at a time.  Such a sweep lasts
@@ -1504,7 +1484,9 @@ __global__ void __launch_bounds__(pm_threads(kPmGrouped), 1)
                       float *__restrict__ dist, unsigned long long *counter)
 {
 	const PmSmem m = pm_smem<kPmGrouped>(a, p);
+	next_launch_may_start();
 	load_weights(a, m.w);
+	previous_launch_done();
 	const uint2 key = pm_key(p);
 	const PmLane at = pm_lane(p.group);
 	unsigned *list = reinterpret_cast<unsigned *>(m.list);
@@ -1685,8 +1667,8 @@ static void launch_grouped(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int
 	const size_t smem = pm_smem_bytes(a.px * a.py, shape.block / 32);
 	{
 		ProfScope ps(ctx, "pm_init");
-		k_pm_init_grouped<KIND, C, P><<<shape.grid, shape.block, smem, ctx->stream>>>(a, p, init, b.nnf_x, b.dist_x,
-		                                                                              counter);
+		launch_early(ctx->stream, shape.grid, shape.block, smem, k_pm_init_grouped<KIND, C, P>, a, p, init, b.nnf_x,
+		             b.dist_x, counter);
 		NLI_CHECK_LAUNCH();
 	}
 	const int team = pm_team(p.nt, ctx->num_sms);
@@ -1697,16 +1679,16 @@ static void launch_grouped(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int
 		auto by_team = [&](auto nw) {
 			constexpr int NW = decltype(nw)::value;
 			const int grid = std::min(p.nt, team_blocks(NW) * ctx->num_sms);
-			launch_early(ctx->stream, grid, 32 * NW, pm_smem_bytes(a.px * a.py, NW), k_pm_sweep_team<KIND, C, P, NW>, a, p,
-			             it, jump, b.io(it), counter, prop, mt.shots);
+			launch_early<true>(ctx->stream, grid, 32 * NW, pm_smem_bytes(a.px * a.py, NW),
+			                   k_pm_sweep_team<KIND, C, P, NW>, a, p, it, jump, b.io(it), counter, prop, mt.shots);
 		};
 		if (team == 4)
 			by_team(std::integral_constant<int, 4>());
 		else if (team == 2)
 			by_team(std::integral_constant<int, 2>());
 		else
-			launch_early(ctx->stream, shape.grid, shape.block, smem, k_pm_sweep_grouped<KIND, C, P>, a, p, it, jump,
-			             b.io(it), counter, prop, mt.shots);
+			launch_early<true>(ctx->stream, shape.grid, shape.block, smem, k_pm_sweep_grouped<KIND, C, P>, a, p, it,
+			                   jump, b.io(it), counter, prop, mt.shots);
 		NLI_CHECK_LAUNCH();
 		if (mt.energy) sweep_energy(ctx->stream, p, b.io(it).dist_out, mt, it);
 	}

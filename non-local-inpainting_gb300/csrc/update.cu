@@ -109,6 +109,8 @@ __global__ void __launch_bounds__(256) k_nlmeans(UpdArgs u, const float *__restr
                                                  const float *__restrict__ conf, float *__restrict__ newval,
                                                  double *__restrict__ partials)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	__shared__ double red[8];
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	const int k = i / u.C, c = i - k * u.C;
@@ -121,6 +123,8 @@ __global__ void __launch_bounds__(256) k_nlmeans(UpdArgs u, const float *__restr
 __global__ void k_scatter_values(const int32_t *__restrict__ hole, int nh, int C, const float *__restrict__ newval,
                                  float *__restrict__ img)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= nh * C) return;
 	const int k = i / C, c = i % C;
@@ -300,6 +304,8 @@ __global__ void __launch_bounds__(32 * kMedWarps) k_nlmedians(UpdArgs u, const f
                                                               const float *__restrict__ conf,
                                                               float *__restrict__ newval, double *__restrict__ partials)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	__shared__ __align__(16) MedSmem<NB> sm[kMedWarps];
 	__shared__ double red[kMedWarps];
 	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -438,6 +444,8 @@ __global__ void __launch_bounds__(128) k_poisson_coef(UpdArgs u, const int32_t *
                                                       const float *__restrict__ conf, const float4 *__restrict__ pad,
                                                       CoefOut out, int32_t *__restrict__ index)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= nh) return;
 	coef_hole_pixel<C>(u, u.W, u.H, i, hole, dom, ext, nnf, conf, pad, out, index);
@@ -547,6 +555,8 @@ __global__ void __launch_bounds__(256) k_poisson_coef8(UpdArgs u, const int32_t 
                                                        const float *__restrict__ conf, const float4 *__restrict__ pad,
                                                        CoefOut out, int32_t *__restrict__ index)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	coef8_item<C>(u, u.W, u.H, (blockIdx.x * blockDim.x + threadIdx.x) >> 3, threadIdx.x & 7, hole, nh, dom, ext, nnf,
 	              conf, pad, out, index);
 }
@@ -664,6 +674,8 @@ __global__ void k_poisson_setup(PoissonArgs a, int chunk, const int32_t *__restr
                                 Unknown *__restrict__ unk, UnkC *__restrict__ unkc, float *__restrict__ b,
                                 float *__restrict__ x0)
 {
+	next_launch_may_start();
+	previous_launch_done();
 	const int k = blockIdx.x * blockDim.x + threadIdx.x;
 	if (k >= a.nh) return;
 	poisson_setup_unknown(a, chunk, k, hole, dom, hole_index, co, img, orig, unk, unkc, b, x0);
@@ -1933,11 +1945,11 @@ static PoissonSystem poisson_system(nli_ctx *ctx, const UpdArgs &u, const nli_up
 		ProfScope ps(ctx, "poisson_coef");
 		if (u.px % 2 == 1 && u.py % 2 == 1) {
 			const long long threads = 3LL * nh * 8;
-			k_poisson_coef8<CC><<<(int)((threads + 255) / 256), 256, 0, s>>>(u, hole, nh, dom, ext, nnf, conf, pad, P.co,
+			launch_early(s, (int)((threads + 255) / 256), 256, 0, k_poisson_coef8<CC>, u, hole, nh, dom, ext, nnf, conf, pad, P.co,
 			                                                                 index);
 		} else {
 			// even patch sides: the window of gather_coef is one wider than the patch
-			k_poisson_coef<CC><<<(nh + 127) / 128, 128, 0, s>>>(u, hole, nh, dom, ext, nnf, conf, pad, P.co, index);
+			launch_early(s, (nh + 127) / 128, 128, 0, k_poisson_coef<CC>, u, hole, nh, dom, ext, nnf, conf, pad, P.co, index);
 		}
 		NLI_CHECK_LAUNCH();
 	});
@@ -1960,7 +1972,7 @@ static PoissonSystem poisson_system(nli_ctx *ctx, const UpdArgs &u, const nli_up
 		P.unk = ctx->buf<Unknown>("poi.unk", nh);
 	{
 		ProfScope ps(ctx, "poisson_setup");
-		k_poisson_setup<<<(nh + 255) / 256, 256, 0, s>>>(pa, P.chunk, hole, dom, index, P.co, image, orig, P.unk,
+		launch_early(s, (nh + 255) / 256, 256, 0, k_poisson_setup, pa, P.chunk, hole, dom, index, P.co, image, orig, P.unk,
 		                                                  P.unkc, P.b, P.x);
 		NLI_CHECK_LAUNCH();
 	}
@@ -2204,20 +2216,20 @@ double update_run(nli_ctx *ctx, const nli_update_params &up, float *image, const
 		grid = (int)(((long long)nh * C + 255) / 256);
 		partials = ctx->buf<double>("upd.partials", grid + 1);
 		ProfScope ps(ctx, "nlmeans");
-		k_nlmeans<<<grid, 256, 0, s>>>(u, image, hole, nh, dom, nnf, conf, newval, partials);
+		launch_early(s, grid, 256, 0, k_nlmeans, u, image, hole, nh, dom, nnf, conf, newval, partials);
 	} else {
 		grid = (nh + kMedWarps - 1) / kMedWarps;
 		partials = ctx->buf<double>("upd.partials", grid + 1);
 		ProfScope ps(ctx, "nlmedians");
 		if (med_window(u) <= 32 * kMedSmall)
-			k_nlmedians<kMedSmall><<<grid, 32 * kMedWarps, 0, s>>>(u, image, hole, nh, dom, nnf, conf, newval,
+			launch_early(s, grid, 32 * kMedWarps, 0, k_nlmedians<kMedSmall>, u, image, hole, nh, dom, nnf, conf, newval,
 			                                                       partials);
 		else
-			k_nlmedians<kMedLarge><<<grid, 32 * kMedWarps, 0, s>>>(u, image, hole, nh, dom, nnf, conf, newval,
+			launch_early(s, grid, 32 * kMedWarps, 0, k_nlmedians<kMedLarge>, u, image, hole, nh, dom, nnf, conf, newval,
 			                                                       partials);
 	}
 	NLI_CHECK_LAUNCH();
-	k_scatter_values<<<(nh * C + 255) / 256, 256, 0, s>>>(hole, nh, C, newval, image);
+	launch_early(s, (nh * C + 255) / 256, 256, 0, k_scatter_values, hole, nh, C, newval, image);
 	NLI_CHECK_LAUNCH();
 	if (!read_back) {
 		launch_sum_partials(s, partials, grid, partials + grid);
