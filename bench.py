@@ -707,11 +707,11 @@ def main():
                     help="NL-Poisson CG: 0 plain (the reference's), 1 Jacobi-preconditioned "
                          "(default: the library's, 0)")
     ap.add_argument("--pm-bound", type=int, default=None, choices=[0, 1, 2],
-                    help="PatchMatch lower bound: 1 patch means, 2 means and deviations, 0 every candidate "
+                    help="PatchMatch lower bound: 1 patch means and slopes, 2 also deviations, 0 every candidate "
                          "evaluated (default: the library's, 1)")
     ap.add_argument("--pm-tile", type=int, default=None,
                     help="PatchMatch work distribution: 0 static block ranges, n > 0 a device work queue of n "
-                         "target points per grab (default: the library's, 1)")
+                         "groups of target points per grab (default: the library's, 1)")
     ap.add_argument("--graph-loop", type=int, default=None, choices=[0, 1, 2],
                     help="iteration loops as CUDA graphs: 1 plain runs and lockstep batches, 2 also worker "
                          "batches, 0 host loops (for profilers that cannot see into conditional graphs); "

@@ -407,7 +407,8 @@ int nli_ctx_set_batch_width(nli_ctx *ctx, int width);
  *   NLI_TUNE_CG_UNKNOWNS_PER_CTA   unknowns per CG CTA at least (default 1024)
  *   NLI_TUNE_BATCH_WIDTH           as nli_ctx_set_batch_width
  *   NLI_TUNE_PM_VARIANT            how 9x9 PatchMatch works: 0 (default) groups
- *                                  of up to three target points per warp, both
+ *                                  of up to three target points per warp (in
+ *                                  small calls up to four warps per point), both
  *                                  windows by plain loads; 1 one point per
  *                                  warp, its window in shared memory and
  *                                  source windows staged there by tensor
@@ -479,7 +480,8 @@ int nli_ctx_set_batch_width(nli_ctx *ctx, int width);
  *                                  (variants 1 and 2: points) per atomic
  *                                  grab (1..1024, default 1); 0 static
  *                                  ranges (block b takes the b-th contiguous
- *                                  range).  Identical fields.
+ *                                  range).  Identical fields; warps that share
+ *                                  a point take no part in it.
  * nli_ctx_get_tuning reads them back. */
 #define NLI_TUNE_CG_CLUSTER_CAP 0
 #define NLI_TUNE_CG_UNKNOWNS_PER_CTA 1

@@ -1,7 +1,7 @@
 """Autotuner for the launch shapes the library leaves open: the size of the
 thread-block clusters of the NL-Poisson conjugate gradient (CTAs per
 cluster, unknowns per CTA), the largest CG system one CTA solves alone
-(NLI_TUNE_CG_SINGLE_MAX), the way the 9x9 PatchMatch kernels read their
+(NLI_TUNE_CG_SINGLE_MAX), how the 9x9 PatchMatch kernels work and read their
 windows (NLI_TUNE_PM_VARIANT), the PatchMatch lower-bound test
 (NLI_TUNE_PM_BOUND) and work distribution (NLI_TUNE_PM_TILE: static ranges
 or a device work queue, and its tile), how a batch runs (NLI_TUNE_BATCH_MODE, the worker
@@ -186,7 +186,7 @@ def tune_pm_bound(ctx, case=None, repeats=3, seed=0):
 
 def tune_pm_tile(ctx, case=None, tiles=(0, 4, 16, 64), repeats=3, seed=0):
     """Times one PatchMatch call per work distribution (0: static block
-    ranges; n: a device work queue handing out n target points per grab)
+    ranges; n: a device work queue handing out n groups of points per grab)
     and keeps the fastest.  Returns {"best": tile, "ms": {tile: ms}}."""
     import torch
     dist, pm, u, src, tgt = case if case is not None else patchmatch_case(ctx)

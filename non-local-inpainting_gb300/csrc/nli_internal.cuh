@@ -296,7 +296,7 @@ static inline void launch_early(cudaStream_t s, int grid, int block, size_t smem
 	NLI_CUDA(e);
 }
 
-// compact.cu: raster-order list of the pixels with mask != 0; returns count
+// gradient.cu: raster-order list of the pixels with mask != 0; returns count
 int compact_mask(nli_ctx *ctx, const uint8_t *mask, int W, int H, int32_t *list, const char *tag);
 
 // reductions

@@ -1294,14 +1294,6 @@ __device__ __forceinline__ void pm_sweep_group(const PmArgs &p, const float *s_w
 	}
 }
 
-// ------------------------------------------------ sweeps back to back
-// A sweep needs all of the one before, but not its launch: it is launched early
-// (launch_early), loads its weights and waits for that one's results.  This
-// takes about 2 us off a sweep: a call on 64 x 48 goes from 252 to 231 us, on
-// 512 x 512 from 1378 to 1360, a run at 256 x 256 from 40.2 to 39.3 ms.  The batch
-// kernels stay with plain launches: their loop's sweeps got slower this way (a
-// batch of 8 images of 64 to 160 pixels 95 -> 109 ms).
-
 // ------------------------------------------------- warps sharing a point
 // Small calls: a block of NW warps takes one point at a time.  Such a sweep lasts
 // as long as one point's chain of instructions (about 2900 in a first call,
@@ -1672,6 +1664,11 @@ static void launch_grouped(nli_ctx *ctx, const DistArgs &a, const PmArgs &p, int
 		NLI_CHECK_LAUNCH();
 	}
 	const int team = pm_team(p.nt, ctx->num_sms);
+	// Launched early a sweep loads its weights while the one before runs: about
+	// 2 us less each, a call on 64 x 48 goes from 252 to 231 us, on 512 x 512
+	// from 1378 to 1360, a run at 256 x 256 from 40.2 to 39.3 ms.  (The batch's
+	// sweeps got slower this way, 8 images of 64 to 160 pixels 95 -> 109 ms, and
+	// keep plain launches.)
 	for (int it = 0; it < iterations; it++) {
 		ProfScope ps(ctx, "pm_sweep");
 		const int jump = jump_for(it, p.tW, p.tH);

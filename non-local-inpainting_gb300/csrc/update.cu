@@ -1,11 +1,11 @@
 // AImageUpdating subclasses as gather kernels over the nearest-neighbour
 // field:
 //   NL-means   (patch_non_local_means.cpp:23-100)   - one thread per hole pixel
+//              and channel
 //   NL-medians (patch_non_local_medians.cpp:23-127) - one warp per hole pixel
 //   NL-Poisson (patch_non_local_poisson.cpp:36-477) - coefficient gather,
-//              right-hand side, and one cooperative kernel running the
-//              conjugate gradient of every channel with fused stencil,
-//              dot products and axpys
+//              right-hand side, and the conjugate gradient of every channel
+//              in one launch: a CTA, a cluster or all SMs, by the system's size
 //   NL-depth   (patch_non_local_depth.cpp:36-55)    - NL-Poisson with a
 //              per-channel lambda on the 4-channel image, orig = image
 #include <cooperative_groups.h>
