@@ -21,6 +21,7 @@ enum CheckSite : unsigned {
 	kSitePmMask = 2,      // PatchMatch: source mask at a candidate
 	kSitePmField = 3,     // PatchMatch: a neighbour's match / the initial field
 	kSitePmTarget = 4,    // PatchMatch: target list entry
+	kSitePmWindow = 5,    // PatchMatch: target window row
 	kSiteMeansSource = 10,  // NL-means / NL-medians: NNF-shifted source pixel
 	kSiteHole = 11,         // hole list entry
 	kSiteCoefSource = 12,   // NL-Poisson coefficient gather: NNF-shifted pixel

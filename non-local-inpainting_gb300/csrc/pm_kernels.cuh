@@ -613,15 +613,19 @@ struct PmCount {
 	unsigned evals, partial, improved, pad;
 };
 
+// The first pixel of the window around target (x, y), in the padded target.
+__device__ __forceinline__ int tgt_window(const PmArgs &p, int x, int y) { return (y - p.ry) * p.tWp + (x - p.rx); }
+
 // One round: this lane's part (column c of sub-warp sw) of candidate `cand`
-// (x | y << 15) against the target at t (x | y << 16).  Lanes with c == 0 return
+// (x | y << 15) against the target whose window starts at t (tgt_window: target
+// sides have no limit, so no packed position holds them).  Lanes with c == 0 return
 // their sub-warp's distance, or infinity when every active candidate of the
 // warp had reached its `bound` by the early test.  count->partial takes the
 // active candidates that had reached `start` by then.
 // P > 0: square P x P patch known at compile time (rows unrolled); P == 0:
 // sizes from the arguments.
 template <int KIND, int C, int P>
-__device__ __forceinline__ float eval_round(const PmArgs &p, const float *s_w, unsigned cand, unsigned t, int sw, int c,
+__device__ __forceinline__ float eval_round(const PmArgs &p, const float *s_w, unsigned cand, int t, int sw, int c,
                                             bool active, float bound, float start, PmCount *count)
 {
 	constexpr bool G = Kind<KIND>::grad;
@@ -635,15 +639,15 @@ __device__ __forceinline__ float eval_round(const PmArgs &p, const float *s_w, u
 	const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 	// this lane's pixel of the next row to load (sides below 32768: 31 bits)
 	int so = ((int)((cand >> 15) & 0x7fffu) - p.ry) * p.sWp + ((int)(cand & 0x7fffu) - p.rx) + c;
-	int to = ((int)(t >> 16) - p.ry) * p.tWp + ((int)(t & 0xffffu) - p.rx) + c;
-	const int s_n = p.sWp * (p.sH + 1);
+	int to = t + c;
+	const int s_n = p.sWp * (p.sH + 1), t_n = p.tWp * (p.tH + 1);
 	auto load_s = [&](float4 &v) {
 		// the lanes left over hold no column of a window
 		if (sw < K && nli_in_bounds(so, s_n, kSitePmSource)) v = __ldg(p.src + so);
 		so += p.sWp;
 	};
 	auto load_t = [&](float4 &v) {
-		if (sw < K) v = __ldg(p.tgt + to);
+		if (sw < K && nli_in_bounds(to, t_n, kSitePmWindow)) v = __ldg(p.tgt + to);
 		to += p.tWp;
 	};
 	// source rows in flight (fewer for 4 channels: registers); the target's
@@ -707,13 +711,13 @@ __device__ __forceinline__ float eval_round(const PmArgs &p, const float *s_w, u
 // Evaluates the list's n entries (candidate x | y << 15 | group << 30), K at a
 // time, and accepts each in order when strictly better than the match of
 // the point it belongs to.  A lane holds its own point's state: group index
-// g, target position txy (x | y << 16), match (as the list's, without the
+// g, target window twin (tgt_window), match (as the list's, without the
 // group) and distance bd; lane g * lanes speaks for group g.  A candidate
 // counts as partial against its point's distance of before the call, which
 // does not depend on how points are grouped.
 template <int KIND, int C, int P>
 __device__ __forceinline__ void eval_list(const PmArgs &p, const float *s_w, const unsigned *list, int n, int g,
-                                          unsigned txy, unsigned &match, float &bd, PmCount *count)
+                                          int twin, unsigned &match, float &bd, PmCount *count)
 {
 	constexpr bool G = Kind<KIND>::grad;
 	const int L = P ? P + G : p.L;
@@ -728,7 +732,7 @@ __device__ __forceinline__ void eval_list(const PmArgs &p, const float *s_w, con
 		// idle lanes repeat the round's first entry; nothing reads their sums
 		const unsigned e = list[active ? idx : b];
 		const int speaker = (int)(e >> 30) * p.group.lanes;
-		const unsigned t = __shfl_sync(kFull, txy, speaker);
+		const int t = __shfl_sync(kFull, twin, speaker);
 		const float bound = __shfl_sync(kFull, bd, speaker), start = __shfl_sync(kFull, bd0, speaker);
 		const float sum = eval_round<KIND, C, P>(p, s_w, e, t, sw, c, active, bound, start, count);
 		const int in_round = min(K, n - b);
@@ -1240,7 +1244,7 @@ __device__ __forceinline__ void pm_init_group(const PmArgs &p, const float *s_w,
 	unsigned match = kNoMatch;
 	float d = FLT_MAX;
 	const int listed = list_proposals(valid && at.k == 0, (unsigned)n.x | ((unsigned)n.y << 15), match, at.g, list);
-	eval_list<KIND, C, P>(p, s_w, list, listed, at.g, (unsigned)x | ((unsigned)y << 16), match, d, count);
+	eval_list<KIND, C, P>(p, s_w, list, listed, at.g, tgt_window(p, x, y), match, d, count);
 	if (has && at.k == 0) {
 		nnf[pix] = match == kNoMatch ? make_int2(-1, -1) : make_int2(match & 0x7fffu, match >> 15);
 		dist[pix] = d;
@@ -1260,7 +1264,7 @@ __device__ __forceinline__ void pm_sweep_group(const PmArgs &p, const float *s_w
 	const int pix = has ? p.tlist[first + at.g] : 0;
 	has = has && nli_in_bounds(pix, (long long)p.tW * p.tH, kSitePmTarget);
 	const int x = pix % p.tW, y = pix / p.tW;
-	const unsigned txy = (unsigned)x | ((unsigned)y << 16);
+	const int twin = tgt_window(p, x, y);
 	const bool inside = has && tgt_patch_inside(p, x, y);
 	unsigned match = kNoMatch;
 	float bd = FLT_MAX;
@@ -1275,7 +1279,7 @@ __device__ __forceinline__ void pm_sweep_group(const PmArgs &p, const float *s_w
 	             propagated<KIND, C>(p, x, y, at.k, sweep, jump, io, bd, cx, cy);
 	int n = list_proposals(valid, (unsigned)cx | ((unsigned)cy << 15), match, at.g, list);
 	if (n) {
-		eval_list<KIND, C, P>(p, s_w, list, n, at.g, txy, match, bd, count);
+		eval_list<KIND, C, P>(p, s_w, list, n, at.g, twin, match, bd, count);
 		const unsigned better = __ballot_sync(kFull, at.k == 0 && bd < bd_in);
 		if (better && at.g == 0 && at.k == 0) count->improved += __popc(better);
 	}
@@ -1284,7 +1288,7 @@ __device__ __forceinline__ void pm_sweep_group(const PmArgs &p, const float *s_w
 	valid = inside && at.k < windows &&
 	        drawn<KIND, C>(p, key, pix, x, y, bx, by, at.k, sweep, bd, cx, cy, max_shot);
 	n = list_proposals(valid, (unsigned)cx | ((unsigned)cy << 15), match, at.g, list);
-	eval_list<KIND, C, P>(p, s_w, list, n, at.g, txy, match, bd, count);
+	eval_list<KIND, C, P>(p, s_w, list, n, at.g, twin, match, bd, count);
 	if (has && at.k == 0) {
 		io.nnf_out[pix] = match == kNoMatch ? make_int2(-1, -1) : make_int2(match & 0x7fffu, match >> 15);
 		io.dist_out[pix] = bd;
@@ -1383,7 +1387,7 @@ __device__ __forceinline__ void team_draws(const PmArgs &p, const uint2 key, int
 // together and accepted in order.  `first`: the warp that counts.
 template <int KIND, int C, int P, int NW>
 __device__ __forceinline__ void team_step(const PmArgs &p, const float *s_w, unsigned *list, PmTeam *team, bool valid,
-                                          unsigned packed, unsigned txy, unsigned &match, float &bd)
+                                          unsigned packed, int twin, unsigned &match, float &bd)
 {
 	constexpr bool G = Kind<KIND>::grad;
 	const int L = P ? P + G : p.L;
@@ -1395,7 +1399,7 @@ __device__ __forceinline__ void team_step(const PmArgs &p, const float *s_w, uns
 	for (int b = wid * K; b < n; b += NW * K) {
 		const int idx = b + sw;
 		const bool active = sw < K && idx < n;
-		const float d = eval_round<KIND, C, P>(p, s_w, list[active ? idx : b], txy, sw, c, active, bd, bd, pm_count(list));
+		const float d = eval_round<KIND, C, P>(p, s_w, list[active ? idx : b], twin, sw, c, active, bd, bd, pm_count(list));
 		if (active && c == 0) team->dist[idx] = d;
 	}
 	__syncthreads();
@@ -1418,7 +1422,7 @@ __device__ __forceinline__ void pm_sweep_team(const PmArgs &p, const float *s_w,
 	if (!nli_in_bounds(pix, (long long)p.tW * p.tH, kSitePmTarget)) return;
 	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 	const int x = pix % p.tW, y = pix / p.tW;
-	const unsigned txy = (unsigned)x | ((unsigned)y << 16);
+	const int twin = tgt_window(p, x, y);
 	unsigned match = kNoMatch;
 	float bd = FLT_MAX;
 	const bool inside = tgt_patch_inside(p, x, y);
@@ -1436,7 +1440,7 @@ __device__ __forceinline__ void pm_sweep_team(const PmArgs &p, const float *s_w,
 		}
 		__syncthreads();
 		unsigned packed = lane < 8 ? team->prop[lane] : kNoProposal;
-		team_step<KIND, C, P, NW>(p, s_w, list, team, packed != kNoProposal, packed, txy, match, bd);
+		team_step<KIND, C, P, NW>(p, s_w, list, team, packed != kNoProposal, packed, twin, match, bd);
 		if (match != before) {
 			if (wid == 0 && lane == 0) pm_count(list)->improved++;
 			team_draws<KIND, C>(p, key, pix, x, y, match, bd, windows, sweep, wid, NW, team);
@@ -1444,7 +1448,7 @@ __device__ __forceinline__ void pm_sweep_team(const PmArgs &p, const float *s_w,
 		}
 		packed = lane < windows ? team->draw[lane] : kNoProposal;
 		if (wid == 0 && lane < windows) max_shot = max(max_shot, team->shot[lane]);
-		team_step<KIND, C, P, NW>(p, s_w, list, team, packed != kNoProposal, packed, txy, match, bd);
+		team_step<KIND, C, P, NW>(p, s_w, list, team, packed != kNoProposal, packed, twin, match, bd);
 	}
 	if (threadIdx.x == 0) {
 		io.nnf_out[pix] = match == kNoMatch ? make_int2(-1, -1) : make_int2(match & 0x7fffu, match >> 15);
