@@ -2877,7 +2877,7 @@ __global__ void __launch_bounds__(256) k_means_backward(UpdArgs u, const __grid_
 #pragma unroll
 		for (int c = 0; c < C; c++) tv[c] = tw;
 		int k = 0;
-		float w = 0.f;
+		float w = 0.f, most = 0.f;  // the largest value
 		for (int t = lane; t < taps; t += 32) {
 			const int src = tap(t, k, w);
 			if (src < 0) continue;
@@ -2886,8 +2886,10 @@ __global__ void __launch_bounds__(256) k_means_backward(UpdArgs u, const __grid_
 			for (int c = 0; c < C; c++) {
 				const float v = img[(size_t)C * src + c], p = fm(v, w);
 				pair_add(tv[c], make_float2(p, fmaf(v, w, -p)));
+				most = fmaxf(most, fabsf(v));
 			}
 		}
+		most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(most)));
 #pragma unroll
 		for (int o = 16; o > 0; o >>= 1) {
 			pair_add(tw, make_float2(__shfl_xor_sync(0xffffffffu, tw.x, o), __shfl_xor_sync(0xffffffffu, tw.y, o)));
@@ -2899,6 +2901,35 @@ __global__ void __launch_bounds__(256) k_means_backward(UpdArgs u, const __grid_
 		const float *gp = g + (size_t)C * pix;
 		if (!(tw.x > 0.0f)) {
 			if (lane < C) atomicAdd(gacc + (size_t)lane * W * H + pix, (double)gp[lane]);
+			continue;
+		}
+		if (!(tw.x >= 0x1p-30f && tw.x <= 0x1p60f && (most == 0.f || (most >= 0x1p-60f && most <= 0x1p60f)))) {
+			// weights or values so small or large that the pairs lose bits or
+			// overflow (a pixel whose only matches lie where the patch weight is
+			// subnormal, a confidence near 0): the same in doubles
+			double D = 0.0, N[C];
+#pragma unroll
+			for (int c = 0; c < C; c++) N[c] = 0.0;
+			for (int t = lane; t < taps; t += 32) {
+				const int src = tap(t, k, w);
+				if (src < 0) continue;
+				D += (double)w;
+#pragma unroll
+				for (int c = 0; c < C; c++) N[c] += (double)w * img[(size_t)C * src + c];
+			}
+			const double inv = 1.0 / __shfl_sync(0xffffffffu, warp_sum(D), 0);
+#pragma unroll
+			for (int c = 0; c < C; c++) N[c] = __shfl_sync(0xffffffffu, warp_sum(N[c]), 0) * inv;
+			for (int t = lane; t < taps; t += 32) {
+				const int src = tap(t, k, w);
+				if (src < 0) continue;
+				const double wd = (double)w * inv, dw = wd * ((double)s_rho[k].x + (double)s_rho[k].y);
+#pragma unroll
+				for (int c = 0; c < C; c++) {
+					atomicAdd(gacc + (size_t)c * W * H + src, (double)gp[c] * wd);
+					dsig += (double)gp[c] * dw * ((double)img[(size_t)C * src + c] - N[c]);
+				}
+			}
 			continue;
 		}
 		// 1 / D to second order, and the output
