@@ -11,6 +11,7 @@
 #include <cooperative_groups.h>
 
 #include <atomic>
+#include <cmath>
 #include <type_traits>
 
 #include "nli_device.cuh"
@@ -2700,7 +2701,9 @@ void update_batch_run(nli_ctx *ctx, const nli_update_params *ups, int C, int n, 
 // weights w_k = e_k / sum_j e_j, e_k = exp(-r_k^2 / (2 sigma^2))
 // (gaussian_weights.cpp:19-79): dw_k/dsigma = w_k (rho_k - m), rho_k =
 // r_k^2 / sigma^3, m = sum_j w_j rho_j.
-// The factor rho_k - m per tap as a pair of floats, formed once on the host.
+// The factor rho_k - m per tap as a pair of floats, formed once on the host and
+// scaled by a power of two so that the largest is near 1 (at sigma 1e13 they are
+// below the smallest float): the kernels' dL/dsigma are scaled so too.
 struct AdjArgs {
 	float2 rho_m[kMaxTaps];
 };
@@ -3123,8 +3126,11 @@ void update_backward_run(nli_ctx *ctx, const nli_update_params &up, const float 
 		rho[k] = u.weights[k] != 0.f ? (double)(kx * kx + ky * ky) / sigma3 : 0.0;
 		if (k < u.px * u.py) m += (double)u.weights[k] * rho[k];
 	}
+	double most = 0.0;
+	for (int k = 0; k < kMaxTaps; k++) most = std::max(most, std::fabs(rho[k] - m));
+	const int exponent = most > 0.0 && std::isfinite(most) ? std::ilogb(most) : 0;
 	for (int k = 0; k < kMaxTaps; k++) {
-		const double d = rho[k] - m;
+		const double d = std::ldexp(rho[k] - m, -exponent);
 		a.rho_m[k].x = (float)d;
 		a.rho_m[k].y = (float)(d - (double)a.rho_m[k].x);
 	}
@@ -3147,7 +3153,7 @@ void update_backward_run(nli_ctx *ctx, const nli_update_params &up, const float 
 			                                                          gacc, part);
 			NLI_CHECK_LAUNCH();
 		});
-		*grad_sigma = sum_on_host(ctx, part, grid, 1, 0);
+		*grad_sigma = std::ldexp(sum_on_host(ctx, part, grid, 1, 0), exponent);
 	} else if (nh > 0) {
 		// system of the forward step with orig = image; its right-hand side
 		// is replaced by g on the hole, and z = A^-1 g is written as an image
@@ -3180,7 +3186,7 @@ void update_backward_run(nli_ctx *ctx, const nli_update_params &up, const float 
 		});
 		*grad_lambda = sum_on_host(ctx, lam_part, grid, 2, 0);
 		*grad_lambda_d = sum_on_host(ctx, lam_part, grid, 2, 1);
-		*grad_sigma = sum_on_host(ctx, sig_part, grid2, 1, 0);
+		*grad_sigma = std::ldexp(sum_on_host(ctx, sig_part, grid2, 1, 0), exponent);
 	}
 	k_to_float<<<(int)std::min<size_t>((n * C + 255) / 256, 8192), 256, 0, s>>>(gacc, (int)n, C, grad_image);
 	NLI_CHECK_LAUNCH();

@@ -1,5 +1,6 @@
 """The adjoints where weights and values lie far from one, against FP64: weight
-sums below the smallest normal float."""
+sums below the smallest normal float, patch sigmas whose derivative lies below
+it, and images and confidences scaled up and down."""
 import numpy as np
 import pytest
 import torch
@@ -70,3 +71,48 @@ def test_means_adjoint_subnormal_confidence(gpu_ctx):
     eps = 2.0 ** -150 / 2.0 ** -134 + 2.0 ** -22
     assert (np.abs(got - want) <= eps * 2 * np.abs(g).max() * 40).all()
     assert abs(ds - ds_want) <= eps * np.abs(g[dom != 0]).sum() * 255 * 32 / 27
+
+
+@pytest.mark.parametrize("sigma", [1e13, 1e6, 3.0])
+@pytest.mark.parametrize("scale", [2.0 ** 119.5, 1.0, 2.0 ** -100])
+def test_means_adjoint_scaled(gpu_ctx, sigma, scale):
+    rng = np.random.default_rng(5)
+    img = (rng.uniform(-255, 255, (H, W, 2)) * scale).astype(np.float32)
+    assert np.isfinite(img).all()
+    dom = np.zeros((H, W), np.uint8)
+    dom[rng.random((H, W)) < 0.3] = 1
+    nnf = field(rng)
+    g = rng.standard_normal((H, W, 2)).astype(np.float32)
+    want, ds_want = means64(img, sigma, nnf, dom, None, g)
+    got, ds = means_ours(gpu_ctx, img, sigma, nnf, dom, None, g)
+    eps = 16 * 2.0 ** -24  # of the float weights, on the sum of the terms' sizes
+    assert (np.abs(got - want) <= eps * 40).all()
+    assert abs(ds - ds_want) <= eps * np.abs(g[dom != 0]).astype(np.float64).sum() * 510 * scale * 32 / sigma ** 3
+
+
+@pytest.mark.parametrize("sigma", [1e13, 3.0])
+@pytest.mark.parametrize("scale,conf", [(1.0, 1.0), (2.0 ** 100, 1.0), (2.0 ** -100, 1.0), (1.0, 2.0 ** -70),
+                                        (1.0, 2.0 ** 60)])
+def test_poisson_adjoint_scaled(gpu_ctx, sigma, scale, conf):
+    """dL/du does not depend on the image's scale (the step is linear in it) nor
+    on the confidence's (it cancels), dL/dsigma follows the image's."""
+    rng = np.random.default_rng(6)
+    img = (rng.uniform(0, 255, (H, W, 2)) * scale).astype(np.float32)
+    dom = np.zeros((H, W), np.uint8)
+    dom[6:18, 5:20] = 1
+    ext = gpu_ctx.extended_domain(dom, 9, 9).cpu().numpy()
+    nnf = field(rng)
+    cf = (rng.uniform(0.1, 1, (H, W)) * conf).astype(np.float32)
+    g = (rng.standard_normal((H, W, 2)) * (dom != 0)[..., None]).astype(np.float32)
+    u = torch.tensor(img / scale, dtype=torch.float64, requires_grad=True)
+    s = torch.tensor(sigma, dtype=torch.float64, requires_grad=True)
+    out = update64.poisson(u, 0.05, s, nnf, dom != 0, ext, cf.astype(np.float64) / conf)
+    (out * torch.tensor(g, dtype=torch.float64)).sum().backward()
+    p = params("nlpoisson", sigma, lam=0.05)
+    o32 = (out.detach().numpy() * scale).astype(np.float32)
+    gi, _, _, ds = gpu_ctx.update_backward(p, img, o32, dom, ext, nnf, cf, g)
+    gi = gi.cpu().numpy().reshape(H, W, 2).astype(np.float64)
+    want = u.grad.numpy()
+    # the solve's |r| < 1e-6 |r0| with a condition number of 153, as tests of the adjoint allow
+    assert np.linalg.norm(gi - want) <= 1e-4 * np.linalg.norm(want)
+    assert abs(ds / scale - s.grad.item()) <= 1e-3 * abs(s.grad.item())
