@@ -1465,7 +1465,12 @@ __global__ void __launch_bounds__(kClusterBlock, 1)
 //
 // The per-thread and per-CTA sums are pairs of floats (exact to 2^-43 of their
 // terms' magnitudes, products included), in place of the double sums of
-// k_poisson_cg.
+// k_poisson_cg.  Products of floats vanish or overflow where doubles do not
+// (tiny or huge gradients, a tolerance near 0): a channel with a sum or quotient
+// outside 1e-28 .. 1e28 is left as it was, and a second launch, DBL, whose blocks
+// otherwise leave at once, solves it with every sum and quotient in double.  (One
+// kernel that forms such sums again in double, by one more exchange, was 20 % slower
+// on systems that never need it: 1680 us instead of 1400 for the update below.)
 //
 // 1024 x 685 (175 000 unknowns, 3 x 50 CTAs, 117 iterations a channel, ncu): 1255
 // us, 10.7 us an iteration, of which the two exchanges take about 8: between
@@ -1481,12 +1486,18 @@ struct GridCgArgs {
 	ulonglong2 *sums;   // [groups of the launch][1 + NV][ctas]
 	DevStatus *st;
 	int *iters;
+	int *redo;  // per channel: left to the launch with double sums
 	const int32_t *hole;
 	const float *orig;
 	float *img;
 	double *diff;
 	const int *active;
 };
+
+// Whether a total or a quotient in pairs has lost nothing to the range of floats:
+// what underflows is below 2^-149 a product, 1e-39 over all unknowns that the
+// SMs hold.
+__device__ __forceinline__ bool wide_safe(float v) { return fabsf(v) >= 1e-28f && fabsf(v) <= 1e28f; }
 
 // Running sum of products as a pair.
 struct Dot2 {
@@ -1500,11 +1511,56 @@ struct Dot2 {
 	}
 };
 
-__device__ __forceinline__ void grid_put(ulonglong2 *p, float x, float y, uint32_t tag)
+// A sum of the solve, as pairs (DBL false) or doubles: of a thread's products, and
+// how it travels in two words.
+template <bool DBL>
+struct WideSum;
+
+template <>
+struct WideSum<false> {
+	typedef Sum2 T;
+	static __device__ __forceinline__ T of(const Dot2 &v) { return {v.h, v.l, 0.f}; }
+	static __device__ __forceinline__ T of(float2 w) { return {w.x, w.y, 0.f}; }
+	static __device__ __forceinline__ float2 words(T v) { return make_float2(v.h, v.l); }
+	static __device__ __forceinline__ T add(T a, T b) { return sum2_add(a, b); }
+	static __device__ __forceinline__ T shfl(T a, int o) { return sum2_shfl(a, o); }
+	static __device__ __forceinline__ double value(T v) { return (double)v.h + (double)v.l; }
+	static __device__ __forceinline__ float quotient(T n, T m)
+	{
+		const float y = __fdividef(1.0f, m.h), q0 = n.h * y;
+		return q0 + fmaf(-q0, m.l, fmaf(-q0, m.h, n.h) + n.l) * y;
+	}
+	static __device__ __forceinline__ bool below(T a, T b) { return (a.h - b.h) + (a.l - b.l) < 0.f; }
+	static __device__ __forceinline__ bool safe(T v) { return wide_safe(v.h); }
+};
+
+struct DotD {
+	double s = 0.0;
+	__device__ __forceinline__ void add(float a, float b) { s += (double)a * b; }
+};
+
+template <>
+struct WideSum<true> {
+	typedef double T;
+	static __device__ __forceinline__ T of(const DotD &v) { return v.s; }
+	static __device__ __forceinline__ T of(float2 w) { return __hiloint2double(__float_as_int(w.x), __float_as_int(w.y)); }
+	static __device__ __forceinline__ float2 words(T v)
+	{
+		return make_float2(__int_as_float(__double2hiint(v)), __int_as_float(__double2loint(v)));
+	}
+	static __device__ __forceinline__ T add(T a, T b) { return a + b; }
+	static __device__ __forceinline__ T shfl(T a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+	static __device__ __forceinline__ double value(T v) { return v; }
+	static __device__ __forceinline__ float quotient(T n, T m) { return (float)(n / m); }
+	static __device__ __forceinline__ bool below(T a, T b) { return a < b; }
+	static __device__ __forceinline__ bool safe(T) { return true; }
+};
+
+__device__ __forceinline__ void grid_put(ulonglong2 *p, float2 v, uint32_t tag)
 {
 	const unsigned long long t = (unsigned long long)tag << 32;
-	asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(t | __float_as_uint(x)),
-	             "l"(t | __float_as_uint(y))
+	asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(t | __float_as_uint(v.x)),
+	             "l"(t | __float_as_uint(v.y))
 	             : "memory");
 }
 
@@ -1536,11 +1592,17 @@ __device__ __forceinline__ bool grid_get(const ulonglong2 *const (&p)[N], int n,
 	}
 }
 
-template <bool PRE, int U>
+// How a solve goes on after an iteration.
+enum { kCgDone, kCgOn, kCgUnsafe };
+
+template <bool PRE, int U, bool DBL>
 __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __grid_constant__ GridCgArgs A)
 {
 	// a batch image that has stopped iterating: every block leaves at once
 	if (A.active && *A.active == 0) return;
+	typedef WideSum<DBL> S;
+	typedef typename S::T Sum;
+	typedef typename std::conditional<DBL, DotD, Dot2>::type Dot;
 	constexpr int NV = PRE ? 2 : 1;
 	extern __shared__ float2 s_pair[];  // two buffers of cg_slots(chunk)
 	__shared__ float2 s_red[NV][16];
@@ -1551,6 +1613,7 @@ __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __gr
 	const int ctas = A.ctas, chunk = A.chunk;
 	const int group = (int)blockIdx.x / ctas, rank = (int)blockIdx.x - group * ctas;
 	const int ch = A.ch0 + group, C = A.a.C, nh = A.a.nh;
+	if (DBL && !A.redo[ch]) return;
 	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 	const int lo = rank * chunk, own = max(0, min(nh, lo + chunk) - lo);
 	const int slots = cg_slots(chunk), zero_slot = 3 * chunk + 2;
@@ -1574,7 +1637,7 @@ __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __gr
 	uint32_t nud[U], nlr[U];
 	uint32_t far = 0;  // 4 bits per unknown: up, left, down, right
 	float r[U], x[U], d[U], q[U];
-	Dot2 acc, accz;
+	Dot acc, accz;
 #pragma unroll
 	for (int u = 0; u < U; u++) {
 		const int l = threadIdx.x + u * kClusterBlock;
@@ -1622,7 +1685,7 @@ __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __gr
 			if (l >= own) break;
 			const float2 v = make_float2(PRE ? fm(minv[u], r[u]) : r[u], d[u]);
 			buf[l] = v;
-			if (far >> (4 * u) & 15u) grid_put(pairs + h * pair_stride + lo + l, v.x, v.y, tag);
+			if (far >> (4 * u) & 15u) grid_put(pairs + h * pair_stride + lo + l, v, tag);
 		}
 	};
 	// the pairs of the neighbours in other ranges (f) of thread t's unknowns into
@@ -1663,20 +1726,21 @@ __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __gr
 	};
 	if (wid == 0) s_far[lane] = far;
 	// a warp's sum into s_red
-	auto warp_pair = [&](const Dot2 &v, float2 *red) {
-		Sum2 t = {v.h, v.l, 0.f};
+	auto warp_pair = [&](const Dot &v, float2 *red) {
+		Sum t = S::of(v);
 #pragma unroll
-		for (int o = 16; o > 0; o >>= 1) t = sum2_add(t, sum2_shfl(t, o));
-		if (lane == 0) red[wid] = make_float2(t.h, t.l);
+		for (int o = 16; o > 0; o >>= 1) t = S::add(t, S::shfl(t, o));
+		if (lane == 0) red[wid] = S::words(t);
 	};
 	// warp 0, after a block barrier: the CTA's sum to the group, and the group's
 	auto send = [&](int v, ulonglong2 *row, uint32_t tag) {
-		const float2 w = s_red[v][lane & 15];
-		const Sum2 t = sum2_16(Sum2{w.x, w.y, 0.f});
-		if (lane == 0) grid_put(row + rank, t.h, t.l, tag);
+		Sum t = S::of(s_red[v][lane & 15]);
+#pragma unroll
+		for (int o = 8; o > 0; o >>= 1) t = S::add(t, S::shfl(t, o));
+		if (lane == 0) grid_put(row + rank, S::words(t), tag);
 	};
 	auto total = [&](const ulonglong2 *row, uint32_t tag) {
-		Sum2 t = {0.f, 0.f, 0.f};
+		Sum t = S::of(make_float2(0.f, 0.f));
 		bool ok = true;
 		constexpr int kRounds = 5;  // up to 160 CTAs
 		const ulonglong2 *p[kRounds];
@@ -1691,48 +1755,48 @@ __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __gr
 		if (n > 0) ok = grid_get(p, n, tag, v, A.st, limit);
 #pragma unroll
 		for (int i = 0; i < kRounds; i++)
-			if (i < n) t = sum2_add(t, Sum2{v[i].x, v[i].y, 0.f});
+			if (i < n) t = S::add(t, S::of(v[i]));
 		__syncwarp();
 #pragma unroll
-		for (int o = 16; o > 0; o >>= 1) t = sum2_add(t, sum2_shfl(t, o));
+		for (int o = 16; o > 0; o >>= 1) t = S::add(t, S::shfl(t, o));
 		if (!ok) s_failed = 1;
 		__syncwarp();
 		return t;
 	};
-	auto quotient = [&](Sum2 n, Sum2 m) -> float {
-		if (!(sum2_safe(n.h) && sum2_safe(m.h)))
-			return (float)(((double)n.h + (double)n.l) / ((double)m.h + (double)m.l));
-		const float y = __fdividef(1.0f, m.h), q0 = n.h * y;
-		return q0 + fmaf(-q0, m.l, fmaf(-q0, m.h, n.h) + n.l) * y;
-	};
-
-	publish(0, 1u);
+	// the first launch's numbers stay below the second's
+	uint32_t tag = DBL ? 0x80000001u : 1u;  // of the current pairs
+	publish(0, tag);
 	warp_pair(acc, s_red[0]);
 	if (PRE) warp_pair(accz, s_red[NV - 1]);
 	__syncthreads();
 	// warp 0 holds the solve's scalars
-	Sum2 rho = {0.f, 0.f, 0.f}, stop = rho;  // <r, z>; tol |r0|^2
+	Sum rho = S::of(make_float2(0.f, 0.f)), stop = rho;  // <r, z>; tol |r0|^2
+	bool unsafe = false;
 	int it = 0;
-	uint32_t tag = 1u;  // of the current pairs
 	if (wid != 0) {
 		fetch(0, tag);
 	} else {
 		for (int v = 0; v < NV; v++) send(v, sums + (1 + v) * ctas, tag);
-		const Sum2 nr0 = total(sums + ctas, tag);
+		const Sum nr0 = total(sums + ctas, tag);
 		rho = PRE ? total(sums + NV * ctas, tag) : nr0;
-		const double t = (double)A.a.tol * ((double)nr0.h + (double)nr0.l);
-		stop.h = (float)t;
-		stop.l = (float)(t - (double)stop.h);
-		if (lane == 0) s_active = nr0.h > 0.f && !s_failed;
+		const double t = (double)A.a.tol * S::value(nr0);
+		if constexpr (DBL) {
+			stop = t;
+		} else {
+			stop.h = (float)t;
+			stop.l = t < 3e38 ? (float)(t - (double)stop.h) : 0.f;
+		}
+		unsafe = !(S::safe(nr0) && S::safe(rho));
+		if (lane == 0) s_active = s_failed ? kCgDone : unsafe ? kCgUnsafe : S::value(nr0) > 0.0 ? kCgOn : kCgDone;
 	}
 	__syncthreads();
-	bool active = s_active != 0;
+	int active = s_active;
 	float beta = 0.f;
 	int h = 0;  // buffer of the current pairs
-	while (active) {
+	while (active == kCgOn) {
 		// d = z + beta d_old (own and neighbours) ; q = A d ; <z, q>
 		const float2 *buf = s_pair + h * slots;
-		acc = Dot2();
+		acc = Dot();
 #pragma unroll
 		for (int u = 0; u < U; u++) {
 			if ((int)threadIdx.x + u * kClusterBlock >= own) break;
@@ -1754,14 +1818,16 @@ __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __gr
 		__syncthreads();
 		if (wid == 0) {
 			send(0, sums, tag);
-			const float alpha = quotient(rho, total(sums, tag));
+			const Sum rq = total(sums, tag);
+			const float alpha = S::quotient(rho, rq);
+			unsafe = !DBL && !(S::safe(rq) && wide_safe(alpha));
 			if (lane == 0) s_coef = alpha;
 		}
 		__syncthreads();
 		const float alpha = s_coef;
 		// r -= alpha q ; z = M r ; |r|^2 (and <r, z>) ; x += alpha d
-		acc = Dot2();
-		accz = Dot2();
+		acc = Dot();
+		accz = Dot();
 #pragma unroll
 		for (int u = 0; u < U; u++) {
 			if ((int)threadIdx.x + u * kClusterBlock >= own) break;
@@ -1779,13 +1845,18 @@ __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __gr
 			fetch(h, tag);
 		} else {
 			for (int v = 0; v < NV; v++) send(v, sums + (1 + v) * ctas, tag);
-			const Sum2 nrn = total(sums + ctas, tag);
-			const Sum2 rhon = PRE ? total(sums + NV * ctas, tag) : nrn;
-			const float bt = quotient(rhon, rho);
-			const bool done = (nrn.h - stop.h) + (nrn.l - stop.l) < 0.f;
+			const Sum nrn = total(sums + ctas, tag);
+			const Sum rhon = PRE ? total(sums + NV * ctas, tag) : nrn;
+			const float bt = S::quotient(rhon, rho);
+			// what underflows in |r|^2 does not matter below a threshold that is safe
+			const bool done = (S::safe(nrn) || S::safe(stop)) && S::below(nrn, stop);
 			if (lane == 0) {
 				s_coef = bt;
-				s_active = !(done || it >= A.a.limit || s_failed);
+				s_active = s_failed                                             ? kCgDone
+				           : unsafe                                             ? kCgUnsafe
+				           : done || it >= A.a.limit                            ? kCgDone
+				           : DBL || (S::safe(nrn) && S::safe(rhon) && wide_safe(bt)) ? kCgOn
+				                                                                : kCgUnsafe;
 			}
 			rho = rhon;
 			it++;
@@ -1799,10 +1870,14 @@ __global__ void __launch_bounds__(kClusterBlock, 1) k_poisson_cg_wide(const __gr
 		// which every thread has read them
 		__syncthreads();
 		beta = s_coef;
-		active = s_active != 0;
+		active = s_active;
 	}
-	if (rank == 0 && threadIdx.x == 0) A.iters[ch] = it;
+	if (rank == 0 && threadIdx.x == 0) {
+		A.iters[ch] = it;
+		if (!DBL) A.redo[ch] = active == kCgUnsafe;
+	}
 	if (s_failed) return;  // reported by the status word
+	if (active == kCgUnsafe) return;
 	// u = orig + delta on the hole (:89-104)
 	double dacc = 0.0;
 #pragma unroll
@@ -1996,10 +2071,16 @@ typedef void (*WideKernel)(GridCgArgs);
 static size_t wide_smem_bytes(int chunk) { return cg_smem_bytes(chunk) + sizeof(uint32_t) * (size_t)chunk; }
 static_assert(2 * sizeof(float2) * (3 * kClusterMaxChunk + 3) + 4 * kClusterMaxChunk <= kSmemBudget, "every chunk fits");
 
+template <bool DBL>
 static WideKernel wide_kernel(bool pre, int chunk)
 {
-	if (chunk <= 5 * kClusterBlock) return pre ? k_poisson_cg_wide<true, 5> : k_poisson_cg_wide<false, 5>;
-	return pre ? k_poisson_cg_wide<true, kClusterPerThread> : k_poisson_cg_wide<false, kClusterPerThread>;
+	if (chunk <= 5 * kClusterBlock) return pre ? k_poisson_cg_wide<true, 5, DBL> : k_poisson_cg_wide<false, 5, DBL>;
+	return pre ? k_poisson_cg_wide<true, kClusterPerThread, DBL> : k_poisson_cg_wide<false, kClusterPerThread, DBL>;
+}
+
+static WideKernel wide_kernel(bool pre, int chunk, bool dbl)
+{
+	return dbl ? wide_kernel<true>(pre, chunk) : wide_kernel<false>(pre, chunk);
 }
 
 static GridLayout grid_layout(nli_ctx *ctx, int nh, int C, int W)
@@ -2018,8 +2099,9 @@ static GridLayout grid_layout(nli_ctx *ctx, int nh, int C, int W)
 		if (!(raised.load(std::memory_order_acquire) & bit)) {
 			for (int pr = 0; pr < 2; pr++)
 				for (int c : {1, kClusterMaxChunk})
-					NLI_CUDA(cudaFuncSetAttribute(wide_kernel(pr, c), cudaFuncAttributeMaxDynamicSharedMemorySize,
-					                              (int)kSmemBudget));
+					for (int dbl = 0; dbl < 2; dbl++)
+						NLI_CUDA(cudaFuncSetAttribute(wide_kernel(pr, c, dbl), cudaFuncAttributeMaxDynamicSharedMemorySize,
+						                              (int)kSmemBudget));
 			raised.fetch_or(bit, std::memory_order_release);
 		}
 		return g;
@@ -2061,6 +2143,7 @@ static void launch_wide_cg(nli_ctx *ctx, const PoissonSystem &P, const GridLayou
 	const int nh = P.pa.nh, C = P.pa.C, rows = pre ? 3 : 2;  // sums per group and CTA
 	const size_t npairs = 2 * (size_t)g.groups * nh, nsums = (size_t)g.groups * rows * g.ctas;
 	ulonglong2 *words = ctx->buf<ulonglong2>("poi.words", npairs + nsums);
+	int *redo = ctx->buf<int>("poi.redo", 4);
 	GridCgArgs A;
 	A.a = P.pa;
 	A.chunk = g.chunk;
@@ -2072,6 +2155,7 @@ static void launch_wide_cg(nli_ctx *ctx, const PoissonSystem &P, const GridLayou
 	A.sums = words + npairs;
 	A.st = ctx->status;
 	A.iters = iters;
+	A.redo = redo;
 	A.hole = hole;
 	A.orig = orig;
 	A.img = img;
@@ -2082,8 +2166,9 @@ static void launch_wide_cg(nli_ctx *ctx, const PoissonSystem &P, const GridLayou
 		A.ch0 = c;
 		void *args[] = {&A};
 		NLI_CUDA(cudaMemsetAsync(words, 0, sizeof(ulonglong2) * (npairs + nsums), ctx->stream));
-		launch_cooperative(ctx, (const void *)wide_kernel(pre, g.chunk), std::min(g.groups, C - c) * g.ctas,
-		                   kClusterBlock, wide_smem_bytes(g.chunk), args);
+		for (int dbl = 0; dbl < 2; dbl++)
+			launch_cooperative(ctx, (const void *)wide_kernel(pre, g.chunk, dbl), std::min(g.groups, C - c) * g.ctas,
+			                   kClusterBlock, wide_smem_bytes(g.chunk), args);
 	}
 }
 
