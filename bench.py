@@ -436,8 +436,8 @@ def run_ours(args):
                 "evaluated_candidates": cand,
                 "evaluated_tflops": eval_tflops,
                 "evaluated_note": "candidates the kernels evaluated (the patch-mean lower bound skips the rest), "
-                                  "each counted at the full 2519 FLOP though %.1f %% of them stopped after 4 of "
-                                  "10 rows" % (100.0 * (c1["candidates_partial"] - c0["candidates_partial"])
+                                  "each counted at the full 2519 FLOP though %.1f %% of them were at their match after 4 of "
+                                  "10 rows, where a round of such candidates stops" % (100.0 * (c1["candidates_partial"] - c0["candidates_partial"])
                                                 / max(cand, 1))}
     cg = prof.get("poisson_cg", (0, 0.0))
     cg_work = c1["cg_unknown_iterations"] - c0["cg_unknown_iterations"]

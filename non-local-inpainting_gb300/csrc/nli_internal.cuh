@@ -104,7 +104,7 @@ struct nli_ctx {
 	nli::DevStatus *status = nullptr;
 	// running counters (for stats)
 	int64_t candidates = 0;
-	int64_t candidates_partial = 0;  // candidates rejected after the first 32 taps
+	int64_t candidates_partial = 0;  // of these, at their point's match by the early-termination test
 	int64_t cg_iterations = 0;
 	int64_t cg_unknown_iterations = 0;  // sum over solves of iterations x unknowns
 	// optional per-region GPU timing with CUDA events (nli_ctx_set_profiling)

@@ -436,7 +436,7 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 	// from being launched early
 	unsigned *vmax = ctx->tune_pm_bound ? ctx->buf<unsigned>("pm.vmax", 1) : nullptr;
 	if (vmax) NLI_CUDA(cudaMemsetAsync(vmax, 0, sizeof(unsigned), s));
-	// [0]: candidates evaluated, [1]: of these, stopped after the first 32 taps
+	// [0]: candidates evaluated, [1]: of these, at their point's match by the early-termination test
 	unsigned long long *counter = ctx->buf<unsigned long long>("pm.counter", 2);
 	if (energy) NLI_CUDA(cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned long long), s));
 

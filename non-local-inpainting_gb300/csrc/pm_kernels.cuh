@@ -771,6 +771,7 @@ __device__ __forceinline__ void eval_candidates(const PmArgs &p, const float *s_
 	const bool tapcol = c < P;
 	const size_t sWp = (size_t)p.sWp;
 	const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+	const float bd0 = bd;  // what a partial candidate is counted against, as in eval_list
 #pragma unroll 1
 	for (int b = 0; b < n; b += K) {
 		const int idx = b + sw;
@@ -848,6 +849,7 @@ __device__ __forceinline__ void eval_candidates(const PmArgs &p, const float *s_
 		};
 		auto check = [&]() {
 			const float part = subwarp_sum(combine<KIND>(A, p), c, L);
+			partial += __popc(__ballot_sync(kFull, active && c == 0 && part >= bd0));
 			return __all_sync(kFull, !active || c != 0 || part >= bound);
 		};
 #pragma unroll
@@ -858,11 +860,8 @@ __device__ __forceinline__ void eval_candidates(const PmArgs &p, const float *s_
 				break;
 			}
 		}
+		if (stop) continue;
 		const int in_step = min(K, n - b);
-		if (stop) {
-			partial += in_step;
-			continue;
-		}
 		const float sum = subwarp_sum(combine<KIND>(A, p), c, L);
 #pragma unroll 1
 		for (int s = 0; s < in_step; s++) {
