@@ -321,7 +321,9 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 // Batched PatchMatch (lockstep batch driver): one image's call.  The image
 // is both source and target; the driver supplies the scratch buffers.
 constexpr int kBatchMax = 64;  // images per batched launch
-constexpr int kPmMomentTables = 6;  // of the lower bound: means, slopes (2), deviations (3)
+// Tables of the lower bound (float4 per padded pixel) that a call of nt target
+// points reads: means, slopes (2), deviations (3).
+int pm_moment_tables(const nli_ctx *ctx, const nli_distance_params &d, int nt);
 struct PmBatchItem {
 	const float *img;
 	int W, H;
@@ -338,7 +340,7 @@ struct PmBatchItem {
 	unsigned long long *calls;    // the image's PatchMatch call index (device)
 	unsigned long long *counter;  // the image's candidate counters (2, device) or null
 	int flag;                     // index of the image's active flag
-	float4 *mom;                  // kPmMomentTables * (W + 1) * (H + 1): tables of the lower bound, or null
+	float4 *mom;                  // pm_moment_tables() * (W + 1) * (H + 1): tables of the lower bound, or null
 	unsigned *vmax;               // the image's largest absolute value (float bits), with mom
 };
 // active: device flags (null: all), item i reads active[items[i].flag];

@@ -52,6 +52,13 @@ static int bound_slopes(const nli_distance_params &d, int nt, int num_sms)
 	return share(d.lambda) && (d.kind != NLI_DIST_L2_RGBD || share(d.lambda_d));
 }
 
+int pm_moment_tables(const nli_ctx *ctx, const nli_distance_params &d, int nt)
+{
+	if (!ctx->tune_pm_bound) return 0;
+	if (ctx->tune_pm_bound == 2 && d.kind != NLI_DIST_L1_NORM) return 6;
+	return bound_slopes(d, nt, ctx->num_sms) ? 3 : 1;
+}
+
 // Means and slopes of every position of the padded (W + 1) x (H + 1) grid
 // (window clamped to the grid), and the largest absolute pixel value (atomicMax
 // on the float bits of non-negative values).  The weights are a product of
@@ -352,7 +359,6 @@ void patchmatch_batch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli
 		p.calls = it.calls;
 		p.smom = p.tmom = it.mom;
 		p.vmax = it.mom ? it.vmax : nullptr;
-		// the item's buffer holds room for every table (kPmMomentTables)
 		p.slopes = it.mom ? bound_slopes(dp, it.nt, ctx->num_sms) : 0;
 		T.moment_tiles = moment_tiles(it.W, it.H);
 		maxtiles = std::max(maxtiles, T.moment_tiles);
@@ -465,7 +471,7 @@ void patchmatch_run(nli_ctx *ctx, const nli_distance_params &dp, const nli_patch
 		patch_factors(f, a);
 		auto tables = [&](const char *name, const float4 *pad, int W, int H) {
 			const size_t n = (size_t)(W + 1) * (H + 1);
-			float4 *mom = ctx->buf<float4>(name, n * (dev ? 6 : slopes ? 3 : 1));
+			float4 *mom = ctx->buf<float4>(name, n * pm_moment_tables(ctx, dp, n_target));
 			launch_early(s, moment_tiles(W, H), kMomW * kMomH, 0, k_pm_moments, f, pad, W, H, mom, vmax, slopes);
 			NLI_CHECK_LAUNCH();
 			if (dev) {

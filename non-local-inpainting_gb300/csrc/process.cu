@@ -686,8 +686,8 @@ class Lockstep {
 			m.scaled = a.take<int32_t>(2 * n0);
 			m.nnf_y = a.take<int32_t>(2 * n0);
 			m.pad = a.take<float4>((size_t)(m.W + 1) * (m.H + 1));
-			// the tables of the PatchMatch bound
-			m.mom = a.take<float4>((size_t)(m.W + 1) * (m.H + 1) * kPmMomentTables);
+			// the tables of the PatchMatch bound, for as many targets as there are pixels
+			m.mom = a.take<float4>((size_t)(m.W + 1) * (m.H + 1) * pm_moment_tables(ctx, p.distance, m.W * m.H));
 			m.dist_x = a.take<float>(n0);
 			m.dist_y = a.take<float>(n0);
 			m.hist_x = a.take<uint8_t>(n0);
