@@ -1347,7 +1347,7 @@ __device__ __forceinline__ void team_draws(const PmArgs &p, const uint2 key, int
 	const int j = lane / per, sub = lane - j * per, k = first + stride * j;
 	const bool has = j < mine;
 	const unsigned group = has ? ((per == 32 ? kFull : (1u << per) - 1u) << (j * per)) : 0u;
-	const int w = p.max_window >> k;
+	const int w = has ? p.max_window >> k : 0;  // (k runs past 31 in the lanes left over)
 	const int x_min = max(bx - w, 0), y_min = max(by - w, 0);
 	const uint32_t nx = (uint32_t)(min(bx + w + 1, p.sW) - x_min), ny = (uint32_t)(min(by + w + 1, p.sH) - y_min);
 	bool found = !has;
