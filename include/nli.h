@@ -505,8 +505,9 @@ uint64_t nli_batch_seed(uint64_t seed, int index);
  * throw std::bad_alloc); this one checks that a failed call leaves the
  * context usable. */
 int nli_debug_fail_allocation(nli_ctx *ctx, int countdown);
-/* Test hook for the bounded device waits: the grid CG's grid barrier gives
- * up after `polls` polls (0 restores the default, 2^26).  A wait that runs
+/* Test hook for the bounded device waits: the waits of the CG on more than a
+ * cluster (for other CTAs' words, or at the grid barrier of the largest systems)
+ * give up after `polls` polls (0 restores the defaults).  A wait that runs
  * out sets the context's timeout word, every block of the kernel leaves,
  * and the call returns NLI_E_TIMEOUT ("a device-side wait timed out"); the
  * word is then cleared, so the context stays usable.  The reference has no

@@ -83,7 +83,7 @@ struct DevStatus {
 	unsigned int barrier_count;
 	unsigned int barrier_gen;
 	int timeout;
-	unsigned int wait_limit;  // grid barrier polls before giving up (0: the default)
+	unsigned int wait_limit;  // polls of the grid CGs' waits before giving up (0: their defaults)
 	unsigned long long pm_calls;
 };
 
@@ -265,8 +265,8 @@ void launch_pad4(cudaStream_t s, const float *img, int W, int H, int C, float4 *
 // a kernel calls that before it touches memory that earlier launches write; a
 // launch's completion then implies that of all before it.  Both calls do nothing
 // in a kernel that was launched plainly.  A call of a few short kernels gains
-// 5 to 15 us: PatchMatch on 64 x 48 goes from 220 to 206 us, NL-medians on
-// 382 x 388 from 165 to 152, a Poisson update of 512 x 512 from 301 to 291.
+// 10 to 15 us: PatchMatch on 64 x 48 goes from 220 to 204 us, NL-medians on
+// 382 x 388 from 165 to 153, a Poisson update of 512 x 512 from 301 to 290.
 // in_graph: also while the stream is captured.  There the short kernels are
 // faster with plain edges (a captured run at 256 x 256: 39.3 ms, with all edges
 // programmatic 40.0), the sweeps are not (40.2 with none).

@@ -1309,8 +1309,9 @@ __device__ __forceinline__ void pm_sweep_group(const PmArgs &p, const float *s_w
 // takes 14.3 us instead of 18.5, the call 252 us instead of 297; the coarse
 // sweeps of a run at 256 x 256 (255 points) 13 us instead of 18.
 // Blocks of NW warps per SM that the team kernels' registers are held to (80 a
-// thread; at 64 they spill and a sweep of 2 warps a point is 5 % slower, at 128
-// too few points run at once: 20 us instead of 14 for 750 points).
+// thread, where the 9 x 9 ones spill 16 bytes; at 64 they spill more and a sweep of 2
+// warps a point is 5 % slower, at 128 too few points run at once: 20 us instead of 14
+// for 750 points).
 constexpr int team_blocks(int NW) { return 24 / NW; }
 
 // Warps that share a point in a call of nt points; 1: points are grouped by
@@ -1723,7 +1724,7 @@ static void run_sweeps(nli_ctx *ctx, const DistArgs &a, PmArgs p, int iterations
 
 // ====================================================== batched launches
 // PatchMatch calls of up to kBatchMax images in one launch per kernel (the
-// lockstep batch driver, lockstep.cu).  Every image is both source and
+// lockstep batch driver, process.cu).  Every image is both source and
 // target (as in the inpainting driver), with its own sizes, masks, target
 // list, seed and call index; the distance, patch and PatchMatch parameters
 // are shared.  Per target point the work is exactly that of the one-image

@@ -1416,8 +1416,14 @@ __device__ __forceinline__ void cg_team_solve(const PoissonArgs &a, int chunk, c
 	if (!SINGLE) cooperative_groups::this_cluster().sync();
 }
 
-// Unknowns per thread the solvers are compiled for: the registers of the
-// larger counts would leave fewer loads in flight on the smaller systems.
+// Unknowns per thread the solvers are compiled for.  The arrays of unused ones cost
+// time: an update whose CTAs hold 1024 unknowns takes 184 us with 2, 3 or 5 per thread
+// and 207 with 8, with 2048 unknowns 207 us with 4, 210 with 5 and 236 with 8, with 2430
+// (a 512 x 512 image's 39 000) 222 with 5, 229 with 6 and 254 with 8.  Above, 6 and 7 where they suffice
+// would gain too (3000 unknowns: 242, 263 and 268 us with 6, 7 and 8; 3480: 280
+// and 297 with 7 and 8), at six more kernels for each count.  k_poisson_cg_wide:
+// 1390 unknowns 365 us with 3, 360 with 4, 377 with 5, 510 with 8; 2500 unknowns 640 us with 5
+// and with 8; 3000: 728 with 6, 760 with 7 and 8; 3500: 685 with 7, 694 with 8.
 constexpr int cg_per_thread(int chunk)
 {
 	return chunk <= 2 * kClusterBlock ? 2 : chunk <= 5 * kClusterBlock ? 5 : kClusterPerThread;
@@ -1472,11 +1478,14 @@ __global__ void __launch_bounds__(kClusterBlock, 1)
 // kernel that forms such sums again in double, by one more exchange, was 20 % slower
 // on systems that never need it: 1680 us instead of 1400 for the update below.)
 //
-// 1024 x 685 (175 000 unknowns, 3 x 50 CTAs, 117 iterations a channel, ncu): 1255
-// us, 10.7 us an iteration, of which the two exchanges take about 8: between
-// 50 CTAs of both dies one takes 3700 to 4200 cycles on its own, between 8
-// neighbouring ones 800 to 1500.  k_poisson_cg, with three grid barriers and
-// its vectors in L2, took 4520 us.
+// 1024 x 685 (175 000 unknowns, 3 x 50 CTAs, 117 iterations a channel, ncu): 1.12
+// ms, 9.6 us an iteration, of which the two exchanges take most: between 50 CTAs of
+// both dies one takes 3700 to 4200 cycles on its own, between 8 neighbouring ones
+// 800 to 1500; the empty launch with double sums takes 2.7 us.  k_poisson_cg, with
+// three grid barriers and its vectors in L2, took 4.52 ms.  The same update (1.47
+// ms) takes 2.08 ms on the image scaled by 2^-70 (all of it in doubles) and 2.63 ms by
+// 2^-50 (in pairs until |r|^2 leaves the range, then again in doubles); it took 5.3
+// ms with k_poisson_cg.
 struct GridCgArgs {
 	PoissonArgs a;
 	int chunk, ctas, ch0;
@@ -2328,7 +2337,7 @@ double update_run(nli_ctx *ctx, const nli_update_params &up, float *image, const
 
 // ======================================================= batched updates
 // The update step of up to kBatchMax images in one launch per kernel (the
-// lockstep batch driver, lockstep.cu).  Each image keeps its own sizes,
+// lockstep batch driver, process.cu).  Each image keeps its own sizes,
 // method, lambda and CG tolerance; the patch and its weights are shared.
 // Every per-pixel / per-unknown value comes from the same device functions
 // as the one-image kernels, and every reduction keeps the one-image
@@ -2923,7 +2932,7 @@ __device__ __forceinline__ float2 pair_mul(float2 a, float2 b)
 // product per atomic is left in double.  Forward and backward of 512 x 512 take
 // 550 us instead of 954, of 66 x 68 454 instead of 700 (most of what is left is
 // launches and waits of the host); the error against 64 bits falls from 1e-6 to
-// 2e-7 for dL/du and from 2e-6 relative to 1e-8 for dL/dsigma, as the sum of the
+// 2e-7 for dL/du and from 5e-6 relative to 1e-8 for dL/dsigma, as the sum of the
 // weights is no longer rounded tap by tap.
 template <int C>
 __global__ void __launch_bounds__(256) k_means_backward(UpdArgs u, const __grid_constant__ AdjArgs a,
